@@ -1733,9 +1733,11 @@ int reverse_core(const snapb_hydro_config* c, const Geo& g, Phys p, const double
   cudaError_t e;
   {
     ScopedTimer t(SNAPB_K_ADJ_RECOMPUTE, st);
-    e = a1 ? launch_x1(g, p, b, last_axis == 1, st) : launch_c2p_only(g, p, b, st);
+    e = a1 ? launch_x1(g, p, b, st) : launch_c2p_only(g, p, b, st);
     if (e != cudaSuccess) return cuda_rc(e, who);
     if (p.implicit_scheme != 0) {
+      if (last_axis == 1 && (e = launch_finalize(g, p, b, nullptr, st)) != cudaSuccess)
+        return cuda_rc(e, who);
       if (a2 && (e = launch_march(2, g, p, b, !a1, last_axis == 2, st)) != cudaSuccess)
         return cuda_rc(e, who);
       if (a3 && (e = launch_march(3, g, p, b, !a1 && !a2, true, st)) != cudaSuccess)

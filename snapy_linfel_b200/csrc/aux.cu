@@ -57,32 +57,6 @@ cudaError_t launch_prim2cons(const Geo& g, const Phys& p, const double* w, doubl
 // of the reflecting axes it crossed.  One thread per cell of the ghost shell
 // (bc_shell_cell enumerates exactly the ghost cells).
 // ---------------------------------------------------------------------------
-struct AxisBC {
-  int n, ng, lo_type, hi_type;
-};
-
-__device__ __forceinline__ int bc_map(const AxisBC& a, int i, bool& flip) {
-  flip = false;
-  if (a.n == 1) return i;
-  if (i < a.ng) {
-    switch (a.lo_type) {
-      case SNAPB_BC_REFLECTING: flip = true; return 2 * a.ng - 1 - i;
-      case SNAPB_BC_PERIODIC: return a.n - 2 * a.ng + i;
-      case SNAPB_BC_OUTFLOW: return a.ng;
-      default: return i;
-    }
-  }
-  if (i >= a.n - a.ng) {
-    switch (a.hi_type) {
-      case SNAPB_BC_REFLECTING: flip = true; return 2 * (a.n - a.ng) - 1 - i;
-      case SNAPB_BC_PERIODIC: return i - a.n + 2 * a.ng;
-      case SNAPB_BC_OUTFLOW: return a.n - a.ng - 1;
-      default: return i;
-    }
-  }
-  return i;
-}
-
 __global__ void k_bc(Geo g, AxisBC a1, AxisBC a2, AxisBC a3, double* var, int nv,
                      int flip_normals) {
   const int64_t s = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;

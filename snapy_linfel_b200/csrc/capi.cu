@@ -159,15 +159,15 @@ int run_stage(const snapb_hydro_config* c, int stage, const double* dt, double* 
   const bool a1 = g.nc1 > 1, a2 = g.nc2 > 1, a3 = g.nc3 > 1;
   const bool diff = p.nu > 0. || p.kappa > 0.;
   if (!a1 && !a2 && !a3) return fail(SNAPB_ERR_ARG, std::string(who) + ": no active axis");
-  // the sweep that finishes the cell: the last active axis, unless only x1 is
-  // active and diffusion must be added after it
-  int last_axis = a3 ? 3 : (a2 ? 2 : 1);
-  bool separate_finalize = (last_axis == 1 && diff);
+  // the sweep that finishes the cell: the last active axis; a 1-D block's cells
+  // (and its ghosts) are finished by their own kernel after the x1 sweep
+  const int last_axis = a3 ? 3 : (a2 ? 2 : 1);
+  const bool fill_1d = last_axis == 1 && mode == 0 && p.implicit_scheme == 0;
   cudaError_t e;
   {
     KernelTimer t(SNAPB_K_X1, st);
     if (a1)
-      e = launch_x1(g, p, b, last_axis == 1 && !separate_finalize, st);
+      e = launch_x1(g, p, b, st);
     else
       e = launch_c2p_only(g, p, b, st);
   }
@@ -187,9 +187,9 @@ int run_stage(const snapb_hydro_config* c, int stage, const double* dt, double* 
     e = launch_march(3, g, p, b, !a1 && !a2, true, st);
     if (e != cudaSuccess) return cuda_status(e, "x3 sweep");
   }
-  if (separate_finalize) {
+  if (last_axis == 1) {
     KernelTimer t(SNAPB_K_FINAL, st);
-    e = launch_finalize(g, p, b, st);
+    e = launch_finalize(g, p, b, fill_1d ? c : nullptr, st);
     if (e != cudaSuccess) return cuda_status(e, "finalize");
   }
   if (p.implicit_scheme != 0) {
@@ -197,7 +197,7 @@ int run_stage(const snapb_hydro_config* c, int stage, const double* dt, double* 
     e = launch_vic(g, p, b, st);
     if (e != cudaSuccess) return cuda_status(e, "implicit solve");
   }
-  if (mode == 0) {
+  if (mode == 0 && !fill_1d) {
     KernelTimer t(SNAPB_K_BC, st);
     e = launch_bc(g, *c, u, c->nvar, SNAPB_CONSERVED, st);
     if (e != cudaSuccess) return cuda_status(e, "hydro boundary");

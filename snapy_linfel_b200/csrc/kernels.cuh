@@ -260,13 +260,43 @@ __device__ __forceinline__ void cfl32_limits(const Geo& g, int use1, int use2, i
   m3 = fmin(m3, 1.7e308);
 }
 
+// source of ghost cell i along one axis (itself inside the block and for
+// 'custom' boundaries); flip: across a reflecting face
+struct AxisBC {
+  int n, ng, lo_type, hi_type;
+};
+
+__device__ __forceinline__ int bc_map(const AxisBC& a, int i, bool& flip) {
+  flip = false;
+  if (a.n == 1) return i;
+  if (i < a.ng) {
+    switch (a.lo_type) {
+      case SNAPB_BC_REFLECTING: flip = true; return 2 * a.ng - 1 - i;
+      case SNAPB_BC_PERIODIC: return a.n - 2 * a.ng + i;
+      case SNAPB_BC_OUTFLOW: return a.ng;
+      default: return i;
+    }
+  }
+  if (i >= a.n - a.ng) {
+    switch (a.hi_type) {
+      case SNAPB_BC_REFLECTING: flip = true; return 2 * (a.n - a.ng) - 1 - i;
+      case SNAPB_BC_PERIODIC: return i - a.n + 2 * a.ng;
+      case SNAPB_BC_OUTFLOW: return a.n - a.ng - 1;
+      default: return i;
+    }
+  }
+  return i;
+}
+
 // launchers (return a cudaError_t of the launch)
-cudaError_t launch_x1(const Geo& g, const Phys& p, const StageBufs& b, bool last,
-                      cudaStream_t st);
+cudaError_t launch_x1(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_c2p_only(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_march(int axis, const Geo& g, const Phys& p, const StageBufs& b, bool first,
                          bool last, cudaStream_t st);
-cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
+// the cells of a 1-D block after its x1 sweep; fill: also its ghost cells
+// (null: left as they are)
+cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b,
+                            const snapb_hydro_config* fill, cudaStream_t st);
 cudaError_t launch_diffusion(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_vic(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_vic32(const Geo& g, const Phys& p, const StageBufs32& b, cudaStream_t st);
@@ -321,8 +351,7 @@ struct ScopedTimer {
 const char* internal_check_config(const snapb_hydro_config* c);
 int internal_fail(int code, const std::string& msg);
 
-// bytes of dynamic shared memory the x1 column kernel needs per column
+// the x1 column size that check_config bounds
 size_t x1_smem_per_column(const Geo& g, int nvt);
-int x1_columns_per_cta(const Geo& g, int nvt);
 
 }  // namespace snapb

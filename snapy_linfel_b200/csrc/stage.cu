@@ -1,17 +1,9 @@
-// stage.cu — the fused per-direction sweeps of one RK stage (FP64 plain form).
+// stage.cu — one RK stage of the FP64 plain form: the launchers of the sweeps
+// (sweep64.cuh), and the kernels beside them:
 //
-//   k_x1     one CTA per group of x1 columns (x1 is the contiguous, vertical
-//            axis): U->W into shared memory, the isentropic x1 ghost revision,
-//            W written back for the other sweeps, WENO/PLM reconstruction +
-//            Riemann flux at every x1 face of the column in registers, and the
-//            x1 flux difference per cell.  Interface states never touch HBM.
-//   k_march  x2 / x3 sweeps: one thread per (x1 cell, other horizontal index)
-//            marches along the sweep axis with a six-cell register window;
-//            consecutive threads are consecutive x1 cells, so every load is
-//            coalesced.  The last active direction finalises the cell:
-//            du = -dt * div / V + gravity (+ diffusion) and either the RK
-//            combination in place or du for the implicit solve.
-//   k_diff   isotropic viscosity / heat-conduction flux differences.
+//   k_diff      isotropic viscosity / heat-conduction flux differences;
+//   k_finalize  the cells of a 1-D block after its x1 sweep (tendency, RK
+//               combination and ghost fill).
 //
 // Reference path: HydroImpl::forward (src/hydro/hydro_forward.cpp:14-217),
 // ReconstructImpl::forward (src/recon/reconstruct.cpp:75-154), the Riemann
@@ -20,241 +12,14 @@
 // (src/hydro/hydro.cpp:217-269), ScalarImpl::forward (src/scalar/scalar.cpp:50-132).
 #include <algorithm>
 
-#include "kernels.cuh"
+#include "sweep64.cuh"
 
 namespace snapb {
 
-// du = -dt*div + forcing for one cell, then the RK combination (or du for the
-// implicit solve).  d holds the flux-difference sums of the nvar hydro
-// variables followed by the scalars; wc is the cell's primitive state.
-template <int NS>
-__device__ __forceinline__ void finalize_cell(const Geo& g, const Phys& p, const StageBufs& b,
-                                              int64_t off, const double* d, const double* wc) {
-  const int64_t sv = g.sv;
-  const double dt = *b.dt;
-  double du[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) du[v] = -dt * (d[v] / g.vol);
-  if (p.grav1 != 0.) {
-    du[IVX] += dt * wc[IDN] * p.grav1 * p.nh;
-    du[IPR] += dt * wc[IDN] * wc[IVX] * p.grav1 * p.nh;
-  }
-  if (p.grav2 != 0.) {
-    du[IVY] += dt * wc[IDN] * p.grav2;
-    du[IPR] += dt * wc[IDN] * wc[IVY] * p.grav2;
-  }
-  if (p.grav3 != 0.) {
-    du[IVZ] += dt * wc[IDN] * p.grav3;
-    du[IPR] += dt * wc[IDN] * wc[IVZ] * p.grav3;
-  }
-  if (p.nu > 0. || p.kappa > 0.) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) du[v] -= dt * (b.DD[v * sv + off] / g.vol);
-  }
-  if (p.has_grav && p.nh < 1.) {
-    double rg = b.RG[off];
-    du[IVX] += dt * rg * (1. - p.nh);
-    du[IPR] += dt * wc[IVX] * rg * (1. - p.nh);
-  }
-  double ds[NS > 0 ? NS : 1];
-#pragma unroll
-  for (int n = 0; n < NS; ++n) ds[n] = -dt * (d[5 + n] / g.vol);
-  if (b.write_du) {
-#pragma unroll
-    for (int v = 0; v < 5; ++v) b.D[v * sv + off] = du[v];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) b.D[(5 + n) * sv + off] = ds[n];
-    return;
-  }
-  double unew_rho = 0.;
-#pragma unroll
-  for (int v = 0; v < 5; ++v) {
-    int64_t o = v * sv + off;
-    double uo = b.u[o];
-    double u0v;
-    if (b.stage == 0) {
-      u0v = uo;
-      b.u0[o] = uo;
-    } else {
-      u0v = b.u0[o];
-    }
-    double un = b.wgt0 * u0v + b.wgt1 * uo + b.wgt2 * du[v];
-    b.u[o] = un;
-    if (v == IDN) unew_rho = un;
-  }
-#pragma unroll
-  for (int n = 0; n < NS; ++n) {
-    int64_t o = n * sv + off;
-    double so = b.s[o];
-    double s0v;
-    if (b.stage == 0) {
-      s0v = so;
-      b.s0[o] = so;
-    } else {
-      s0v = b.s0[o];
-    }
-    double sn = b.wgt0 * s0v + b.wgt1 * so + b.wgt2 * ds[n];
-    b.s[o] = sn;
-    if (b.r) b.r[o] = sn / unew_rho;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// x1 column kernel
-// ---------------------------------------------------------------------------
+// Blocks whose x1 column would not fit this many bytes (W and face fluxes of
+// every variable, two face pressures) are refused by check_config.
 size_t x1_smem_per_column(const Geo& g, int nvt) {
-  // w + face fluxes per variable, plus left/right face pressures
   return (size_t)(2 * nvt + 2) * g.nc1 * sizeof(double);
-}
-
-int x1_columns_per_cta(const Geo& g, int nvt) {
-  size_t per = x1_smem_per_column(g, nvt);
-  int c = (int)std::max<size_t>(1, (96 * 1024) / per);
-  return std::min(c, 16);
-}
-
-template <int NS>
-__global__ void __launch_bounds__(256) k_x1(Geo g, Phys p, StageBufs b, int C, int last) {
-  constexpr int NV = 5 + NS;
-  extern __shared__ double sm[];
-  const int nc1 = g.nc1;
-  double* sw = sm;
-  double* sf = sw + (size_t)C * NV * nc1;
-  double* spl = sf + (size_t)C * NV * nc1;
-  double* spr = spl + (size_t)C * nc1;
-  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  const int64_t col0 = (int64_t)blockIdx.x * C;
-  const int tid = threadIdx.x, nt = blockDim.x;
-  const int64_t sv = g.sv;
-  const double gm1 = p.gammad - 1.;
-
-  // (1) U -> W for every cell of the columns (ghosts included)
-  for (int idx = tid; idx < C * nc1; idx += nt) {
-    int c = idx / nc1, i = idx - c * nc1;
-    int64_t col = col0 + c;
-    if (col >= ncol) continue;
-    int64_t off = col * nc1 + i;
-    double uc[5], wc[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) uc[v] = b.u[v * sv + off];
-    cons2prim_cell(uc, wc, gm1);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) sw[(c * NV + v) * nc1 + i] = wc[v];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      double rr = b.s[n * sv + off] / uc[IDN];
-      sw[(c * NV + 5 + n) * nc1 + i] = rr;
-      b.R[n * sv + off] = rr;
-    }
-  }
-  __syncthreads();
-
-  // (2) isentropic extrapolation of p and rho into the x1 ghosts, one thread
-  // per (column, end)
-  if (p.grav1 != 0. && tid < 2 * C && col0 + (tid >> 1) < ncol) {
-    const int c = tid >> 1, top = tid & 1;
-    double* pp = sw + (c * NV + IPR) * nc1;
-    double* rr = sw + (c * NV + IDN) * nc1;
-    const double gamma = p.gammad;
-    const double a = (gamma - 1.) / gamma, ig = 1. / gamma, ia = 1. / a;
-    const double grav = -p.grav1, dz = g.dx1;
-    const int e = top ? g.iu : g.il, dir = top ? 1 : -1;
-    const double K = pp[e] / pow(rr[e], gamma);
-    const double kg = pow(K, ig);
-    for (int n = 0; n < g.ng; ++n) {
-      double h = top ? pow(pp[e + dir * n], a) - a * grav * dz / kg
-                     : pow(pp[e + dir * n], a) + a * grav * dz / kg;
-      pp[e + dir * (n + 1)] = pow(h, ia);
-      rr[e + dir * (n + 1)] = pow(pp[e + dir * (n + 1)] / K, ig);
-    }
-  }
-  __syncthreads();
-
-  // (3) W back to HBM for the x2/x3 sweeps, the implicit solve and the CFL
-  for (int idx = tid; idx < C * nc1; idx += nt) {
-    int c = idx / nc1, i = idx - c * nc1;
-    int64_t col = col0 + c;
-    if (col >= ncol) continue;
-    int64_t off = col * nc1 + i;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) b.w[v * sv + off] = sw[(c * NV + v) * nc1 + i];
-  }
-
-  // (4) x1 faces il .. iu+1 of interior columns
-  const int nf = g.nx1 + 1;
-  for (int idx = tid; idx < C * nf; idx += nt) {
-    int c = idx / nf, f = g.il + (idx - c * nf);
-    int64_t col = col0 + c;
-    if (col >= ncol) continue;
-    int j = umod(col, g.nc2), k = udiv(col, g.nc2);
-    if (j < g.jl || j > g.ju || k < g.kl || k > g.ku) continue;
-    const double* base = sw + (size_t)c * NV * nc1;
-    double L[NV], R[NV], F[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      double q[6];
-#pragma unroll
-      for (int t = 0; t < 6; ++t) q[t] = base[v * nc1 + min(max(f - 3 + t, 0), nc1 - 1)];
-      if (v < 5) {
-        int typ = (p.r1_shock || v == IDN) ? p.r1_type : interp2_of(p.r1_type);
-        face_states(typ, p.r1_scale != 0, q, L[v], R[v]);
-      } else {
-        face_states(p.rs_type, p.rs_scale != 0, q, L[v], R[v]);
-        L[v] = L[v] < 0. ? 0. : L[v];
-        R[v] = R[v] < 0. ? 0. : R[v];
-      }
-    }
-    if (p.grav1 != 0.) {
-      if (f == g.il) {
-        L[IPR] = R[IPR];
-        L[IDN] = R[IDN];
-      }
-      if (f == g.iu + 1) {
-        R[IPR] = L[IPR];
-        R[IDN] = L[IDN];
-      }
-    }
-    spl[c * nc1 + f] = L[IPR];
-    spr[c * nc1 + f] = R[IPR];
-    if (p.disable1) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) F[v] = 0.;
-    } else {
-      riemann_flux(p.riemann, L, R, IVX, p.gammad, F);
-    }
-#pragma unroll
-    for (int n = 0; n < NS; ++n) F[5 + n] = F[IDN] > 0. ? F[IDN] * L[5 + n] : F[IDN] * R[5 + n];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) sf[(c * NV + v) * nc1 + f] = F[v];
-  }
-  __syncthreads();
-
-  // (5) flux difference per interior cell
-  const bool need_rg = p.grav1 != 0. && p.has_grav && p.nh < 1.;
-  for (int idx = tid; idx < C * g.nx1; idx += nt) {
-    int c = idx / g.nx1, i = g.il + (idx - c * g.nx1);
-    int64_t col = col0 + c;
-    if (col >= ncol) continue;
-    int j = umod(col, g.nc2), k = udiv(col, g.nc2);
-    if (j < g.jl || j > g.ju || k < g.kl || k > g.ku) continue;
-    int64_t off = col * nc1 + i;
-    double d[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const double* fv = sf + (c * NV + v) * nc1;
-      d[v] = g.A1 * fv[i + 1] - g.A1 * fv[i];
-    }
-    if (need_rg) b.RG[off] = (spl[c * nc1 + i + 1] - spr[c * nc1 + i]) / g.dx1;
-    if (last) {
-      double wc[5];
-#pragma unroll
-      for (int v = 0; v < 5; ++v) wc[v] = sw[(c * NV + v) * nc1 + i];
-      finalize_cell<NS>(g, p, b, off, d, wc);
-    } else {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) b.D[v * sv + off] = d[v];
-    }
-  }
 }
 
 // U -> W (and scalar mixing ratios) when x1 is inactive
@@ -270,100 +35,6 @@ __global__ void k_c2p_r(Geo g, Phys p, StageBufs b) {
   for (int v = 0; v < 5; ++v) b.w[v * g.sv + t] = wc[v];
 #pragma unroll
   for (int n = 0; n < NS; ++n) b.R[n * g.sv + t] = b.s[n * g.sv + t] / uc[IDN];
-}
-
-// ---------------------------------------------------------------------------
-// x2 / x3 marching sweeps
-// ---------------------------------------------------------------------------
-template <int NS, int AX>
-__global__ void __launch_bounds__(128) k_march(Geo g, Phys p, StageBufs b, int seglen, int first,
-                                               int last) {
-  constexpr int NV = 5 + NS;
-  const int ni = g.iu - g.il + 1;
-  int lo, hi, olo, ohi;
-  int64_t st, ost;
-  if (AX == 2) {
-    lo = g.jl, hi = g.ju, st = g.s2, olo = g.kl, ohi = g.ku, ost = g.s3;
-  } else {
-    lo = g.kl, hi = g.ku, st = g.s3, olo = g.jl, ohi = g.ju, ost = g.s2;
-  }
-  const int no = ohi - olo + 1;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (int64_t)ni * no) return;
-  const int i = g.il + umod(tid, ni);
-  const int o = olo + udiv(tid, ni);
-  const int f0 = lo + blockIdx.y * seglen;
-  if (f0 > hi) return;
-  const int f1 = min(f0 + seglen, hi + 1);
-  const int64_t base = i + o * ost;
-  const int64_t sv = g.sv;
-  const int ivx = AX == 2 ? IVY : IVZ;
-  const double A = AX == 2 ? g.A2 : g.A3;
-  const int disabled = AX == 2 ? p.disable2 : p.disable3;
-
-  const int ncax = AX == 2 ? g.nc2 : g.nc3;
-  double q[NV][6];
-  // window slots outside the array (only possible for stencils narrower than
-  // the ghost width allows) are clamped; they never enter a narrower stencil
-  auto load = [&](int cell, int slot) {
-    cell = min(max(cell, 0), ncax - 1);
-    int64_t off = base + cell * st;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) q[v][slot] = b.w[v * sv + off];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) q[5 + n][slot] = b.R[n * sv + off];
-  };
-#pragma unroll
-  for (int t = 0; t < 5; ++t) load(f0 - 3 + t, t);
-
-  double Fp[NV];
-  for (int f = f0; f <= f1; ++f) {
-    load(f + 2, 5);
-    double L[NV], R[NV], F[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      if (v < 5) {
-        int typ = (p.r23_shock || v == IDN) ? p.r23_type : interp2_of(p.r23_type);
-        face_states(typ, p.r23_scale != 0, q[v], L[v], R[v]);
-      } else {
-        face_states(p.rs_type, p.rs_scale != 0, q[v], L[v], R[v]);
-        L[v] = L[v] < 0. ? 0. : L[v];
-        R[v] = R[v] < 0. ? 0. : R[v];
-      }
-    }
-    if (disabled) {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) F[v] = 0.;
-    } else {
-      riemann_flux(p.riemann, L, R, ivx, p.gammad, F);
-    }
-#pragma unroll
-    for (int n = 0; n < NS; ++n) F[5 + n] = F[IDN] > 0. ? F[IDN] * L[5 + n] : F[IDN] * R[5 + n];
-    if (f > f0) {
-      const int64_t off = base + (int64_t)(f - 1) * st;
-      double d[NV];
-#pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        d[v] = A * F[v] - A * Fp[v];
-        if (!first) d[v] = b.D[v * sv + off] + d[v];
-      }
-      if (last) {
-        double wc[5];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) wc[v] = q[v][2];
-        finalize_cell<NS>(g, p, b, off, d, wc);
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) b.D[v * sv + off] = d[v];
-      }
-    }
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      Fp[v] = F[v];
-#pragma unroll
-      for (int t = 0; t < 5; ++t) q[v][t] = q[v][t + 1];
-    }
-  }
 }
 
 // ---------------------------------------------------------------------------
@@ -450,9 +121,13 @@ __global__ void k_diff(Geo g, Phys p, StageBufs b) {
   for (int v = 0; v < 5; ++v) b.DD[v * g.sv + t] = acc[v];
 }
 
-// stand-alone finalisation when no march kernel runs last (1-D with diffusion)
+// The cells of a block whose only active axis is x1, after its sweep (whose
+// warps share a column, so they may not update u while others read it): the
+// tendency, then du or the RK combination; with fill, the thread of a cell
+// also writes the ghost cells that are images of it (a ghost fill without its
+// own launch; at most 2 ng images a cell).
 template <int NS>
-__global__ void k_finalize(Geo g, Phys p, StageBufs b) {
+__global__ void k_finalize(Geo g, Phys p, StageBufs b, AxisBC a1, int fill) {
   constexpr int NV = 5 + NS;
   const int ni = g.iu - g.il + 1, nj = g.ju - g.jl + 1, nk = g.ku - g.kl + 1;
   int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -460,54 +135,142 @@ __global__ void k_finalize(Geo g, Phys p, StageBufs b) {
   int i = g.il + umod(tid, ni);
   int j = g.jl + umod(udiv(tid, ni), nj);
   int k = g.kl + udiv(tid, (int64_t)ni * nj);
-  int64_t off = (int64_t)k * g.s3 + (int64_t)j * g.s2 + i;
+  const int64_t row = (int64_t)k * g.s3 + (int64_t)j * g.s2, off = row + i;
   double d[NV], wc[5];
 #pragma unroll
   for (int v = 0; v < NV; ++v) d[v] = b.D[v * g.sv + off];
 #pragma unroll
   for (int v = 0; v < 5; ++v) wc[v] = b.w[v * g.sv + off];
-  finalize_cell<NS>(g, p, b, off, d, wc);
+  const double dt = *b.dt;
+  finalize_cell<NS>(g, p, b, off, d, wc, dt, dt / g.vol);
+  if (!fill) return;
+  for (int m = 0; m < 2 * g.ng; ++m) {
+    const int gi = m < g.ng ? m : g.nc1 - 2 * g.ng + m;
+    bool flip;
+    if (bc_map(a1, gi, flip) != i) continue;
+#pragma unroll
+    for (int v = 0; v < 5; ++v) {
+      const double x = b.u[v * g.sv + off];
+      b.u[v * g.sv + row + gi] = v == IVX && flip ? -x : x;
+    }
+#pragma unroll
+    for (int n = 0; n < NS; ++n) b.s[n * g.sv + row + gi] = b.s[n * g.sv + off];
+  }
 }
 
 // ---------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------
-cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
+// Profile of the sweeps along `axis` (sweep64.cuh): the reconstruction profile
+// that the options amount to, 0 when none does.
+static int recon_profile64(const Phys& p, int axis) {
+  const int typ = axis == 1 ? p.r1_type : p.r23_type;
+  const int shock = axis == 1 ? p.r1_shock : p.r23_shock;
+  const int scale = axis == 1 ? p.r1_scale : p.r23_scale;
+  if (scale || (p.nscalar > 0 && (p.rs_type != typ || p.rs_scale))) return 0;
+  if (typ == SNAPB_RECON_PLM) return 3;
+  if (typ != SNAPB_RECON_WENO5) return 0;
+  return shock ? (p.nscalar ? 0 : 2) : 1;
+}
+
+// f(NS, RP, SV) as compile-time constants
+template <class F>
+static cudaError_t with_profile64(const Phys& p, int axis, F&& f) {
+  auto with = [&](auto ns) -> cudaError_t {
+    using std::integral_constant;
+    constexpr int NS = decltype(ns)::value;
+    auto solver = [&](auto rp) -> cudaError_t {
+      switch (p.riemann) {
+        case SNAPB_RIEMANN_LMARS:
+          return f(ns, rp, integral_constant<int, SNAPB_RIEMANN_LMARS>{});
+        case SNAPB_RIEMANN_HLLC: return f(ns, rp, integral_constant<int, SNAPB_RIEMANN_HLLC>{});
+        default: return f(ns, rp, integral_constant<int, SNAPB_RIEMANN_ROE>{});
+      }
+    };
+    switch (recon_profile64(p, axis)) {
+      case 1: return solver(integral_constant<int, 1>{});
+      case 2:
+        if constexpr (NS == 0) return solver(integral_constant<int, 2>{});
+        break;
+      case 3: return solver(integral_constant<int, 3>{});
+    }
+    return f(ns, integral_constant<int, 0>{}, integral_constant<int, -1>{});
+  };
+  switch (p.nscalar) {
+    case 0: return with(std::integral_constant<int, 0>{});
+    case 1: return with(std::integral_constant<int, 1>{});
+    case 2: return with(std::integral_constant<int, 2>{});
+    case 3: return with(std::integral_constant<int, 3>{});
+  }
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b,
+                            const snapb_hydro_config* fill, cudaStream_t st) {
   int64_t n = (int64_t)(g.iu - g.il + 1) * (g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   unsigned grid = (unsigned)((n + 127) / 128);
+  const AxisBC a1{g.nc1, g.ng, fill ? fill->bc[0] : 0, fill ? fill->bc[1] : 0};
+  const int fl = fill ? 1 : 0;
   switch (p.nscalar) {
-    case 0: k_finalize<0><<<grid, 128, 0, st>>>(g, p, b); break;
-    case 1: k_finalize<1><<<grid, 128, 0, st>>>(g, p, b); break;
-    case 2: k_finalize<2><<<grid, 128, 0, st>>>(g, p, b); break;
-    case 3: k_finalize<3><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 0: k_finalize<0><<<grid, 128, 0, st>>>(g, p, b, a1, fl); break;
+    case 1: k_finalize<1><<<grid, 128, 0, st>>>(g, p, b, a1, fl); break;
+    case 2: k_finalize<2><<<grid, 128, 0, st>>>(g, p, b, a1, fl); break;
+    case 3: k_finalize<3><<<grid, 128, 0, st>>>(g, p, b, a1, fl); break;
     default: return cudaErrorInvalidValue;
   }
   return cudaGetLastError();
 }
 
-template <int NS>
-static cudaError_t launch_x1_t(const Geo& g, const Phys& p, const StageBufs& b, bool last,
-                               cudaStream_t st) {
-  const int nvt = 5 + NS;
-  int C = x1_columns_per_cta(g, nvt);
-  size_t smem = (size_t)C * x1_smem_per_column(g, nvt);
-  if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
-  raise_smem_limit(k_x1<NS>, 200 * 1024);
-  int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  int64_t grid = (ncol + C - 1) / C;
-  k_x1<NS><<<(unsigned)grid, 256, smem, st>>>(g, p, b, C, last ? 1 : 0);
-  return cudaGetLastError();
+// How the x1 sweep is split over warps.  A warp's time is about one unit per
+// round of 32 cells, a third of one per 32 cells converted, and a start-up;
+// 16 warps per SM are resident when a warp's rows stay within 14 KB.  Packing
+// K short columns end to end fills the last round of each column (64 layers
+// alone: 66 cells in 3 rounds, 69 %; five columns: 330 in 11, 94 %);
+// segments of a column spread a few long columns over the SMs (1024 cells of
+// a 1-D block: one CTA took 43 us).
+constexpr size_t kX1RowBytes = 14 * 1024;
+static X1Split x1_split(const Geo& g, int nvt) {
+  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
+  const double resident = 148. * 16.;
+  X1Split best{1, 1, g.nx1, g.nc1};
+  double best_cost = 0.;
+  size_t best_bytes = 0;
+  auto consider = [&](X1Split s, int n, int nn) {
+    const int64_t items = (ncol + s.K - 1) / s.K * s.nseg;
+    const size_t bytes = (size_t)s.pitch * nvt * sizeof(double);
+    const double waves = std::max(1., items / resident + 0.5);
+    const double cost = waves * (1. + (s.K * nn + 31) / 32 + ((s.K * n + 31) / 32) / 3.);
+    const bool fits = bytes <= kX1RowBytes, best_fits = best_bytes <= kX1RowBytes;
+    if (best_bytes == 0 || (fits && !best_fits) ||
+        (fits == best_fits && (fits ? cost < best_cost : bytes < best_bytes))) {
+      best = s;
+      best_cost = cost;
+      best_bytes = bytes;
+    }
+  };
+  for (int K = 1; K <= 8; ++K) consider({K, 1, g.nx1, K * g.nc1}, g.nc1, g.nx1 + 2);
+  for (int want = 2; want <= (g.nx1 + 29) / 30; ++want) {
+    const int S = (g.nx1 + want - 1) / want, nseg = (g.nx1 + S - 1) / S;
+    if (nseg > 1) consider({1, nseg, S, S + g.ng + 3}, S + 6, S + 2);
+  }
+  return best;
 }
 
-cudaError_t launch_x1(const Geo& g, const Phys& p, const StageBufs& b, bool last,
-                      cudaStream_t st) {
-  switch (p.nscalar) {
-    case 0: return launch_x1_t<0>(g, p, b, last, st);
-    case 1: return launch_x1_t<1>(g, p, b, last, st);
-    case 2: return launch_x1_t<2>(g, p, b, last, st);
-    case 3: return launch_x1_t<3>(g, p, b, last, st);
-  }
-  return cudaErrorInvalidValue;
+cudaError_t launch_x1(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
+  const X1Split sp = x1_split(g, 5 + p.nscalar);
+  const int64_t items = ((int64_t)g.nc2 * g.nc3 + sp.K - 1) / sp.K * sp.nseg;
+  const size_t per = (size_t)sp.pitch * (5 + p.nscalar) * sizeof(double);
+  // warps per CTA: four, fewer when the items would not reach every SM
+  int wpc = items >= 148 * 4 ? 4 : (items >= 148 * 2 ? 2 : 1);
+  while (wpc > 1 && wpc * per > 64 * 1024) wpc /= 2;
+  if (per > 200 * 1024) return cudaErrorInvalidConfiguration;
+  return with_profile64(p, 1, [&](auto ns, auto rp, auto sv) {
+    constexpr int NS = decltype(ns)::value, RP = decltype(rp)::value, SV = decltype(sv)::value;
+    raise_smem_limit(k_x1<NS, RP, SV>, 200 * 1024);
+    k_x1<NS, RP, SV><<<(unsigned)((items + wpc - 1) / wpc), 32 * wpc, wpc * per, st>>>(g, p, b, sp,
+                                                                                     items);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_c2p_only(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
@@ -522,35 +285,27 @@ cudaError_t launch_c2p_only(const Geo& g, const Phys& p, const StageBufs& b, cud
   return cudaGetLastError();
 }
 
-template <int NS, int AX>
-static cudaError_t launch_march_t(const Geo& g, const Phys& p, const StageBufs& b, bool first,
-                                  bool last, cudaStream_t st) {
-  int ni = g.iu - g.il + 1;
-  int no = AX == 2 ? g.ku - g.kl + 1 : g.ju - g.jl + 1;
-  int n = AX == 2 ? g.nx2 : g.nx3;
+cudaError_t launch_march(int axis, const Geo& g, const Phys& p, const StageBufs& b, bool first,
+                         bool last, cudaStream_t st) {
+  const int ni = g.iu - g.il + 1;
+  const int no = axis == 2 ? g.ku - g.kl + 1 : g.ju - g.jl + 1;
+  const int n = axis == 2 ? g.nx2 : g.nx3;
   int seglen = 32;
   int64_t threads = (int64_t)ni * no;
   // keep at least ~4 waves of threads on 148 SMs: shorter segments for small grids
   while (seglen > 8 && threads * ((n + seglen - 1) / seglen) < 148LL * 1024 * 2) seglen /= 2;
-  dim3 grid((unsigned)((threads + 127) / 128), (unsigned)((n + seglen - 1) / seglen));
-  k_march<NS, AX><<<grid, 128, 0, st>>>(g, p, b, seglen, first ? 1 : 0, last ? 1 : 0);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_march(int axis, const Geo& g, const Phys& p, const StageBufs& b, bool first,
-                         bool last, cudaStream_t st) {
-#define SNAPB_MARCH(NS)                                                  \
-  case NS:                                                               \
-    return axis == 2 ? launch_march_t<NS, 2>(g, p, b, first, last, st)  \
-                     : launch_march_t<NS, 3>(g, p, b, first, last, st);
-  switch (p.nscalar) {
-    SNAPB_MARCH(0)
-    SNAPB_MARCH(1)
-    SNAPB_MARCH(2)
-    SNAPB_MARCH(3)
-  }
-#undef SNAPB_MARCH
-  return cudaErrorInvalidValue;
+  const dim3 grid((unsigned)((threads + kMarchThreads - 1) / kMarchThreads),
+                  (unsigned)((n + seglen - 1) / seglen));
+  return with_profile64(p, axis, [&](auto ns, auto rp, auto sv) {
+    constexpr int NS = decltype(ns)::value, RP = decltype(rp)::value, SV = decltype(sv)::value;
+    constexpr size_t smem = march_smem_bytes<NS>();
+    static_assert(smem <= 48 * 1024, "march ring");
+    if (axis == 2)
+      k_march<NS, 2, RP, SV><<<grid, kMarchThreads, smem, st>>>(g, p, b, seglen, first, last);
+    else
+      k_march<NS, 3, RP, SV><<<grid, kMarchThreads, smem, st>>>(g, p, b, seglen, first, last);
+    return cudaGetLastError();
+  });
 }
 
 cudaError_t launch_diffusion(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {

@@ -1,0 +1,74 @@
+"""The FP64 sweeps at the sizes where their split changes: segments and packed
+columns of the x1 sweep, remainders of 32-cell rounds, short march segments,
+every compile-time face profile and the run-time one, against the CPU oracle.
+
+One RK3 step of a rough random state; the bound is the per-step one of
+test_gpu_parity.py (1e-12 of each variable's state scale per step)."""
+import numpy as np
+import pytest
+
+from snapy_linfel_b200.config import Integration, MeshBlockOptions, make_config
+
+from errnorm import assert_finite, state_err
+from test_gpu_parity import _run_gpu, _run_oracle, random_prim
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def _check(oracle, nx, seed=3, **kw):
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    ns = kw.get("nscalar", 0)
+    grav = kw.pop("g", -0.2)
+    cfg = make_config(nx1=nx[0], nx2=nx[1], nx3=nx[2], x1=(0.0, 0.1 * nx[0]),
+                      x2=(0.0, 0.1 * nx[1]), x3=(0.0, 0.1 * nx[2]),
+                      grav=(grav if nx[0] > 1 else 0.0, 0.0, 0.0), **kw)
+    opts = MeshBlockOptions(cfg, Integration(cfl=0.3))
+    rng = np.random.default_rng(seed)
+    w = random_prim(rng, cfg.shape)
+    r = rng.random(cfg.scalar_shape) if ns else None
+    dts = [0.01]
+    mb, _ = _run_gpu(opts, w, r, 1, dts=dts)
+    u, s, _ = _run_oracle(oracle, opts, w, r, 1, dts=dts)
+    got = mb.hydro_u.cpu().numpy()
+    assert state_err(got, u, u) < 1e-12  # ghost cells included
+    if ns:
+        gs = mb.scalar_s.cpu().numpy()
+        assert_finite(gs)
+        assert np.max(np.abs(gs - s)) < 1e-12 * np.max(np.abs(s))
+
+
+@pytest.mark.parametrize("nx1", [3, 28, 29, 30, 31, 33, 61, 62, 127, 257, 1500])
+@pytest.mark.parametrize("bc", ["outflow", "reflecting", "periodic"])
+def test_one_dimensional_segments(oracle, nx1, bc):
+    """a column split into segments over warps, ghosts filled by the cells"""
+    _check(oracle, (nx1, 1, 1), shock1=True, bc=(bc,) * 6, nscalar=nx1 % 2,
+           scalar_recon="weno5", g=-0.2 if bc == "reflecting" else 0.0)
+
+
+@pytest.mark.parametrize("nx", [(30, 7, 1), (31, 40, 1), (65, 3, 5), (5, 60, 50), (9, 61, 45),
+                                (33, 50, 50), (64, 52, 48)])
+def test_column_packing_and_remainders(oracle, nx):
+    """whole columns end to end in one warp, and a few long ones"""
+    _check(oracle, nx, riemann="lmars", bc=("reflecting",) * 4 + ("periodic",) * 2)
+
+
+@pytest.mark.parametrize("n2", [3, 7, 8, 9, 33, 64, 65])
+def test_march_segments(oracle, n2):
+    _check(oracle, (6, n2, 4), riemann="roe", bc=("outflow",) * 2 + ("reflecting",) * 4)
+
+
+@pytest.mark.parametrize("riemann", ["lmars", "hllc", "roe"])
+@pytest.mark.parametrize("recon", ["weno5", "shock", "scaled", "plm", "weno3", "cp3", "mixed"])
+@pytest.mark.parametrize("nscalar", [0, 1, 2, 3])
+def test_face_profiles(oracle, riemann, recon, nscalar):
+    kw = {"weno5": dict(scalar_recon="weno5"),
+          "shock": dict(shock1=True, shock23=True, scalar_recon="weno5"),
+          "scaled": dict(scale1=True, scale23=True, scalar_recon="weno5", scalar_scale=True),
+          "plm": dict(recon1="plm", recon23="plm", scalar_recon="plm"),
+          "weno3": dict(recon1="weno3", recon23="weno3", scalar_recon="weno3"),
+          "cp3": dict(recon1="cp3", recon23="cp3", scalar_recon="cp3"),
+          "mixed": dict(recon1="plm", recon23="weno5", scalar_recon="dc")}[recon]
+    _check(oracle, (11, 6, 5), riemann=riemann, nscalar=nscalar,
+           bc=("reflecting",) * 2 + ("periodic",) * 4, **kw)
