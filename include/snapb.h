@@ -297,13 +297,14 @@ typedef struct snapb_member_f32 {
 
 /* tile shapes and kernel variants; 0 = default.  x1_columns: columns per x1
  * tile (a power of two); march_segment: faces per x2/x3 segment; ctas_per_sm:
- * persistent CTAs per SM cap; vic_kernel: the implicit solve (0 the column
- * kernel + finish kernel; 1 block cyclic reduction, one CTA per column, where
- * it applies: 3x3 blocks and columns of at most 256 layers, else 0; 2 the
- * fused kernel: blocks, twisted elimination from both column ends, back
- * substitution and finish in one launch); vic_block: columns per tile of the
- * column kernel (32, 64 or 128); vic_regs: its register budget (0 the
- * compiler's, 1 ~168, 2 128). */
+ * persistent CTAs per SM cap (of 128 threads); vic_kernel: the implicit solve
+ * (0 one warp per group of columns for 3x3 blocks and columns of at most 1216
+ * layers, else the column kernel + finish kernel; 1 block cyclic reduction,
+ * one CTA per column, where it applies: 3x3 blocks and columns of at most 256
+ * layers, else 0; 2 the fused kernel: blocks, twisted elimination from both
+ * column ends, back substitution and finish in one launch); vic_block: columns
+ * per tile of the column kernel (32, 64 or 128); vic_regs: its register budget
+ * (0 the compiler's, 1 ~168, 2 128). */
 typedef struct snapb_ensemble_tuning {
   int32_t x1_columns, march_segment, ctas_per_sm, vic_block, vic_regs, vic_kernel;
 } snapb_ensemble_tuning;

@@ -99,8 +99,8 @@ __global__ void k_fill_u64(unsigned long long* p, int n, unsigned long long v) {
 // host plan
 // ---------------------------------------------------------------------------
 enum Phase {
-  PH_X1 = 0, PH_X1REV, PH_X2, PH_X3, PH_VCOL, PH_VFIN, PH_VFUSED, PH_VCR, PH_BCU, PH_BCS, PH_CFL,
-  PH_COUNT
+  PH_X1 = 0, PH_X1REV, PH_X2, PH_X3, PH_VCOL, PH_VFIN, PH_VFUSED, PH_VCR, PH_VCH8, PH_VCH16,
+  PH_VCH32, PH_BCU, PH_BCS, PH_CFL, PH_COUNT
 };
 
 // vic_kernel values of the tuning: the implicit-solve variants
@@ -121,6 +121,7 @@ struct snapb_ensemble {
   int x1_nc1 = 1;   // longest member column (x1 cells with ghosts): the x1 tile layout
   int vic_kernel = kVicColumn;  // the implicit-solve variant in use
   int max_layers = 0;           // longest member column (cyclic reduction's shared memory)
+  int chunk_max[3] = {0, 0, 0}; // longest column of the members that take 8, 16, 32 lanes
   std::vector<int64_t> prefix[PH_COUNT];
   // device layout (offsets into the bound workspace)
   size_t o_mem = 0, o_prefix = 0, o_counter = 0, o_dts = 0, o_slots = 0, total = 0;
@@ -158,6 +159,15 @@ int plan(snapb_ensemble* e) {
   const auto& t = e->tune;
   e->x1_smem = 0;
   for (auto& v : e->prefix) v.assign(e->M + 1, 0);
+  for (int& x : e->chunk_max) x = 0;
+  // column groups per item of the one-warp implicit solve: a few, to amortise
+  // the queue, while every resident warp still gets about eight items
+  int64_t warps = 0;
+  for (const Member32& mb : e->mem) {
+    const int cw = 32 / vic_chunk_lanes(mb.g.nx1);
+    warps += ((int64_t)(mb.g.ju - mb.g.jl + 1) * (mb.g.ku - mb.g.kl + 1) + cw - 1) / cw;
+  }
+  const int chunk_groups = (int)std::min<int64_t>(8, std::max<int64_t>(1, warps / (e->sms * 64)));
   for (int m = 0; m < e->M; ++m) {
     Member32& mb = e->mem[m];
     const Geo& g = mb.g;
@@ -184,9 +194,19 @@ int plan(snapb_ensemble* e) {
                           ? (ncol1 * 2 * g.ng + kRevisionItem - 1) / kRevisionItem : 0;
     tiles[PH_X2] = e->a2 ? ((lines2 + 127) / 128) * mb.nseg2 : 0;
     tiles[PH_X3] = e->a3 ? ((lines3 + 127) / 128) * mb.nseg3 : 0;
-    tiles[PH_VCOL] = e->p.implicit_scheme ? (ncolv + mb.vic_cols - 1) / mb.vic_cols : 0;
+    // implicit solve, default variant: the one-warp kernel where it applies
+    // (a launch per lane count), else the column + finish pair
+    const bool chunk = vic_chunk_applies(g, e->p), column = e->p.implicit_scheme && !chunk;
+    if (chunk) {
+      const int lanes = vic_chunk_lanes(g.nx1), ph = lanes == 8 ? 0 : (lanes == 16 ? 1 : 2);
+      const int64_t groups = (ncolv + 32 / lanes - 1) / (32 / lanes);
+      mb.chunk_groups = chunk_groups;
+      tiles[PH_VCH8 + ph] = (groups + chunk_groups - 1) / chunk_groups;
+      e->chunk_max[ph] = std::max(e->chunk_max[ph], g.nx1);
+    }
+    tiles[PH_VCOL] = column ? (ncolv + mb.vic_cols - 1) / mb.vic_cols : 0;
     const int fl = vic_finish_layers32(e->p);
-    tiles[PH_VFIN] = e->p.implicit_scheme
+    tiles[PH_VFIN] = column
                          ? ((ncolv + kVicFinishCols - 1) / kVicFinishCols) * ((g.nx1 + fl - 1) / fl)
                          : 0;
     const int fc = vicf_tile_columns();
@@ -275,6 +295,7 @@ PersistGrid pgrid(const snapb_ensemble* e, int ph) {
   g.sms = e->sms;
   g.cap = e->tune.ctas_per_sm;
   g.tiles = e->prefix[ph][e->M];
+  if (ph >= PH_VCH8 && ph <= PH_VCH32) g.cap *= 4;  // CTAs of one warp instead of four
   return g;
 }
 
@@ -446,11 +467,17 @@ int snapb_ensemble_stage_f32(snapb_ensemble* e, int stage, void* stream) {
     } else if (e->vic_kernel == kVicFused) {
       c = launch_vicf_batch(mem, p, queue(e, PH_VFUSED), stage, pgrid(e, PH_VFUSED), st);
     } else {
-      int blk = e->mem.empty() ? 64 : e->mem[0].vic_cols;
-      c = launch_vic_column_batch(mem, p, queue(e, PH_VCOL), stage, pgrid(e, PH_VCOL), blk,
-                                  e->tune.vic_regs, st);
-      if (c == cudaSuccess)
-        c = launch_vic_finish_batch(mem, p, queue(e, PH_VFIN), stage, pgrid(e, PH_VFIN), st);
+      for (int k = 0; k < 3 && c == cudaSuccess; ++k)
+        if (e->prefix[PH_VCH8 + k][e->M])
+          c = launch_vic_chunk_batch(mem, p, queue(e, PH_VCH8 + k), stage, 8 << k,
+                                     e->chunk_max[k], pgrid(e, PH_VCH8 + k), st);
+      if (c == cudaSuccess && e->prefix[PH_VCOL][e->M]) {
+        int blk = e->mem.empty() ? 64 : e->mem[0].vic_cols;
+        c = launch_vic_column_batch(mem, p, queue(e, PH_VCOL), stage, pgrid(e, PH_VCOL), blk,
+                                    e->tune.vic_regs, st);
+        if (c == cudaSuccess)
+          c = launch_vic_finish_batch(mem, p, queue(e, PH_VFIN), stage, pgrid(e, PH_VFIN), st);
+      }
     }
     if (c != cudaSuccess) return cuda_e(c, "ensemble implicit");
   }

@@ -80,7 +80,7 @@ struct Member32 {
   int seglen2, nseg2;    // x2 march: faces per segment, segments
   int seglen3, nseg3;    // x3 march
   int vic_cols;          // columns per implicit-column tile
-  int pad;
+  int chunk_groups;      // column groups per item of the one-warp implicit solve
 };
 
 // Work items of one persistent launch: item k belongs to member m when
@@ -191,6 +191,10 @@ cudaError_t launch_vic_finish_batch(const Member32* mem, const Phys& p, const Wo
 cudaError_t launch_vic_cr32_batch(const Member32* mem, const Phys& p, const WorkQueue& q,
                                   int stage, const PersistGrid& pg, int max_layers,
                                   cudaStream_t st);
+// the members whose columns take `lanes` lanes; max_layers: their longest column
+cudaError_t launch_vic_chunk_batch(const Member32* mem, const Phys& p, const WorkQueue& q,
+                                   int stage, int lanes, int max_layers, const PersistGrid& pg,
+                                   cudaStream_t st);
 // the fused implicit-solve kernel (vicf.cu): one launch per solve, tiles of
 // vicf_tile_columns() columns
 cudaError_t launch_vicf_batch(const Member32* mem, const Phys& p, const WorkQueue& q, int stage,
@@ -300,6 +304,13 @@ cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b,
 cudaError_t launch_diffusion(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_vic(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_vic32(const Geo& g, const Phys& p, const StageBufs32& b, cudaStream_t st);
+// the one-warp implicit solve (vic_chunk.cuh): 3x3 blocks, columns of up to
+// 1216 layers; lanes a column takes, by its length
+bool vic_chunk_applies(const Geo& g, const Phys& p);
+int vic_chunk_lanes(int nl);
+cudaError_t launch_vic_chunk(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
+cudaError_t launch_vic_chunk32(const Geo& g, const Phys& p, const StageBufs32& b,
+                               cudaStream_t st);
 size_t vic_scratch_bytes(const Geo& g, const Phys& p);
 size_t vic_column_scratch_bytes(const Geo& g, const Phys& p);
 size_t vicf_scratch_bytes(const Geo& g, const Phys& p);

@@ -1,4 +1,6 @@
-// vic.cu — vertically implicit correction (VIC) of one RK stage, FP64.
+// vic.cu — vertically implicit correction (VIC) of one RK stage: the choice of
+// the solver, and the column sweep for 5x5 blocks, very long columns and the
+// entry point without workspace (the rest takes vic_chunk.cuh).
 //
 // Two kernels per solve:
 //   k_vic_column    one thread per x1 column (x1 is the vertical axis): the
@@ -1059,10 +1061,16 @@ static cudaError_t launch_vic_n(const Geo& g, const Phys& p, const B& b, cudaStr
   return cudaGetLastError();
 }
 
-// Variant of the implicit solve, from the environment (read at every launch):
-// the column + finish pair by default; SNAPB_VIC_KERNEL=fused selects the
-// fused kernel of vicf.cu, =cr block cyclic reduction (vic_cr.cu, FP32 form,
-// where it applies).
+// Variant of the implicit solve, from the environment (read at every launch).
+// By default the one-warp kernel (vic_chunk.cuh) where it applies (3x3 blocks,
+// columns of at most 1216 layers) and the column + finish pair elsewhere;
+// SNAPB_VIC_KERNEL=column selects the pair everywhere, =fused the fused kernel
+// of vicf.cu, =cr block cyclic reduction (vic_cr.cu, FP32 form, where it
+// applies).  The one-warp kernel was the faster at every size measured, ms per
+// stage before (pair) and after: FP64, 512 x 256 columns x layers 0.241 ->
+// 0.017, 128^3 0.327 -> 0.190, 384 x 384 x 192 with two tracers 4.38 -> 3.00;
+// FP32, 512 x 256 0.238 -> 0.017, 384 x 384 x 192 3.58 -> 2.49, 48 members of
+// 64 and 128 layers 4.30 -> 4.00.
 static const char* vic_kernel_env() {
   const char* v = std::getenv("SNAPB_VIC_KERNEL");
   return v ? v : "";
@@ -1078,12 +1086,16 @@ cudaError_t launch_vic_column(const Geo& g, const Phys& p, const StageBufs& b,
 
 cudaError_t launch_vic(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
   if (vic_fused_selected()) return launch_vicf(g, p, b, st);
+  if (vic_chunk_applies(g, p) && std::strcmp(vic_kernel_env(), "column") != 0)
+    return launch_vic_chunk(g, p, b, st);
   return launch_vic_column(g, p, b, st);
 }
 
 cudaError_t launch_vic32(const Geo& g, const Phys& p, const StageBufs32& b, cudaStream_t st) {
   if (vic_fused_selected()) return launch_vicf32(g, p, b, st);
   if (vic_cr_selected() && vic_cr_applies(g, p)) return launch_vic_cr32(g, p, b, st);
+  if (vic_chunk_applies(g, p) && std::strcmp(vic_kernel_env(), "column") != 0)
+    return launch_vic_chunk32(g, p, b, st);
   if (vic_n(p) == 5) return launch_vic_n<5>(g, p, b, st);
   return launch_vic_n<3>(g, p, b, st);
 }

@@ -1,0 +1,561 @@
+// vic_chunk.cuh — the vertically implicit correction with 3x3 blocks, one warp
+// per group of columns: blocks, block-tridiagonal solve, mass redistribution
+// and RK combination in one kernel, with nothing of the solve in HBM.
+//
+// A column's nl layers are cut into G chunks of m layers, one lane each
+// (32 / G columns a warp).  A lane eliminates its chunk's first m - 1 layers
+// downwards, which expresses them by the last layer of the chunk below (y-)
+// and by its own last layer (y):
+//     x_j = p_j - A'_j x_{j+1} - f_j y-          (kept in shared memory)
+//     x_0 = P - Q y - S y-                       (carried in registers)
+// The G last layers then form a block-tridiagonal system of their own, solved
+// by parallel cyclic reduction across the lanes (shuffles), and each lane
+// substitutes back.  Against the sequential sweep (one thread per column) a
+// layer costs 3 to 4 times the FP64 operations, but its chain is m layers and
+// log2 G reductions long instead of nl layers, the reduced blocks (96 B a
+// layer, written and read back through HBM by the sweep) stay in shared
+// memory, and the finish needs no pass of its own.
+//
+// Bound: instruction issue (about half of it FP64) at 8 resident warps per SM
+// (registers).  48 members of 64 and 128 layers, FP32 form: chunks of four
+// layers 4.0 ms a stage, of eight 4.75 (twice the shared memory, so five
+// warps); a budget of 168 registers for 12 warps spills, 5.4; the reduction
+// unrolled over its five levels 5.3 (instruction cache); the finish's inputs
+// fetched before the reduction instead of after it 4.5 -> 4.0.
+#pragma once
+
+#include <type_traits>
+
+#include "kernels.cuh"
+#include "vic_blocks.cuh"
+#include "vic_common.cuh"
+
+namespace snapb {
+
+// Precision of the blocks (|A|, J and the assembled a, b, c): FP64 for the
+// FP64 form, FP32 for the FP32 perturbation form, whose states are FP32; the
+// elimination is FP64 in both.
+template <class B>
+using ChunkBlockT = std::conditional_t<std::is_same_v<B, StageBufs32>, float, double>;
+
+constexpr int kChunkElems = 21;  // p, A', f of a layer
+__host__ __device__ constexpr size_t chunk_smem_bytes(int m) {
+  return (((size_t)(m - 1) * kChunkElems + 3) * 32 + 4) * sizeof(double) + 4 * sizeof(int);
+}
+
+// Lanes per column: chunks of two to four layers up to 128 layers, longer ones
+// above (one warp per column at most).  By the column length alone, so that a
+// block gives the same bits alone and in an ensemble.
+inline int chunk_lanes(int nl) { return nl <= 32 ? 8 : (nl <= 64 ? 16 : 32); }
+inline int chunk_layers(int nl) {
+  const int G = chunk_lanes(nl);
+  return (nl + G - 1) / G;
+}
+// Chunks whose layers fit in one CTA's shared memory (columns of up to 1216
+// layers); the 5x5 form keeps the column sweep.
+inline bool chunk_applies(const Geo& g, const Phys& p) {
+  return p.implicit_scheme != 0 && vic_n(p) == 3 &&
+         chunk_smem_bytes(chunk_layers(g.nx1)) <= 200 * 1024;
+}
+
+__device__ __forceinline__ double chunk_rsqrt(double x) { return rsqrt(x); }
+__device__ __forceinline__ float chunk_rsqrt(float x) { return rsqrtf(x); }
+// A product that is never contracted into a following sum.  Every contraction
+// below is spelled out with mul and fma: the one-block and the batched kernels
+// must round alike, and the compiler's own choice depends on the code around.
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+
+// What a cell gives to its two faces and to its Jacobian.
+template <class T>
+struct ChunkCell {
+  T u, v, w, sd, ke, hp, H;  // velocities, sqrt(rho), kinetic energy, enthalpy parts
+  __device__ __forceinline__ void set(T rho, T vx, T vy, T vz, T p, T gog) {
+    const T is = chunk_rsqrt(rho);
+    u = vx;
+    v = vy;
+    w = vz;
+    sd = mul(rho, is);
+    hp = mul(mul(gog, p), mul(is, is));
+    ke = mul(T(0.5), fma(vx, vx, fma(vy, vy, mul(vz, vz))));
+    H = hp + ke;
+  }
+};
+
+// s |A| of the face between two cells: the rows and columns (IDN, IVX, IPR) of
+// R |Lambda| R^-1 at the Roe average (absA_block), with the sums over the
+// acoustic waves written out: hp = H - ke is c^2 / (gamma - 1), so one
+// reciprocal square root gives c, 1 / c and 1 / hp.
+template <class T>
+__device__ __forceinline__ void chunk_abs_a(const ChunkCell<T>& l, const ChunkCell<T>& r, T gm1,
+                                            T s, T (&A)[3][3]) {
+  const T isd = fdiv(T(1), l.sd + r.sd), a = mul(l.sd, isd), b = mul(r.sd, isd);
+  const T u = fma(a, l.u, mul(b, r.u)), v = fma(a, l.v, mul(b, r.v));
+  const T w = fma(a, l.w, mul(b, r.w)), H = fma(a, l.H, mul(b, r.H));
+  const T vw = fma(v, v, mul(w, w)), ke = mul(T(0.5), fma(u, u, vw));
+  const T hp = H - ke, c2 = mul(gm1, hp);
+  const T ic = chunk_rsqrt(c2), c = mul(c2, ic), ihp = mul(gm1, mul(ic, ic));
+  const T k = mul(mul(T(0.5), ic), ihp), i2hp = mul(T(0.5), ihp);
+  const T lm = mul(s, fabs(u - c)), l0 = mul(s, fabs(u)), lp = mul(s, fabs(u + c));
+  const T cke = mul(c, ke), uhp = mul(u, hp), cu = mul(c, u);
+  const T lmk = mul(lm, k), lpk = mul(lp, k), l0i = mul(l0, ihp);
+  const T Lm[3] = {mul(lmk, cke + uhp), -mul(lmk, hp + cu), mul(lm, i2hp)};
+  const T L0[3] = {mul(l0i, hp - ke), mul(l0i, u), -l0i};
+  const T Lp[3] = {mul(lpk, cke - uhp), mul(lpk, hp - cu), mul(lp, i2hp)};
+#pragma unroll
+  for (int q = 0; q < 3; ++q) {
+    const T sum = Lm[q] + Lp[q], cd = mul(c, Lp[q] - Lm[q]);
+    A[0][q] = sum + L0[q];
+    A[1][q] = fma(u, A[0][q], cd);
+    A[2][q] = fma(H, sum, fma(u, cd, mul(ke, L0[q])));
+  }
+  A[2][0] = fma(-l0, vw, A[2][0]);
+}
+
+// s dF/dU of a cell (jac_block)
+template <class T>
+__device__ __forceinline__ void chunk_jac(const ChunkCell<T>& c, T gm1, T s, T (&J)[3][3]) {
+  const T su = mul(s, c.u), uu = mul(c.u, c.u);
+  J[0][0] = T(0);
+  J[0][1] = s;
+  J[0][2] = T(0);
+  J[1][0] = mul(s, fma(gm1, c.ke, -uu));
+  J[1][1] = mul(T(2) - gm1, su);
+  J[1][2] = mul(s, gm1);
+  J[2][0] = mul(fma(gm1 - T(1), c.ke, -c.hp), su);
+  J[2][1] = mul(s, fma(-gm1, uu, c.H));
+  J[2][2] = mul(gm1 + T(1), su);
+}
+
+// C -= X Y, c -= X y (three fused operations an entry, no separate sum)
+__device__ __forceinline__ void sub_mul3(const double (&X)[3][3], const double (&Y)[3][3],
+                                         double (&C)[3][3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      C[r][q] = fma(-X[r][2], Y[2][q], fma(-X[r][1], Y[1][q], fma(-X[r][0], Y[0][q], C[r][q])));
+}
+__device__ __forceinline__ void sub_mul3(const double (&X)[3][3], const double (&y)[3],
+                                         double (&c)[3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    c[r] = fma(-X[r][2], y[2], fma(-X[r][1], y[1], fma(-X[r][0], y[0], c[r])));
+}
+// Z = X Y, z = X y, Z = -X Y
+__device__ __forceinline__ void mul3(const double (&X)[3][3], const double (&Y)[3][3],
+                                     double (&Z)[3][3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      Z[r][q] = fma(X[r][2], Y[2][q], fma(X[r][1], Y[1][q], mul(X[r][0], Y[0][q])));
+}
+__device__ __forceinline__ void mul3(const double (&X)[3][3], const double (&y)[3],
+                                     double (&z)[3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r) z[r] = fma(X[r][2], y[2], fma(X[r][1], y[1], mul(X[r][0], y[0])));
+}
+__device__ __forceinline__ void neg_mul3(const double (&X)[3][3], const double (&Y)[3][3],
+                                         double (&Z)[3][3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      Z[r][q] = fma(-X[r][2], Y[2][q], fma(-X[r][1], Y[1][q], mul(-X[r][0], Y[0][q])));
+}
+// cofactor inverse (inverse3, vic_blocks.cuh)
+__device__ __forceinline__ void chunk_inverse(const double (&M)[3][3], double (&inv)[3][3]) {
+  double cof[3][3];
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) {
+      const int i1 = (i + 1) % 3, i2 = (i + 2) % 3, j1 = (j + 1) % 3, j2 = (j + 2) % 3;
+      cof[i][j] = fma(M[i1][j1], M[i2][j2], -mul(M[i1][j2], M[i2][j1]));
+    }
+  const double id =
+      1. / fma(cof[2][0], M[2][0], fma(cof[1][0], M[1][0], mul(cof[0][0], M[0][0])));
+#pragma unroll
+  for (int i = 0; i < 3; ++i)
+#pragma unroll
+    for (int j = 0; j < 3; ++j) inv[i][j] = mul(cof[j][i], id);
+}
+// the values of lane d of the column
+template <int G>
+__device__ __forceinline__ void shfl3(const double (&X)[3][3], int d, double (&Y)[3][3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+      Y[r][q] = __shfl_sync(0xffffffffu, X[r][q], d, G);
+}
+template <int G>
+__device__ __forceinline__ void shfl3(const double (&x)[3], int d, double (&y)[3]) {
+#pragma unroll
+  for (int r = 0; r < 3; ++r)
+    y[r] = __shfl_sync(0xffffffffu, x[r], d, G);
+}
+
+// The columns col0 .. col0 + 32/G - 1 of a block by one warp; sm: the warp's
+// chunk_smem_bytes(m).  Ends with the warp's shared memory still in use by
+// other lanes: the caller synchronizes the warp before the next group.
+template <int G, int NS, class B>
+__device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& b, int64_t col0,
+                                          int m, double* sm) {
+  using T = std::remove_pointer_t<decltype(b.u)>;  // stored precision
+  using BT = ChunkBlockT<B>;
+  constexpr int CW = 32 / G;
+  const int lane = threadIdx.x & 31, k = lane & (G - 1), cw = lane / G;
+  // (element indices of every array stay below 2^31: check_config)
+  const int sv = (int)g.sv, nl = g.nx1, l0 = k * m;
+  const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
+  const int cb = (int)column_base(g, min(col0 + cw, ncol - 1));
+  double* mine = sm + lane;  // element e of layer j at mine[(j * kChunkElems + e) * 32]
+  double* backs = sm + ((size_t)(m - 1) * kChunkElems + 3) * 32;  // [4], then the columns' cb
+  int* cbs = reinterpret_cast<int*>(backs + 4);
+
+  const BT gm1 = (BT)(p.gammad - 1.), gog = (BT)(p.gammad / (p.gammad - 1.));
+  const double dt = *b.dt, idtd = 1. / dt;
+  const BT s = (BT)g.A1 * (BT)(0.5 / g.vol), idt = (BT)idtd, grav = (BT)p.grav1;
+
+  // state of layer l (clamped to the ghost above the column), as stored
+  auto load_w = [&](int l, T (&raw)[5]) {
+    const int o = cb + min(l, nl);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) raw[v] = b.w[v * sv + o];
+  };
+  auto load_d = [&](int l, T (&raw)[3]) {
+    const int o = cb + min(l, nl - 1);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) raw[r] = b.D[sel<3>(r) * sv + o];
+  };
+  // full density of the layer (returned in FP64) and its cell quantities
+  auto make = [&](int l, const T (&raw)[5], ChunkCell<BT>& c) {
+    const int xi = g.il + min(l, nl);
+    const double rho = vic_full(b, (double)raw[IDN], IDN, xi);
+    c.set((BT)rho, (BT)raw[IVX], (BT)raw[IVY], (BT)raw[IVZ], vic_full_blk(b, raw[IPR], IPR, xi),
+          gog);
+    return rho;
+  };
+
+  // ---- elimination inside the chunk ----
+  double Ap[3][3] = {}, f[3][3] = {}, pv[3] = {};           // A', f, p of the layer below
+  double Q[3][3] = {}, S[3][3] = {}, P[3] = {};             // first layer's relation
+#pragma unroll
+  for (int r = 0; r < 3; ++r) f[r][r] = Q[r][r] = -1.;      // (none yet: x_0 = x_0)
+  double sum_r2 = 0., sum_du = 0.;
+  double a[3][3], bl[3][3], c[3][3], rhs[3];                // the layer's equation
+  {
+    T rawn[5], rawd[3];
+    ChunkCell<BT> cc, cn;
+    BT Af[3][3], bf[3][3], Jc[3][3];  // s|A| of the lower face, b of the layer, sJ of its cell
+    double rc, rn;
+    {
+      BT Jp[3][3];
+      load_w(l0 - 1, rawn);
+      T raw0[5];
+      load_w(l0, raw0);
+      load_d(l0, rawd);
+      make(l0 - 1, rawn, cn);
+      load_w(l0 + 1, rawn);
+      rc = make(l0, raw0, cc);
+      chunk_abs_a(cn, cc, gm1, s, Af);
+      chunk_jac(cn, gm1, s, Jp);
+      chunk_jac(cc, gm1, s, Jc);
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) bf[r][q] = -(Af[r][q] + Jp[r][q]);
+    }
+    for (int j = 0;; ++j) {
+      const int l = l0 + j;
+      rn = make(l + 1, rawn, cn);
+      double du[3];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) du[r] = (double)rawd[r];
+      if (j < m - 1) {  // the next layer's inputs, ahead of this one's arithmetic
+        load_w(l + 2, rawn);
+        load_d(l + 1, rawd);
+      }
+      BT An[3][3], Jn[3][3];
+      chunk_abs_a(cc, cn, gm1, s, An);
+      chunk_jac(cn, gm1, s, Jn);
+      // a, b, c with the boundary folds of the first and last layers; layers
+      // past the column's end are x = 0
+      const bool real = l < nl, first = l == 0, last = l == nl - 1;
+      BT af[3][3], bv[3][3], cv[3][3];
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          BT av = Af[r][q] + An[r][q];
+          if ((r == 1 && q == 0) || (r == 2 && q == 1)) av -= grav;
+          if (r == q) av += idt;
+          af[r][q] = av;
+          bv[r][q] = bf[r][q];
+          cv[r][q] = Jn[r][q] - An[r][q];
+          bf[r][q] = -(An[r][q] + Jc[r][q]);  // b of the layer above
+          Af[r][q] = An[r][q];
+          Jc[r][q] = Jn[r][q];
+        }
+      }
+      if (first || l >= nl - 1) {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            if (first) af[r][q] += q == 1 ? -bv[r][q] : bv[r][q];
+            if (last) af[r][q] += q == 1 ? -cv[r][q] : cv[r][q];
+            if (first || !real) bv[r][q] = BT(0);
+            if (last || !real) cv[r][q] = BT(0);
+            if (!real) af[r][q] = r == q ? BT(1) : BT(0);
+          }
+          if (!real) du[r] = 0.;
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          a[r][q] = (double)af[r][q];
+          bl[r][q] = (double)bv[r][q];
+          c[r][q] = (double)cv[r][q];
+        }
+        rhs[r] = mul(du[r], idtd);
+      }
+      if (real) {
+        sum_r2 = fma(rc, rc, sum_r2);
+        sum_du += du[0];
+      }
+      cc = cn;
+      rc = rn;
+      if (j == m - 1) break;
+      double inv[3][3], t33[3][3];
+      if (j > 0) {
+        sub_mul3(bl, Ap, a);
+        sub_mul3(bl, pv, rhs);
+        mul3(bl, f, t33);
+      } else {
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) t33[r][q] = -bl[r][q];
+      }
+      chunk_inverse(a, inv);
+      mul3(inv, c, Ap);
+      mul3(inv, rhs, pv);
+      neg_mul3(inv, t33, f);
+      double* out = mine + (size_t)j * kChunkElems * 32;
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        out[r * 32] = pv[r];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          out[(3 + r * 3 + q) * 32] = Ap[r][q];
+          out[(12 + r * 3 + q) * 32] = f[r][q];
+        }
+      }
+      if (j > 0) {
+        sub_mul3(Q, pv, P);
+        sub_mul3(Q, f, S);
+        neg_mul3(Q, Ap, t33);
+#pragma unroll
+        for (int r = 0; r < 3; ++r)
+#pragma unroll
+          for (int q = 0; q < 3; ++q) Q[r][q] = t33[r][q];
+      } else {
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          P[r] = pv[r];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) {
+            Q[r][q] = Ap[r][q];
+            S[r][q] = f[r][q];
+          }
+        }
+      }
+    }
+  }
+
+  // The finish's inputs of the lane's first IT cells, fetched before the
+  // reduction so that it hides their latency; further ones batch by batch.
+  constexpr int IT = sizeof(T) == 4 ? (NS == 0 ? 4 : 2) : (NS == 0 ? 2 : 1), NSA = NS > 0 ? NS : 1;
+  const bool du_only = b.vic_du_only, stage0 = b.stage == 0;
+  const int total = (int)min((int64_t)CW, ncol - col0) * nl;
+  const int magic = (65536 + m - 1) / m;  // l / m = l * magic >> 16 (l m < 65536)
+  T rho[IT], et[IT], dv[IT][2], uo[IT][5], u0o[IT][5];
+  T so[IT][NSA], s0o[IT][NSA], ro[IT][NSA], dso[IT][NSA];
+  auto place = [&](int idx, int& c, int& l) {  // column and layer of a cell of the warp
+    c = 0;
+#pragma unroll
+    for (int q = 1; q < CW; ++q) c += idx >= q * nl;
+    l = idx - c * nl;
+  };
+  if (k == 0) cbs[cw] = cb;
+  __syncwarp();
+  auto fetch = [&](int i0) {
+#pragma unroll
+    for (int q = 0; q < IT; ++q) {
+      int cc, l;
+      place(min(i0 + 32 * q, total - 1), cc, l);
+      const int off = (CW > 1 ? cbs[cc] : cb) + l;
+      rho[q] = b.w[IDN * sv + off];
+      et[q] = b.D[IDN * sv + off];
+      if (du_only) continue;
+      dv[q][0] = b.D[IVY * sv + off];
+      dv[q][1] = b.D[IVZ * sv + off];
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        uo[q][v] = b.u[v * sv + off];
+        u0o[q][v] = stage0 ? T(0) : b.u0[v * sv + off];
+      }
+#pragma unroll
+      for (int n = 0; n < NS; ++n) {
+        const int o = n * sv + off;
+        so[q][n] = b.s[o];
+        s0o[q][n] = stage0 ? T(0) : b.s0[o];
+        ro[q][n] = b.r[o];
+        dso[q][n] = b.D[(5 + n) * sv + off];
+      }
+    }
+  };
+  auto emit = [&](int i0) {
+#pragma unroll
+    for (int q = 0; q < IT; ++q) {
+      if (i0 + 32 * q >= total) break;
+      int cc, l;
+      place(i0 + 32 * q, cc, l);
+      const int ch = l * magic >> 16, j = l - ch * m, xi = g.il + l;
+      const double* at = sm + j * kChunkElems * 32 + cc * G + ch;
+      const double rhok = vic_full(b, (double)rho[q], IDN, xi);
+      const double fix = at[0] - (double)et[q];
+      const double du0 = fma(mul(rhok, rhok), backs[cc], at[0]);
+      const int off = (CW > 1 ? cbs[cc] : cb) + l;
+      if (b.M) b.M[off] = fix;
+      if (du_only) {
+        vic_set_d(b, IDN * sv + off, du0);
+        vic_set_d(b, IVX * sv + off, at[32]);
+        vic_set_d(b, IPR * sv + off, at[64]);
+        continue;
+      }
+      const double du[5] = {du0, at[32], (double)dv[q][0], (double)dv[q][1], at[64]};
+      double unew_rho = 0.;
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        const double un = vic_rk_from(b.u, b.u0, v * sv + off, stage0, uo[q][v], u0o[q][v], b.wgt0,
+                                      b.wgt1, b.wgt2, du[v]);
+        if (v == IDN) unew_rho = vic_full_rho(b, un, xi);
+      }
+#pragma unroll
+      for (int n = 0; n < NS; ++n) {
+        const int o = n * sv + off;
+        const double ds = fma(fix, (double)ro[q][n], (double)dso[q][n]);
+        const double sn = vic_rk_from(b.s, b.s0, o, stage0, so[q][n], s0o[q][n], b.wgt0, b.wgt1,
+                                      b.wgt2, ds);
+        b.r[o] = sn / unew_rho;
+      }
+    }
+  };
+  fetch(lane);
+
+  // ---- the system of the chunks' last layers ----
+  double Bm[3][3], Cm[3][3], y[3];
+  {
+    double Pn[3], Qn[3][3], Sn[3][3], inv[3][3], t33[3][3];
+    shfl3<G>(P, k + 1, Pn);
+    shfl3<G>(Q, k + 1, Qn);
+    shfl3<G>(S, k + 1, Sn);  // (the last chunk's c is zero)
+    sub_mul3(bl, Ap, a);
+    sub_mul3(c, Sn, a);
+    sub_mul3(bl, pv, rhs);
+    sub_mul3(c, Pn, rhs);
+    chunk_inverse(a, inv);
+    mul3(inv, rhs, y);
+    mul3(bl, f, t33);
+    neg_mul3(inv, t33, Bm);
+    mul3(c, Qn, t33);
+    neg_mul3(inv, t33, Cm);
+  }
+  // y_k + B y_{k-h} + C y_{k+h} = r, strides h = 1, 2, 4, ...: a chunk without
+  // a neighbour at that distance has a zero block there, so the values that the
+  // shuffle wraps around to do not enter
+  auto reduce = [&](int h, bool more) {
+    double D[3][3] = {}, Xu[3][3], Xd[3][3], xu[3], xd[3], inv[3][3], Bn[3][3], Cn[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) D[r][r] = 1.;
+    shfl3<G>(Cm, k - h, Xu);
+    shfl3<G>(Bm, k + h, Xd);
+    sub_mul3(Bm, Xu, D);
+    sub_mul3(Cm, Xd, D);
+    shfl3<G>(y, k - h, xu);
+    shfl3<G>(y, k + h, xd);
+    sub_mul3(Bm, xu, y);
+    sub_mul3(Cm, xd, y);
+    if (more) {
+      shfl3<G>(Bm, k - h, Xu);
+      shfl3<G>(Cm, k + h, Xd);
+      mul3(Bm, Xu, Bn);
+      mul3(Cm, Xd, Cn);
+    }
+    chunk_inverse(D, inv);
+    double t[3];
+    mul3(inv, y, t);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) y[r] = t[r];
+    if (more) {
+      neg_mul3(inv, Bn, Bm);
+      neg_mul3(inv, Cn, Cm);
+    }
+  };
+  // (kept a loop: unrolled, its five copies overran the instruction cache)
+#pragma unroll 1
+  for (int h = 1; 2 * h < G; h *= 2) reduce(h, true);
+  reduce(G / 2, false);
+
+  // ---- back substitution; x takes the place of p ----
+  double ym[3], x[3];
+  shfl3<G>(y, k - 1, ym);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    if (k == 0) ym[r] = 0.;
+    x[r] = y[r];
+    mine[((size_t)(m - 1) * kChunkElems + r) * 32] = x[r];
+  }
+  double sum_x = l0 + m - 1 < nl ? x[0] : 0.;
+  for (int j = m - 2; j >= 0; --j) {
+    double* at = mine + (size_t)j * kChunkElems * 32;
+    double t[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      t[r] = at[r * 32];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(12 + r * 3 + q) * 32], ym[q], t[r]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(3 + r * 3 + q) * 32], x[q], t[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) at[r * 32] = x[r] = t[r];
+    if (l0 + j < nl) sum_x += x[0];
+  }
+
+  // ---- mass redistribution factor of the column: sum(du - x) / sum(rho^2) ----
+  double lost = sum_du - sum_x;
+#pragma unroll
+  for (int h = 1; h < G; h *= 2) {
+    lost += __shfl_xor_sync(0xffffffffu, lost, h, G);
+    sum_r2 += __shfl_xor_sync(0xffffffffu, sum_r2, h, G);
+  }
+  if (k == 0) backs[cw] = lost / sum_r2;
+  __syncwarp();
+
+  // ---- finish: the warp's cells along x1 ----
+  for (int i0 = lane;;) {
+    emit(i0);
+    i0 += 32 * IT;
+    if (i0 - lane >= total) break;
+    fetch(i0);
+  }
+}
+
+}  // namespace snapb

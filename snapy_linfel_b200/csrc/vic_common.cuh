@@ -66,13 +66,14 @@ __device__ __forceinline__ void vic_set_d(const StageBufs32& b, int64_t idx, dou
 // RK combination of one stored value (u' for the FP32 form: the reference
 // part of u is constant in time, so the combination is the same), from
 // values already loaded (qo = q[o], q0o = q0[o] when stage > 0); the stored
-// q keeps the stored precision
+// q keeps the stored precision.  The contraction is spelled out: the one-block
+// and the batched kernels must round alike.
 __device__ __forceinline__ double vic_rk_from(double* q, double* q0, int64_t o, bool first,
                                               double qo, double q0o, double w0, double w1,
                                               double w2, double d) {
   double q0v = first ? qo : q0o;
   if (first) q0[o] = qo;
-  double qn = w0 * q0v + w1 * qo + w2 * d;
+  double qn = fma(w2, d, fma(w1, qo, w0 * q0v));
   q[o] = qn;
   return qn;
 }
@@ -81,7 +82,7 @@ __device__ __forceinline__ double vic_rk_from(float* q, float* q0, int64_t o, bo
                                               double w2, double d) {
   double q0v = first ? qo : q0o;
   if (first) q0[o] = (float)qo;
-  float qn = (float)(w0 * q0v + w1 * qo + w2 * d);
+  float qn = (float)fma(w2, d, fma(w1, qo, w0 * q0v));
   q[o] = qn;
   return qn;
 }

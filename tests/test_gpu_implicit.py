@@ -1,0 +1,114 @@
+"""The one-warp implicit solve (3x3 blocks) at the column lengths where its
+split changes: 8, 16 and 32 lanes a column, chunks of one layer and of many,
+chunks past the column's end, warps with columns missing, and the longest
+column it takes.
+
+FP64: the correction and the mass fix against the CPU oracle, bound 1e-12 of
+the state scale per call (test_gpu_parity.py).  FP32 form: against the column
+sweep (SNAPB_VIC_KERNEL=column), which forms the same FP32 blocks with other
+roundings and eliminates in FP64 too; bound 1e-5 of each variable's scale, the
+form's own accuracy target.  Ensembles: every member bit for bit its one-block
+result, members of all three lane counts together."""
+import ctypes
+
+import numpy as np
+import pytest
+
+from snapy_linfel_b200 import problems
+from snapy_linfel_b200.config import Integration, MeshBlockOptions, make_config
+
+from errnorm import assert_finite, state_err, state_scale
+from test_gpu_parity import call, dev, random_prim
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def L():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from snapy_linfel_b200 import _lib
+
+    return _lib
+
+
+def _config(nl, nx2, nx3, **kw):
+    return make_config(nx1=nl, nx2=nx2, nx3=nx3, x1=(0.0, 0.1 * nl), x2=(0.0, 0.1 * nx2),
+                       x3=(0.0, 0.1 * nx3), grav=(-0.2, 0.0, 0.0), implicit_scheme=1,
+                       bc=("reflecting",) * 4 + ("periodic",) * 2, **kw)
+
+
+@pytest.mark.parametrize("nl,nx2,nx3", [
+    (3, 5, 1), (7, 3, 3), (8, 4, 1), (9, 5, 5), (31, 3, 1), (32, 7, 1), (33, 3, 1), (63, 5, 1),
+    (64, 4, 3), (65, 3, 1), (100, 3, 3), (127, 3, 1), (128, 5, 1), (129, 3, 1), (192, 3, 1),
+    (257, 3, 1), (1216, 3, 1), (1217, 3, 1)])
+def test_correction_matches_oracle(L, oracle, nl, nx2, nx3):
+    c = _config(nl, nx2, nx3)
+    rng = np.random.default_rng(nl)
+    w = random_prim(rng, c.shape)
+    u = oracle.prim2cons(c, w)
+    du = 0.05 * (rng.random(c.shape) - 0.5)
+    dt = 0.05
+    ref, m_ref = du.copy(), np.zeros_like(u)
+    oracle.implicit_correction(c, dt, ref, w, m_ref)
+    ws = torch.empty(L.lib().snapb_workspace_size(ctypes.byref(c)), dtype=torch.uint8,
+                     device="cuda")
+    dug, wg, mg = dev(du), dev(w), torch.zeros(c.shape, dtype=torch.float64, device="cuda")
+    dtg = torch.tensor([dt], dtype=torch.float64, device="cuda")
+    call(L, "snapb_implicit_correction", ctypes.byref(c), L.ptr(dtg), L.ptr(dug), L.ptr(wg),
+         L.ptr(mg), L.ptr(ws), ctypes.c_size_t(ws.numel()), L.stream_ptr())
+    it = c.interior()
+    full = (slice(None),) + it
+    assert state_err(dug.cpu().numpy()[full], ref[full], u[full]) < 1e-12
+    got = mg.cpu().numpy()[0][it]
+    assert_finite(got)
+    assert np.max(np.abs(got - m_ref[0][it])) < 1e-12 * np.max(np.abs(u[0]))
+
+
+@pytest.mark.parametrize("form", ["fp64", "fp32"])
+@pytest.mark.parametrize("nl,nx2,nx3,ns", [(5, 9, 1, 0), (20, 6, 7, 2), (50, 5, 3, 1),
+                                           (64, 9, 1, 3), (150, 4, 3, 2), (128, 6, 5, 0)])
+def test_step_matches_column_sweep(L, monkeypatch, form, nl, nx2, nx3, ns):
+    from snapy_linfel_b200.mesh import MeshBlock, MeshBlockF32
+
+    c = _config(nl, nx2, nx3, nscalar=ns, scalar_recon="weno5", riemann="roe")
+    opts = MeshBlockOptions(c, Integration(cfl=0.3))
+    rng = np.random.default_rng(nl)
+    w, r = random_prim(rng, c.shape), rng.random(c.scalar_shape) if ns else None
+    out = []
+    for env in ("", "column"):
+        monkeypatch.setenv("SNAPB_VIC_KERNEL", env)
+        mb = (MeshBlock if form == "fp64" else MeshBlockF32)(opts)
+        mb.initialize(w, r)
+        mb.step(0.01)
+        mb.step(0.01)
+        torch.cuda.synchronize()
+        out.append((mb.hydro_u.double().cpu().numpy(),
+                    mb.scalar_s.double().cpu().numpy() if ns else None))
+    tol = 1e-12 * 2 if form == "fp64" else 1e-5
+    (a, sa), (b, sb) = out
+    assert_finite(a, b)
+    scale = np.maximum(state_scale(b), 1e-3)
+    assert np.all(np.abs(a - b).reshape(5, -1).max(axis=1) < tol * scale)
+    if ns:
+        assert_finite(sa, sb)
+        assert np.max(np.abs(sa - sb)) < tol * np.max(np.abs(sb))
+
+
+def test_ensemble_of_all_lane_counts_is_exact(L):
+    from snapy_linfel_b200.ensemble import Ensemble
+    from snapy_linfel_b200.mesh import MeshBlockF32
+
+    members = problems.ensemble_members(n=9, seed=5, horiz=(6, 9, 13), vert=(20, 45, 100),
+                                        riemann="hllc")
+    assert {m[0].hydro.nx1 for m in members} == {20, 45, 100}
+    ens = Ensemble(members)
+    for _ in range(2):
+        ens.step()
+    for (opts, w, r), b in zip(members, ens.blocks):
+        mb = MeshBlockF32(opts)
+        mb.initialize(w, r)
+        for _ in range(2):
+            mb.step()
+        assert torch.equal(mb.hydro_u, b.hydro_u)
