@@ -311,6 +311,9 @@ int vic_chunk_lanes(int nl);
 cudaError_t launch_vic_chunk(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 cudaError_t launch_vic_chunk32(const Geo& g, const Phys& p, const StageBufs32& b,
                                cudaStream_t st);
+// the 5x5 solve of the FP64 form (vic_pair5.cu): solution rows and column sums
+// into b.vic
+cudaError_t launch_vic_pair5(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st);
 size_t vic_scratch_bytes(const Geo& g, const Phys& p);
 size_t vic_column_scratch_bytes(const Geo& g, const Phys& p);
 size_t vicf_scratch_bytes(const Geo& g, const Phys& p);

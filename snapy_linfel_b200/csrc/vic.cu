@@ -1,6 +1,8 @@
 // vic.cu — vertically implicit correction (VIC) of one RK stage: the choice of
-// the solver, and the column sweep for 5x5 blocks, very long columns and the
-// entry point without workspace (the rest takes vic_chunk.cuh).
+// the solver, the finish of the solvers that leave their solution in the
+// workspace, and the column sweep: for very long columns, the entry point
+// without workspace and the FP32 form's 5x5 blocks (the other 3x3 solves take
+// vic_chunk.cuh, the FP64 form's 5x5 ones vic_pair5.cu).
 //
 // Two kernels per solve:
 //   k_vic_column    one thread per x1 column (x1 is the vertical axis): the
@@ -74,7 +76,7 @@ constexpr int64_t kSplitMaxCols = 8192;
 
 bool vic_split(const Geo& g, const Phys& p) {
   const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
-  return p.implicit_scheme != 0 && ncol <= kSplitMaxCols;
+  return p.implicit_scheme != 0 && vic_n(p) == 3 && ncol <= kSplitMaxCols;
 }
 
 size_t vic_blocks_bytes(const Geo& g, const Phys& p) {
@@ -82,6 +84,18 @@ size_t vic_blocks_bytes(const Geo& g, const Phys& p) {
   int N = vic_n(p);
   int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   return (size_t)((int64_t)(g.nx1 + 2) * 2 * N * N * ncol) * sizeof(double);
+}
+
+// Element index in S of row r of the solution at layer i: with the column
+// index fastest (the column sweep), or thirty doubles per layer and column
+// (vic_pair5.cu: the FP64 form's 5x5 blocks).
+template <int N, class B>
+__device__ __forceinline__ int64_t solution_at(int64_t ncol, int i, int r, int64_t col) {
+  constexpr int ES = VicDims<N>::ES;
+  if constexpr (N == 5 && std::is_same_v<B, StageBufs>)
+    return ((int64_t)i * ncol + col) * ES + N * N + r;
+  else
+    return ((int64_t)i * ES + N * N + r) * ncol + col;
 }
 
 constexpr int kTC = 32;           // columns per tile
@@ -749,14 +763,17 @@ __device__ __forceinline__ void vic_finish_issue(const Geo& g, const B& b, int64
     for (int j = 0; j < CPT; ++j) {
       const int idx = tid + j * kFinThreads, c = idx % kTC, s = idx / kTC;
       sok[j] = col0 + c < ncol && i0 + s < nl;
-      soff[j] = ((int64_t)(i0 + s) * ES + N * N) * ncol + col0 + c;
+      soff[j] = solution_at<N, B>(ncol, i0 + s, 0, col0 + c);
     }
 #pragma unroll
     for (int r = 0; r < N; ++r)
 #pragma unroll
       for (int j = 0; j < CPT; ++j) {
         const int idx = tid + j * kFinThreads;
-        if (sok[j]) cp_async_bytes8(&t.DL(r, idx % kTC, idx / kTC), S + soff[j] + (int64_t)r * ncol);
+        if (sok[j])
+          cp_async_bytes8(&t.DL(r, idx % kTC, idx / kTC),
+                          S + soff[j] + solution_at<N, B>(ncol, 0, r, 0) -
+                              solution_at<N, B>(ncol, 0, 0, 0));
       }
   }
   // cell inputs, layers fastest (the state arrays run along x1)
@@ -891,7 +908,7 @@ __device__ __forceinline__ void vic_finish_tile_regs(const Geo& g, const Phys& p
     int s = rest % kTL, r = rest / kTL;
     int64_t col = col0 + c;
     int i = i0 + s;
-    dl[r][c][s] = (col < ncol && i < nl) ? S[((int64_t)i * ES + N * N + r) * ncol + col] : 0.;
+    dl[r][c][s] = (col < ncol && i < nl) ? S[solution_at<N, B>(ncol, i, r, col)] : 0.;
   }
   if (tid < 2 * kTC) {
     int c = tid % kTC, k = tid / kTC;
@@ -1024,22 +1041,26 @@ static cudaError_t launch_vic_n(const Geo& g, const Phys& p, const B& b, cudaStr
   const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   const int nl = g.nx1;
   // small column counts: narrower CTAs spread the sequential sweeps over more SMs
-  int bs = ncol >= 148 * 128 ? 128 : (ncol >= 148 * 64 ? 64 : 32);
-  bool split = false;
-  if constexpr (std::is_same_v<B, StageBufs>) split = b.vicT != nullptr;
-  if constexpr (std::is_same_v<B, StageBufs>) {
-    if (split) {
-      const int64_t nb = ncol * (nl + 2);
-      k_vic_blocks<N><<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(g, p, b);
-      allow_ring_smem(k_vic_column_pre<N>, pre_ring_bytes<N>(128));
-      k_vic_column_pre<N><<<(unsigned)((ncol + bs - 1) / bs), bs, pre_ring_bytes<N>(bs), st>>>(
-          g, p, b);
+  const int bs = ncol >= 148 * 128 ? 128 : (ncol >= 148 * 64 ? 64 : 32);
+  const unsigned grid = (unsigned)((ncol + bs - 1) / bs);
+  if constexpr (N == 5 && std::is_same_v<B, StageBufs>) {
+    const cudaError_t e = launch_vic_pair5(g, p, b, st);
+    if (e != cudaSuccess) return e;
+  } else {
+    bool split = false;
+    if constexpr (std::is_same_v<B, StageBufs>) {
+      split = b.vicT != nullptr;
+      if (split) {
+        const int64_t nb = ncol * (nl + 2);
+        k_vic_blocks<N><<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(g, p, b);
+        allow_ring_smem(k_vic_column_pre<N>, pre_ring_bytes<N>(128));
+        k_vic_column_pre<N><<<grid, bs, pre_ring_bytes<N>(bs), st>>>(g, p, b);
+      }
     }
-  }
-  if (!split) {
-    allow_ring_smem(k_vic_column<N, B>, back_ring_bytes<N>(128));
-    k_vic_column<N, B><<<(unsigned)((ncol + bs - 1) / bs), bs, back_ring_bytes<N>(bs), st>>>(
-        g, p, b);
+    if (!split) {
+      allow_ring_smem(k_vic_column<N, B>, back_ring_bytes<N>(128));
+      k_vic_column<N, B><<<grid, bs, back_ring_bytes<N>(bs), st>>>(g, p, b);
+    }
   }
   using T = std::remove_pointer_t<decltype(b.u)>;
 #define SNAPB_VF(NS)                                                   \

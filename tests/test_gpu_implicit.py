@@ -1,4 +1,9 @@
-"""The one-warp implicit solve (3x3 blocks) at the column lengths where its
+"""The implicit solves at the sizes where they can go wrong.
+
+5x5 blocks of the FP64 form (sixteen lanes a column, from both ends): odd and
+even columns, the shortest ones, CTAs with columns missing.
+
+The one-warp solve (3x3 blocks) at the column lengths where its
 split changes: 8, 16 and 32 lanes a column, chunks of one layer and of many,
 chunks past the column's end, warps with columns missing, and the longest
 column it takes.
@@ -33,9 +38,9 @@ def L():
     return _lib
 
 
-def _config(nl, nx2, nx3, **kw):
+def _config(nl, nx2, nx3, scheme=1, **kw):
     return make_config(nx1=nl, nx2=nx2, nx3=nx3, x1=(0.0, 0.1 * nl), x2=(0.0, 0.1 * nx2),
-                       x3=(0.0, 0.1 * nx3), grav=(-0.2, 0.0, 0.0), implicit_scheme=1,
+                       x3=(0.0, 0.1 * nx3), grav=(-0.2, 0.0, 0.0), implicit_scheme=scheme,
                        bc=("reflecting",) * 4 + ("periodic",) * 2, **kw)
 
 
@@ -44,12 +49,22 @@ def _config(nl, nx2, nx3, **kw):
     (64, 4, 3), (65, 3, 1), (100, 3, 3), (127, 3, 1), (128, 5, 1), (129, 3, 1), (192, 3, 1),
     (257, 3, 1), (1216, 3, 1), (1217, 3, 1)])
 def test_correction_matches_oracle(L, oracle, nl, nx2, nx3):
-    c = _config(nl, nx2, nx3)
+    _correction(L, oracle, nl, nx2, nx3, 1, 0.05)
+
+
+@pytest.mark.parametrize("dt", [0.05, 5.0])
+@pytest.mark.parametrize("nl,nx2,nx3", [(3, 3, 1), (4, 7, 1), (5, 8, 1), (6, 9, 1), (31, 3, 3),
+                                        (64, 5, 3), (129, 17, 1)])
+def test_five_by_five_correction_matches_oracle(L, oracle, nl, nx2, nx3, dt):
+    _correction(L, oracle, nl, nx2, nx3, 9, dt)
+
+
+def _correction(L, oracle, nl, nx2, nx3, scheme, dt):
+    c = _config(nl, nx2, nx3, scheme)
     rng = np.random.default_rng(nl)
     w = random_prim(rng, c.shape)
     u = oracle.prim2cons(c, w)
     du = 0.05 * (rng.random(c.shape) - 0.5)
-    dt = 0.05
     ref, m_ref = du.copy(), np.zeros_like(u)
     oracle.implicit_correction(c, dt, ref, w, m_ref)
     ws = torch.empty(L.lib().snapb_workspace_size(ctypes.byref(c)), dtype=torch.uint8,
