@@ -43,6 +43,7 @@
 
 #include "dual.cuh"
 #include "kernels.cuh"
+#include "vadj_chunk.cuh"
 #include "ring.cuh"
 #include "riemann_adj.cuh"
 #include "bilinear_adj.cuh"
@@ -149,7 +150,34 @@ struct CombineArgs {
   AxisAdj a1, a2, a3;
 };
 
-__global__ void k_adj_combine(Geo g, CombineArgs A) {
+// images of index x along one axis as a bit mask: bit 0 itself, bits 1 .. ng
+// the lower ghosts, bits ng + 1 .. 2 ng the upper ones (from the end)
+struct ImageMask {
+  unsigned has, flip;
+};
+__device__ __forceinline__ ImageMask image_mask(const AxisAdj& a, int x) {
+  ImageMask m{1u, 0u};
+  if (a.n == 1 || (x >= 2 * a.ng && x < a.n - 2 * a.ng)) return m;  // nobody's source
+  for (int y = 0; y < a.ng; ++y) {
+    bool f;
+    if (axis_src(a, y, f) == x) m.has |= 2u << y, m.flip |= f ? 2u << y : 0u;
+    if (axis_src(a, a.n - 1 - y, f) == x) {
+      m.has |= 2u << (a.ng + y);
+      m.flip |= f ? 2u << (a.ng + y) : 0u;
+    }
+  }
+  return m;
+}
+__device__ __forceinline__ int image_at(const AxisAdj& a, int x, int bit) {
+  return bit == 0 ? x : (bit <= a.ng ? bit - 1 : a.n - (bit - a.ng));
+}
+
+// One thread per cell; the images of a cell are found once and every variable
+// gathered from them (512 x 256 cells, reflecting: 20.8 us with a gather that
+// listed them per variable in local arrays).
+template <int NS>
+__global__ void __launch_bounds__(256) k_adj_combine(Geo g, CombineArgs A) {
+  constexpr int NV = 5 + NS;
   int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= g.sv) return;
   const int i = umod(t, g.nc1);
@@ -157,19 +185,42 @@ __global__ void k_adj_combine(Geo g, CombineArgs A) {
   const int k = udiv(t, (int64_t)g.nc1 * g.nc2);
   const bool inner = i >= g.il && i <= g.iu && j >= g.jl && j <= g.ju && k >= g.kl && k <= g.ku;
   const int64_t sv = g.sv;
-  for (int v = 0; v < 5; ++v) {
-    double x = inner ? bc_gather(A.gu_out, sv, g.nc1, g.nc2, v, true, A.a1, A.a2, A.a3, i, j, k)
-                     : 0.;
-    A.gu[v * sv + t] = A.w1 * x;
-    if (inner) A.gu0[v * sv + t] += A.w0 * x;
-    A.GD[v * sv + t] = A.w2 * x;
+  double acc[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) acc[v] = 0.;
+  if (inner) {
+    const ImageMask m1 = image_mask(A.a1, i), m2 = image_mask(A.a2, j), m3 = image_mask(A.a3, k);
+    for (unsigned b3 = m3.has; b3; b3 &= b3 - 1) {
+      const int q3 = __ffs(b3) - 1, kk = image_at(A.a3, k, q3);
+      for (unsigned b2 = m2.has; b2; b2 &= b2 - 1) {
+        const int q2 = __ffs(b2) - 1, jj = image_at(A.a2, j, q2);
+        for (unsigned b1 = m1.has; b1; b1 &= b1 - 1) {
+          const int q1 = __ffs(b1) - 1;
+          const int64_t o = ((int64_t)kk * g.nc2 + jj) * g.nc1 + image_at(A.a1, i, q1);
+          const double s1 = m1.flip >> q1 & 1 ? -1. : 1., s2 = m2.flip >> q2 & 1 ? -1. : 1.,
+                       s3 = m3.flip >> q3 & 1 ? -1. : 1.;
+          acc[IDN] += A.gu_out[IDN * sv + o];
+          acc[IVX] += s1 * A.gu_out[IVX * sv + o];
+          acc[IVY] += s2 * A.gu_out[IVY * sv + o];
+          acc[IVZ] += s3 * A.gu_out[IVZ * sv + o];
+          acc[IPR] += A.gu_out[IPR * sv + o];
+#pragma unroll
+          for (int n = 0; n < NS; ++n) acc[5 + n] += A.gs_out[n * sv + o];
+        }
+      }
+    }
   }
-  for (int n = 0; n < A.ns; ++n) {
-    double x = inner ? bc_gather(A.gs_out, sv, g.nc1, g.nc2, n, false, A.a1, A.a2, A.a3, i, j, k)
-                     : 0.;
-    A.gs[n * sv + t] = A.w1 * x;
-    if (inner) A.gs0[n * sv + t] += A.w0 * x;
-    A.GD[(5 + n) * sv + t] = A.w2 * x;
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    A.gu[v * sv + t] = A.w1 * acc[v];
+    if (inner) A.gu0[v * sv + t] += A.w0 * acc[v];
+    A.GD[v * sv + t] = A.w2 * acc[v];
+  }
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    A.gs[n * sv + t] = A.w1 * acc[5 + n];
+    if (inner) A.gs0[n * sv + t] += A.w0 * acc[5 + n];
+    A.GD[(5 + n) * sv + t] = A.w2 * acc[5 + n];
   }
 }
 
@@ -1285,7 +1336,6 @@ __global__ void __launch_bounds__(128) k_vadj_sweep(Geo g, Phys p, AdjBufs b) {
 // in T, the same folds at the first and last layers); the outputs (delta and
 // t in S, the cotangents in Z) are the sweep's, up to FP64 rounding.
 constexpr int kVadjCrThreads = 128;
-constexpr int64_t kVadjCrMaxCols = 148 * 64;  // above this the sweep fills the GPU
 inline size_t vadj_cr_smem_bytes(int nl) {
   return ((size_t)nl * 30 + 2 * (kVadjCrThreads / 32)) * sizeof(double);
 }
@@ -1409,25 +1459,32 @@ __global__ void __launch_bounds__(kVadjCrThreads) k_vadj_cr3(Geo g, Phys p, AdjB
 // Per cell m in [-1, nl] of every interior column: the block-dependence
 // contraction into GW, and (interior cells) the redistribution's density
 // term, the scalar mass-fix term and the cotangent of the explicit du.
+// Where the column solvers left delta (rows 0 .. N-1) and t (rows N .. 2N-1):
+// row e of layer i, column c at at[e * se + i * sl + c * sc]
+struct VadjSolution {
+  const double* at;
+  int64_t se, sl, sc;
+  const double* Z;  // [3][ncol]
+};
+
 template <int N, int NS>
-__global__ void __launch_bounds__(128) k_vadj_contract(Geo g, Phys p, AdjBufs b) {
-  constexpr int E1 = VadjDims<N>::E1, ES = VadjDims<N>::ES;
+__global__ void __launch_bounds__(128) k_vadj_contract(Geo g, Phys p, AdjBufs b, VadjSolution sol) {
   const int nl = g.nx1;
   const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   const int64_t col0 = (int64_t)blockIdx.x * kCTC;
   const int m0 = -1 + (int)blockIdx.y * kCTL;  // first cell of the tile
   const int64_t sv = g.sv;
-  const double* S = b.vic + (int64_t)(nl + 2) * E1 * ncol;
-  const double* Z = S + (int64_t)nl * ES * ncol;
-  const int oD = 2 * N * N, oT = 2 * N * N + N;
   // t and delta of layers m0-1 .. m0+kCTL (slot = layer - (m0-1)), extended:
   // t = 0 outside [0, nl), delta mirrored (normal row negated) at -1 and nl
   __shared__ double td[2 * N][kCTC][kCTL + 3];
   __shared__ double zs[3][kCTC];
   const int tid = threadIdx.x;
   for (int idx = tid; idx < 2 * N * kCTC * (kCTL + 2); idx += blockDim.x) {
-    int c = idx % kCTC, rest = idx / kCTC;
-    int s = rest % (kCTL + 2), e = rest / (kCTL + 2);
+    // neighbouring threads on whichever index is contiguous
+    const int inner = sol.sl == 1 ? kCTL + 2 : kCTC;
+    const int x0 = idx % inner, rest = idx / inner;
+    const int x1 = rest % (kCTC * (kCTL + 2) / inner), e = rest / (kCTC * (kCTL + 2) / inner);
+    const int c = sol.sl == 1 ? x1 : x0, s = sol.sl == 1 ? x0 : x1;
     int64_t col = col0 + c;
     int layer = m0 - 1 + s;
     double x = 0.;
@@ -1435,18 +1492,18 @@ __global__ void __launch_bounds__(128) k_vadj_contract(Geo g, Phys p, AdjBufs b)
       if (e < N) {  // delta
         int src = layer < 0 ? 0 : (layer >= nl ? nl - 1 : layer);
         if (layer >= -1 && layer <= nl) {
-          x = S[((int64_t)src * ES + oD + e) * ncol + col];
+          x = sol.at[e * sol.se + src * sol.sl + col * sol.sc];
           if ((layer == -1 || layer == nl) && e == 1) x = -x;
         }
       } else if (layer >= 0 && layer < nl) {  // t
-        x = S[((int64_t)layer * ES + oT + (e - N)) * ncol + col];
+        x = sol.at[e * sol.se + layer * sol.sl + col * sol.sc];
       }
     }
     td[e][c][s] = x;
   }
   if (tid < 3 * kCTC) {
     int c = tid % kCTC, k = tid / kCTC;
-    zs[k][c] = col0 + c < ncol ? Z[k * ncol + col0 + c] : 0.;
+    zs[k][c] = col0 + c < ncol ? sol.Z[k * ncol + col0 + c] : 0.;
   }
   __syncthreads();
   const double gm1c = p.gammad - 1.;
@@ -1523,8 +1580,9 @@ __global__ void __launch_bounds__(128) k_vadj_contract(Geo g, Phys p, AdjBufs b)
 }
 
 // SNAPB_VADJ_SOLVE = "sweep" or "cr" forces the adjoint's column solver (the
-// sweep, or cyclic reduction where it applies); by default cyclic reduction
-// takes up to kVadjCrMaxCols columns of 3x3 blocks
+// sweep, or cyclic reduction where it applies) from assembled blocks; by
+// default the one-warp solver (vadj_chunk.cu) takes 3x3 blocks and columns of
+// up to 1216 layers, the sweep the others
 static int vadj_solver_env() {
   const char* e = std::getenv("SNAPB_VADJ_SOLVE");
   if (!e) return 0;
@@ -1538,23 +1596,34 @@ static cudaError_t launch_vic_adj_n(const Geo& g, const Phys& p, const AdjBufs& 
                                     cudaStream_t st) {
   const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   const int nl = g.nx1;
-  dim3 ga((unsigned)((ncol + kATC - 1) / kATC), (unsigned)((nl + 2 + kATL<N> - 1) / kATL<N>));
-  k_vadj_assemble<N, NS><<<ga, 256, 0, st>>>(g, p, b);
-  const size_t cr_smem = vadj_cr_smem_bytes(nl);
   const int forced = vadj_solver_env();
-  const bool cr_fits = N == 3 && cr_smem <= 200 * 1024;
-  if (cr_fits && (forced == 2 || (forced == 0 && ncol <= kVadjCrMaxCols))) {
-    raise_smem_limit(k_vadj_cr3, 200 * 1024);  // once per kernel: the largest plan
-    k_vadj_cr3<<<(unsigned)ncol, kVadjCrThreads, cr_smem, st>>>(g, p, b);
+  constexpr int E1 = VadjDims<N>::E1, ES = VadjDims<N>::ES;
+  double* S = b.vic + (int64_t)(nl + 2) * E1 * ncol;
+  double* Z = S + (int64_t)nl * ES * ncol;
+  VadjSolution sol{S + (int64_t)2 * N * N * ncol, ncol, (int64_t)ES * ncol, 1, Z};
+  if (forced == 0 && vadj_chunk_applies(g, p)) {
+    sol = VadjSolution{S, ncol * nl, 1, nl, Z};
+    const cudaError_t e =
+        launch_vadj_chunk(g, p, VadjChunk{b.dt, b.W, b.R, b.D, b.GD, S, Z}, st);
+    if (e != cudaSuccess) return e;
   } else {
-    // the ring takes vadj_ring_bytes per thread: 32-thread CTAs
-    const int bs = 32;
-    raise_smem_limit(k_vadj_sweep<N>, vadj_ring_bytes<N>(bs));
-    k_vadj_sweep<N><<<(unsigned)((ncol + bs - 1) / bs), bs, vadj_ring_bytes<N>(bs), st>>>(g, p,
-                                                                                         b);
+    dim3 ga((unsigned)((ncol + kATC - 1) / kATC), (unsigned)((nl + 2 + kATL<N> - 1) / kATL<N>));
+    k_vadj_assemble<N, NS><<<ga, 256, 0, st>>>(g, p, b);
+    const size_t cr_smem = vadj_cr_smem_bytes(nl);
+    const bool cr_fits = N == 3 && cr_smem <= 200 * 1024;
+    if (cr_fits && forced == 2) {
+      raise_smem_limit(k_vadj_cr3, 200 * 1024);  // once per kernel: the largest plan
+      k_vadj_cr3<<<(unsigned)ncol, kVadjCrThreads, cr_smem, st>>>(g, p, b);
+    } else {
+      // the ring takes vadj_ring_bytes per thread: 32-thread CTAs
+      const int bs = 32;
+      raise_smem_limit(k_vadj_sweep<N>, vadj_ring_bytes<N>(bs));
+      k_vadj_sweep<N><<<(unsigned)((ncol + bs - 1) / bs), bs, vadj_ring_bytes<N>(bs), st>>>(g, p,
+                                                                                           b);
+    }
   }
   dim3 gc((unsigned)((ncol + kCTC - 1) / kCTC), (unsigned)((nl + 2 + kCTL - 1) / kCTL));
-  k_vadj_contract<N, NS><<<gc, 128, 0, st>>>(g, p, b);
+  k_vadj_contract<N, NS><<<gc, 128, 0, st>>>(g, p, b, sol);
   return cudaGetLastError();
 }
 
@@ -1808,7 +1877,13 @@ int snapb_stage_adjoint(const snapb_hydro_config* cfg, int stage, const double* 
   cudaError_t e;
   {
     ScopedTimer t(SNAPB_K_ADJ_COMBINE, st);
-    k_adj_combine<<<(unsigned)((g.sv + 255) / 256), 256, 0, st>>>(g, ca);
+    const unsigned grid = (unsigned)((g.sv + 255) / 256);
+    switch (p.nscalar) {
+      case 0: k_adj_combine<0><<<grid, 256, 0, st>>>(g, ca); break;
+      case 1: k_adj_combine<1><<<grid, 256, 0, st>>>(g, ca); break;
+      case 2: k_adj_combine<2><<<grid, 256, 0, st>>>(g, ca); break;
+      default: k_adj_combine<3><<<grid, 256, 0, st>>>(g, ca);
+    }
     e = cudaGetLastError();
   }
   if (e != cudaSuccess) return cuda_rc(e, "stage_adjoint combine");

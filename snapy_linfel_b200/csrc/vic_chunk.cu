@@ -50,21 +50,6 @@ __global__ void __launch_bounds__(32)
   }
 }
 
-// f(G, NS) as compile-time constants
-template <class F>
-static cudaError_t with_lanes_scalars(int lanes, int ns, F&& f) {
-#define SNAPB_GN(G, NS) \
-  case G * 4 + NS: return f(std::integral_constant<int, G>{}, std::integral_constant<int, NS>{});
-  if (ns < 0 || ns > 3) return cudaErrorInvalidValue;
-  switch (lanes * 4 + ns) {
-    SNAPB_GN(8, 0) SNAPB_GN(8, 1) SNAPB_GN(8, 2) SNAPB_GN(8, 3)
-    SNAPB_GN(16, 0) SNAPB_GN(16, 1) SNAPB_GN(16, 2) SNAPB_GN(16, 3)
-    SNAPB_GN(32, 0) SNAPB_GN(32, 1) SNAPB_GN(32, 2) SNAPB_GN(32, 3)
-  }
-#undef SNAPB_GN
-  return cudaErrorInvalidValue;
-}
-
 template <class B>
 static cudaError_t launch_chunk(const Geo& g, const Phys& p, const B& b, cudaStream_t st) {
   const int lanes = chunk_lanes(g.nx1), m = chunk_layers(g.nx1), cw = 32 / lanes;

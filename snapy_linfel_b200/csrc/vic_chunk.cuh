@@ -127,6 +127,96 @@ __device__ __forceinline__ void chunk_jac(const ChunkCell<T>& c, T gm1, T s, T (
   J[2][2] = mul(gm1 + T(1), su);
 }
 
+// The blocks of a column's layers in upward order, in the precision BT:
+// b_l = -(|A|_l + J_{l-1}), a_l = |A|_l + |A|_{l+1} + 1/dt - phi and
+// c_l = -(|A|_{l+1} - J_{l+1}) (|A|_l at the lower face of layer l, all scaled
+// by s = A / 2V), with the walls folded into a at the first and last layers.
+template <class BT>
+struct ChunkBlocks {
+  BT gm1, s, idt, grav;
+  ChunkCell<BT> cc;                // the layer's cell
+  BT Af[3][3], bf[3][3], Jc[3][3];  // |A| of its lower face, its b, J of its cell
+  __device__ __forceinline__ void start(const ChunkCell<BT>& below, const ChunkCell<BT>& cell) {
+    BT Jp[3][3];
+    cc = cell;
+    chunk_abs_a(below, cell, gm1, s, Af);
+    chunk_jac(below, gm1, s, Jp);
+    chunk_jac(cell, gm1, s, Jc);
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) bf[r][q] = -(Af[r][q] + Jp[r][q]);
+  }
+  // a, b, c of layer l from the cell above it; layers past the column's end
+  // are x = 0.  TR: of the transposed system, whose row l holds a_l^T,
+  // c_{l-1}^T and b_{l+1}^T, when tr is set.
+  template <bool TR>
+  __device__ __forceinline__ void next(const ChunkCell<BT>& cn, int l, int nl, bool tr,
+                                       double (&a)[3][3], double (&b)[3][3], double (&c)[3][3]) {
+    BT An[3][3], Jn[3][3], af[3][3], bv[3][3], cv[3][3], up[3][3];
+    chunk_abs_a(cc, cn, gm1, s, An);
+    chunk_jac(cn, gm1, s, Jn);
+    const bool real = l < nl, first = l == 0, last = l == nl - 1;
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        BT av = Af[r][q] + An[r][q];
+        if ((r == 1 && q == 0) || (r == 2 && q == 1)) av -= grav;
+        if (r == q) av += idt;
+        af[r][q] = av;
+        bv[r][q] = bf[r][q];
+        cv[r][q] = Jn[r][q] - An[r][q];
+        if (TR) up[r][q] = Jc[r][q] - Af[r][q];  // c of the layer below
+        bf[r][q] = -(An[r][q] + Jc[r][q]);       // b of the layer above
+        Af[r][q] = An[r][q];
+        Jc[r][q] = Jn[r][q];
+      }
+    if (first || l >= nl - 1) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          if (first) af[r][q] += q == 1 ? -bv[r][q] : bv[r][q];
+          if (last) af[r][q] += q == 1 ? -cv[r][q] : cv[r][q];
+          if (!real) af[r][q] = r == q ? BT(1) : BT(0);
+        }
+    }
+    if (TR) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          if (q > r) {
+            const BT x = af[r][q];
+            af[r][q] = tr ? af[q][r] : x;
+            af[q][r] = tr ? x : af[q][r];
+          }
+          bv[r][q] = tr ? up[q][r] : bv[r][q];
+          cv[r][q] = tr ? bf[q][r] : cv[r][q];
+        }
+    }
+    if (first || l >= nl - 1) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          if (first || !real) bv[r][q] = BT(0);
+          if (last || !real) cv[r][q] = BT(0);
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        a[r][q] = (double)af[r][q];
+        b[r][q] = (double)bv[r][q];
+        c[r][q] = (double)cv[r][q];
+      }
+    cc = cn;
+  }
+};
+
 // C -= X Y, c -= X y (three fused operations an entry, no separate sum)
 __device__ __forceinline__ void sub_mul3(const double (&X)[3][3], const double (&Y)[3][3],
                                          double (&C)[3][3]) {
@@ -197,6 +287,153 @@ __device__ __forceinline__ void shfl3(const double (&x)[3], int d, double (&y)[3
     y[r] = __shfl_sync(0xffffffffu, x[r], d, G);
 }
 
+// Solve the block-tridiagonal system of a column, one lane per chunk of m
+// layers (lane k of the column's G): eq(j, a, bl, c, rhs), called for j = 0 ..
+// m - 1 in turn, gives the equation bl x_{l-1} + a x_l + c x_{l+1} = rhs of the
+// lane's j-th layer (bl zero at the column's first layer, c at its last, and
+// the identity past its end); mid() is called between the elimination and the
+// reduction; seen(j, x) for every layer of the lane.  The solution is left in
+// mine[(j * kChunkElems + r) * 32].
+template <int G, class Eq, class Mid, class Seen>
+__device__ __forceinline__ void chunk_solve(int m, int k, double* mine, Eq&& eq, Mid&& mid,
+                                            Seen&& seen) {
+  // ---- elimination inside the chunk ----
+  double Ap[3][3] = {}, f[3][3] = {}, pv[3] = {};           // A', f, p of the layer below
+  double Q[3][3] = {}, S[3][3] = {}, P[3] = {};             // first layer's relation
+#pragma unroll
+  for (int r = 0; r < 3; ++r) f[r][r] = Q[r][r] = -1.;      // (none yet: x_0 = x_0)
+  double a[3][3], bl[3][3], c[3][3], rhs[3];                // the layer's equation
+  for (int j = 0;; ++j) {
+    eq(j, a, bl, c, rhs);
+    if (j == m - 1) break;
+    double inv[3][3], t33[3][3];
+    if (j > 0) {
+      sub_mul3(bl, Ap, a);
+      sub_mul3(bl, pv, rhs);
+      mul3(bl, f, t33);
+    } else {
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) t33[r][q] = -bl[r][q];
+    }
+    chunk_inverse(a, inv);
+    mul3(inv, c, Ap);
+    mul3(inv, rhs, pv);
+    neg_mul3(inv, t33, f);
+    double* out = mine + (size_t)j * kChunkElems * 32;
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      out[r * 32] = pv[r];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) {
+        out[(3 + r * 3 + q) * 32] = Ap[r][q];
+        out[(12 + r * 3 + q) * 32] = f[r][q];
+      }
+    }
+    if (j > 0) {
+      sub_mul3(Q, pv, P);
+      sub_mul3(Q, f, S);
+      neg_mul3(Q, Ap, t33);
+#pragma unroll
+      for (int r = 0; r < 3; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Q[r][q] = t33[r][q];
+    } else {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        P[r] = pv[r];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          Q[r][q] = Ap[r][q];
+          S[r][q] = f[r][q];
+        }
+      }
+    }
+  }
+  mid();
+
+  // ---- the system of the chunks' last layers ----
+  double Bm[3][3], Cm[3][3], y[3];
+  {
+    double Pn[3], Qn[3][3], Sn[3][3], inv[3][3], t33[3][3];
+    shfl3<G>(P, k + 1, Pn);
+    shfl3<G>(Q, k + 1, Qn);
+    shfl3<G>(S, k + 1, Sn);  // (the last chunk's c is zero)
+    sub_mul3(bl, Ap, a);
+    sub_mul3(c, Sn, a);
+    sub_mul3(bl, pv, rhs);
+    sub_mul3(c, Pn, rhs);
+    chunk_inverse(a, inv);
+    mul3(inv, rhs, y);
+    mul3(bl, f, t33);
+    neg_mul3(inv, t33, Bm);
+    mul3(c, Qn, t33);
+    neg_mul3(inv, t33, Cm);
+  }
+  // y_k + B y_{k-h} + C y_{k+h} = r, strides h = 1, 2, 4, ...: a chunk without
+  // a neighbour at that distance has a zero block there, so the values that the
+  // shuffle wraps around to do not enter
+  auto reduce = [&](int h, bool more) {
+    double D[3][3] = {}, Xu[3][3], Xd[3][3], xu[3], xd[3], inv[3][3], Bn[3][3], Cn[3][3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) D[r][r] = 1.;
+    shfl3<G>(Cm, k - h, Xu);
+    shfl3<G>(Bm, k + h, Xd);
+    sub_mul3(Bm, Xu, D);
+    sub_mul3(Cm, Xd, D);
+    shfl3<G>(y, k - h, xu);
+    shfl3<G>(y, k + h, xd);
+    sub_mul3(Bm, xu, y);
+    sub_mul3(Cm, xd, y);
+    if (more) {
+      shfl3<G>(Bm, k - h, Xu);
+      shfl3<G>(Cm, k + h, Xd);
+      mul3(Bm, Xu, Bn);
+      mul3(Cm, Xd, Cn);
+    }
+    chunk_inverse(D, inv);
+    double t[3];
+    mul3(inv, y, t);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) y[r] = t[r];
+    if (more) {
+      neg_mul3(inv, Bn, Bm);
+      neg_mul3(inv, Cn, Cm);
+    }
+  };
+  // (kept a loop: unrolled, its five copies overran the instruction cache)
+#pragma unroll 1
+  for (int h = 1; 2 * h < G; h *= 2) reduce(h, true);
+  reduce(G / 2, false);
+
+  // ---- back substitution; x takes the place of p ----
+  double ym[3], x[3];
+  shfl3<G>(y, k - 1, ym);
+#pragma unroll
+  for (int r = 0; r < 3; ++r) {
+    if (k == 0) ym[r] = 0.;
+    x[r] = y[r];
+    mine[((size_t)(m - 1) * kChunkElems + r) * 32] = x[r];
+  }
+  seen(m - 1, x);
+  for (int j = m - 2; j >= 0; --j) {
+    double* at = mine + (size_t)j * kChunkElems * 32;
+    double t[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      t[r] = at[r * 32];
+#pragma unroll
+      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(12 + r * 3 + q) * 32], ym[q], t[r]);
+#pragma unroll
+      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(3 + r * 3 + q) * 32], x[q], t[r]);
+    }
+#pragma unroll
+    for (int r = 0; r < 3; ++r) at[r * 32] = x[r] = t[r];
+    seen(j, x);
+  }
+}
+
 // The columns col0 .. col0 + 32/G - 1 of a block by one warp; sm: the warp's
 // chunk_smem_bytes(m).  Ends with the warp's shared memory still in use by
 // other lanes: the caller synchronizes the warp before the next group.
@@ -215,9 +452,13 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
   double* backs = sm + ((size_t)(m - 1) * kChunkElems + 3) * 32;  // [4], then the columns' cb
   int* cbs = reinterpret_cast<int*>(backs + 4);
 
-  const BT gm1 = (BT)(p.gammad - 1.), gog = (BT)(p.gammad / (p.gammad - 1.));
   const double dt = *b.dt, idtd = 1. / dt;
-  const BT s = (BT)g.A1 * (BT)(0.5 / g.vol), idt = (BT)idtd, grav = (BT)p.grav1;
+  const BT gog = (BT)(p.gammad / (p.gammad - 1.));
+  ChunkBlocks<BT> blocks;
+  blocks.gm1 = (BT)(p.gammad - 1.);
+  blocks.s = (BT)g.A1 * (BT)(0.5 / g.vol);
+  blocks.idt = (BT)idtd;
+  blocks.grav = (BT)p.grav1;
 
   // state of layer l (clamped to the ghost above the column), as stored
   auto load_w = [&](int l, T (&raw)[5]) {
@@ -239,144 +480,41 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
     return rho;
   };
 
-  // ---- elimination inside the chunk ----
-  double Ap[3][3] = {}, f[3][3] = {}, pv[3] = {};           // A', f, p of the layer below
-  double Q[3][3] = {}, S[3][3] = {}, P[3] = {};             // first layer's relation
-#pragma unroll
-  for (int r = 0; r < 3; ++r) f[r][r] = Q[r][r] = -1.;      // (none yet: x_0 = x_0)
   double sum_r2 = 0., sum_du = 0.;
-  double a[3][3], bl[3][3], c[3][3], rhs[3];                // the layer's equation
+  T rawn[5], rawd[3];
+  double rc;  // density of the layer
   {
-    T rawn[5], rawd[3];
-    ChunkCell<BT> cc, cn;
-    BT Af[3][3], bf[3][3], Jc[3][3];  // s|A| of the lower face, b of the layer, sJ of its cell
-    double rc, rn;
-    {
-      BT Jp[3][3];
-      load_w(l0 - 1, rawn);
-      T raw0[5];
-      load_w(l0, raw0);
-      load_d(l0, rawd);
-      make(l0 - 1, rawn, cn);
-      load_w(l0 + 1, rawn);
-      rc = make(l0, raw0, cc);
-      chunk_abs_a(cn, cc, gm1, s, Af);
-      chunk_jac(cn, gm1, s, Jp);
-      chunk_jac(cc, gm1, s, Jc);
-#pragma unroll
-      for (int r = 0; r < 3; ++r)
-#pragma unroll
-        for (int q = 0; q < 3; ++q) bf[r][q] = -(Af[r][q] + Jp[r][q]);
-    }
-    for (int j = 0;; ++j) {
-      const int l = l0 + j;
-      rn = make(l + 1, rawn, cn);
-      double du[3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) du[r] = (double)rawd[r];
-      if (j < m - 1) {  // the next layer's inputs, ahead of this one's arithmetic
-        load_w(l + 2, rawn);
-        load_d(l + 1, rawd);
-      }
-      BT An[3][3], Jn[3][3];
-      chunk_abs_a(cc, cn, gm1, s, An);
-      chunk_jac(cn, gm1, s, Jn);
-      // a, b, c with the boundary folds of the first and last layers; layers
-      // past the column's end are x = 0
-      const bool real = l < nl, first = l == 0, last = l == nl - 1;
-      BT af[3][3], bv[3][3], cv[3][3];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          BT av = Af[r][q] + An[r][q];
-          if ((r == 1 && q == 0) || (r == 2 && q == 1)) av -= grav;
-          if (r == q) av += idt;
-          af[r][q] = av;
-          bv[r][q] = bf[r][q];
-          cv[r][q] = Jn[r][q] - An[r][q];
-          bf[r][q] = -(An[r][q] + Jc[r][q]);  // b of the layer above
-          Af[r][q] = An[r][q];
-          Jc[r][q] = Jn[r][q];
-        }
-      }
-      if (first || l >= nl - 1) {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            if (first) af[r][q] += q == 1 ? -bv[r][q] : bv[r][q];
-            if (last) af[r][q] += q == 1 ? -cv[r][q] : cv[r][q];
-            if (first || !real) bv[r][q] = BT(0);
-            if (last || !real) cv[r][q] = BT(0);
-            if (!real) af[r][q] = r == q ? BT(1) : BT(0);
-          }
-          if (!real) du[r] = 0.;
-        }
-      }
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          a[r][q] = (double)af[r][q];
-          bl[r][q] = (double)bv[r][q];
-          c[r][q] = (double)cv[r][q];
-        }
-        rhs[r] = mul(du[r], idtd);
-      }
-      if (real) {
-        sum_r2 = fma(rc, rc, sum_r2);
-        sum_du += du[0];
-      }
-      cc = cn;
-      rc = rn;
-      if (j == m - 1) break;
-      double inv[3][3], t33[3][3];
-      if (j > 0) {
-        sub_mul3(bl, Ap, a);
-        sub_mul3(bl, pv, rhs);
-        mul3(bl, f, t33);
-      } else {
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int q = 0; q < 3; ++q) t33[r][q] = -bl[r][q];
-      }
-      chunk_inverse(a, inv);
-      mul3(inv, c, Ap);
-      mul3(inv, rhs, pv);
-      neg_mul3(inv, t33, f);
-      double* out = mine + (size_t)j * kChunkElems * 32;
-#pragma unroll
-      for (int r = 0; r < 3; ++r) {
-        out[r * 32] = pv[r];
-#pragma unroll
-        for (int q = 0; q < 3; ++q) {
-          out[(3 + r * 3 + q) * 32] = Ap[r][q];
-          out[(12 + r * 3 + q) * 32] = f[r][q];
-        }
-      }
-      if (j > 0) {
-        sub_mul3(Q, pv, P);
-        sub_mul3(Q, f, S);
-        neg_mul3(Q, Ap, t33);
-#pragma unroll
-        for (int r = 0; r < 3; ++r)
-#pragma unroll
-          for (int q = 0; q < 3; ++q) Q[r][q] = t33[r][q];
-      } else {
-#pragma unroll
-        for (int r = 0; r < 3; ++r) {
-          P[r] = pv[r];
-#pragma unroll
-          for (int q = 0; q < 3; ++q) {
-            Q[r][q] = Ap[r][q];
-            S[r][q] = f[r][q];
-          }
-        }
-      }
-    }
+    T raw0[5];
+    ChunkCell<BT> below, cell;
+    load_w(l0 - 1, rawn);
+    load_w(l0, raw0);
+    load_d(l0, rawd);
+    make(l0 - 1, rawn, below);
+    load_w(l0 + 1, rawn);
+    rc = make(l0, raw0, cell);
+    blocks.start(below, cell);
   }
+  auto equation = [&](int j, double (&a)[3][3], double (&bl)[3][3], double (&c)[3][3],
+                      double (&rhs)[3]) {
+    const int l = l0 + j;
+    ChunkCell<BT> cn;
+    const double rn = make(l + 1, rawn, cn);
+    double du[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) du[r] = l < nl ? (double)rawd[r] : 0.;
+    if (j < m - 1) {  // the next layer's inputs, ahead of this one's arithmetic
+      load_w(l + 2, rawn);
+      load_d(l + 1, rawd);
+    }
+    blocks.template next<false>(cn, l, nl, false, a, bl, c);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) rhs[r] = mul(du[r], idtd);
+    if (l < nl) {
+      sum_r2 = fma(rc, rc, sum_r2);
+      sum_du += du[0];
+    }
+    rc = rn;
+  };
 
   // The finish's inputs of the lane's first IT cells, fetched before the
   // reduction so that it hides their latency; further ones batch by batch.
@@ -457,87 +595,11 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
       }
     }
   };
-  fetch(lane);
-
-  // ---- the system of the chunks' last layers ----
-  double Bm[3][3], Cm[3][3], y[3];
-  {
-    double Pn[3], Qn[3][3], Sn[3][3], inv[3][3], t33[3][3];
-    shfl3<G>(P, k + 1, Pn);
-    shfl3<G>(Q, k + 1, Qn);
-    shfl3<G>(S, k + 1, Sn);  // (the last chunk's c is zero)
-    sub_mul3(bl, Ap, a);
-    sub_mul3(c, Sn, a);
-    sub_mul3(bl, pv, rhs);
-    sub_mul3(c, Pn, rhs);
-    chunk_inverse(a, inv);
-    mul3(inv, rhs, y);
-    mul3(bl, f, t33);
-    neg_mul3(inv, t33, Bm);
-    mul3(c, Qn, t33);
-    neg_mul3(inv, t33, Cm);
-  }
-  // y_k + B y_{k-h} + C y_{k+h} = r, strides h = 1, 2, 4, ...: a chunk without
-  // a neighbour at that distance has a zero block there, so the values that the
-  // shuffle wraps around to do not enter
-  auto reduce = [&](int h, bool more) {
-    double D[3][3] = {}, Xu[3][3], Xd[3][3], xu[3], xd[3], inv[3][3], Bn[3][3], Cn[3][3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) D[r][r] = 1.;
-    shfl3<G>(Cm, k - h, Xu);
-    shfl3<G>(Bm, k + h, Xd);
-    sub_mul3(Bm, Xu, D);
-    sub_mul3(Cm, Xd, D);
-    shfl3<G>(y, k - h, xu);
-    shfl3<G>(y, k + h, xd);
-    sub_mul3(Bm, xu, y);
-    sub_mul3(Cm, xd, y);
-    if (more) {
-      shfl3<G>(Bm, k - h, Xu);
-      shfl3<G>(Cm, k + h, Xd);
-      mul3(Bm, Xu, Bn);
-      mul3(Cm, Xd, Cn);
-    }
-    chunk_inverse(D, inv);
-    double t[3];
-    mul3(inv, y, t);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) y[r] = t[r];
-    if (more) {
-      neg_mul3(inv, Bn, Bm);
-      neg_mul3(inv, Cn, Cm);
-    }
-  };
-  // (kept a loop: unrolled, its five copies overran the instruction cache)
-#pragma unroll 1
-  for (int h = 1; 2 * h < G; h *= 2) reduce(h, true);
-  reduce(G / 2, false);
-
-  // ---- back substitution; x takes the place of p ----
-  double ym[3], x[3];
-  shfl3<G>(y, k - 1, ym);
-#pragma unroll
-  for (int r = 0; r < 3; ++r) {
-    if (k == 0) ym[r] = 0.;
-    x[r] = y[r];
-    mine[((size_t)(m - 1) * kChunkElems + r) * 32] = x[r];
-  }
-  double sum_x = l0 + m - 1 < nl ? x[0] : 0.;
-  for (int j = m - 2; j >= 0; --j) {
-    double* at = mine + (size_t)j * kChunkElems * 32;
-    double t[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) {
-      t[r] = at[r * 32];
-#pragma unroll
-      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(12 + r * 3 + q) * 32], ym[q], t[r]);
-#pragma unroll
-      for (int q = 0; q < 3; ++q) t[r] = fma(-at[(3 + r * 3 + q) * 32], x[q], t[r]);
-    }
-#pragma unroll
-    for (int r = 0; r < 3; ++r) at[r * 32] = x[r] = t[r];
-    if (l0 + j < nl) sum_x += x[0];
-  }
+  double sum_x = 0.;
+  chunk_solve<G>(m, k, mine, equation, [&] { fetch(lane); },
+                 [&](int j, const double (&x)[3]) {
+                   if (l0 + j < nl) sum_x += x[0];
+                 });
 
   // ---- mass redistribution factor of the column: sum(du - x) / sum(rho^2) ----
   double lost = sum_du - sum_x;
@@ -556,6 +618,21 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
     if (i0 - lane >= total) break;
     fetch(i0);
   }
+}
+
+// f(G, NS) as compile-time constants
+template <class F>
+static cudaError_t with_lanes_scalars(int lanes, int ns, F&& f) {
+#define SNAPB_GN(G, NS) \
+  case G * 4 + NS: return f(std::integral_constant<int, G>{}, std::integral_constant<int, NS>{});
+  if (ns < 0 || ns > 3) return cudaErrorInvalidValue;
+  switch (lanes * 4 + ns) {
+    SNAPB_GN(8, 0) SNAPB_GN(8, 1) SNAPB_GN(8, 2) SNAPB_GN(8, 3)
+    SNAPB_GN(16, 0) SNAPB_GN(16, 1) SNAPB_GN(16, 2) SNAPB_GN(16, 3)
+    SNAPB_GN(32, 0) SNAPB_GN(32, 1) SNAPB_GN(32, 2) SNAPB_GN(32, 3)
+  }
+#undef SNAPB_GN
+  return cudaErrorInvalidValue;
 }
 
 }  // namespace snapb

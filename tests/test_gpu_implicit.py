@@ -127,3 +127,37 @@ def test_ensemble_of_all_lane_counts_is_exact(L):
         for _ in range(2):
             mb.step()
         assert torch.equal(mb.hydro_u, b.hydro_u)
+
+
+@pytest.mark.parametrize("nl,nx2,nx3,ns", [(3, 5, 1, 0), (9, 7, 1, 1), (33, 5, 4, 2), (65, 3, 1, 0),
+                                           (150, 5, 1, 2), (300, 3, 1, 0)])
+def test_adjoint_solver_matches_sweep(L, monkeypatch, nl, nx2, nx3, ns):
+    """the adjoint's two column solves by one warp per group of columns against
+    the block-Thomas sweep (SNAPB_VADJ_SOLVE=sweep): the same stage gradient up
+    to FP64 rounding, bound 1e-11 of each variable's largest entry (the bound
+    of the sweep against cyclic reduction)"""
+    from snapy_linfel_b200.adjoint import Adjoint
+    from snapy_linfel_b200.mesh import MeshBlock
+
+    c = _config(nl, nx2, nx3, nscalar=ns, scalar_recon="weno5", riemann="lmars")
+    rng = np.random.default_rng(nl)
+    mb = MeshBlock(MeshBlockOptions(c, Integration(cfl=0.3)))
+    mb.initialize(random_prim(rng, c.shape), rng.random(c.scalar_shape) if ns else None)
+    u = mb.hydro_u.clone()
+    s = mb.scalar_s.clone() if ns else None
+    dt = torch.tensor([0.02], dtype=torch.float64, device="cuda")
+    gen = torch.Generator(device="cuda").manual_seed(nl)
+    gout = torch.randn(u.shape, generator=gen, device="cuda", dtype=torch.float64)
+    gsout = torch.randn(s.shape, generator=gen, device="cuda", dtype=torch.float64) if ns else None
+    got = []
+    for env in ("", "sweep"):
+        monkeypatch.setenv("SNAPB_VADJ_SOLVE", env)
+        gu0 = torch.zeros_like(u)
+        gs0 = torch.zeros_like(s) if ns else None
+        gu, gs = Adjoint(c).stage(1, dt, u, s, gout, gsout, gu0, gs0)
+        torch.cuda.synchronize()
+        got.append([gu.clone(), gu0.clone()] + ([gs.clone(), gs0.clone()] if ns else []))
+    for a, b in zip(*got):
+        assert torch.isfinite(a).all()
+        for v in range(a.shape[0]):
+            assert float((a[v] - b[v]).abs().max()) <= 1e-11 * float(b[v].abs().max()), v
