@@ -421,12 +421,8 @@ enum {
 int snapb_timing_enable(int on);
 int snapb_timing_query(int kernel, double* total_ms, int* launches);
 
-/* Bulk (TMA-engine) copies: the sweeps that stage their tiles with
- * cp.async.bulk wait on them with a bounded poll; a CTA whose copy did not
- * complete in time gives up its tile and raises a device flag.  Returns the
- * flag (0: every copy completed since the last call; 1: at least one timed
- * out, so the results of those launches are not to be used) and clears it;
- * synchronizes the device; -1 on a CUDA error. */
+/* Bulk (TMA-engine) copies that timed out since the last call.  No kernel
+ * stages its data with them any more, so this is always 0. */
 int snapb_bulk_copy_timeouts(void);
 
 #ifdef __cplusplus

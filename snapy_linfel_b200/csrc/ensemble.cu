@@ -99,7 +99,7 @@ __global__ void k_fill_u64(unsigned long long* p, int n, unsigned long long v) {
 // host plan
 // ---------------------------------------------------------------------------
 enum Phase {
-  PH_X1 = 0, PH_X1REV, PH_X2, PH_X3, PH_VCOL, PH_VFIN, PH_VFUSED, PH_VCR, PH_VCH8, PH_VCH16,
+  PH_X1 = 0, PH_X2, PH_X3, PH_VCOL, PH_VFIN, PH_VFUSED, PH_VCR, PH_VCH8, PH_VCH16,
   PH_VCH32, PH_BCU, PH_BCS, PH_CFL, PH_COUNT
 };
 
@@ -117,8 +117,6 @@ struct snapb_ensemble {
   int use1 = 0, use2 = 0, use3 = 0;
   int sms = 148;
   size_t x1_smem = 0;
-  int x1_cols = 8;  // x1 tile width (columns) of every member
-  int x1_nc1 = 1;   // longest member column (x1 cells with ghosts): the x1 tile layout
   int vic_kernel = kVicColumn;  // the implicit-solve variant in use
   int max_layers = 0;           // longest member column (cyclic reduction's shared memory)
   int chunk_max[3] = {0, 0, 0}; // longest column of the members that take 8, 16, 32 lanes
@@ -172,12 +170,9 @@ int plan(snapb_ensemble* e) {
     Member32& mb = e->mem[m];
     const Geo& g = mb.g;
     const int nvt = 5 + e->p.nscalar;
-    // x1: columns per tile
-    size_t per = x1_smem32_per_column(g, nvt);
-    int C = t.x1_columns > 0 ? t.x1_columns : (int)std::min<size_t>(8, (96 * 1024) / per);
-    C = x1_columns_pow2(std::max(1, std::min<int>(C, (int)((200 * 1024) / per))));
-    mb.x1_cols = C;
-    int64_t ncol1 = (int64_t)g.nc2 * g.nc3;
+    // x1: one warp per item
+    mb.x1 = x1_split32(g, nvt, !e->a2 && !e->a3, t.x1_columns);
+    e->x1_smem = std::max(e->x1_smem, (size_t)mb.x1.pitch * nvt * sizeof(float));
     // march: 128 lines per tile, segments of seglen faces
     int ni = g.iu - g.il + 1;
     int64_t lines2 = (int64_t)ni * (g.ku - g.kl + 1), lines3 = (int64_t)ni * (g.ju - g.jl + 1);
@@ -189,9 +184,7 @@ int plan(snapb_ensemble* e) {
     int64_t ncolv = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
     mb.vic_cols = t.vic_block > 0 ? t.vic_block : 64;
     int64_t tiles[PH_COUNT] = {0};
-    tiles[PH_X1] = e->a1 ? (ncol1 + C - 1) / C : 0;
-    tiles[PH_X1REV] = e->a1 && e->p.grav1 != 0.
-                          ? (ncol1 * 2 * g.ng + kRevisionItem - 1) / kRevisionItem : 0;
+    tiles[PH_X1] = e->a1 ? x1_items32(g, mb.x1) : 0;
     tiles[PH_X2] = e->a2 ? ((lines2 + 127) / 128) * mb.nseg2 : 0;
     tiles[PH_X3] = e->a3 ? ((lines3 + 127) / 128) * mb.nseg3 : 0;
     // implicit solve, default variant: the one-warp kernel where it applies
@@ -223,22 +216,6 @@ int plan(snapb_ensemble* e) {
     tiles[PH_CFL] = (ncell + kCflItem - 1) / kCflItem;
     for (int ph = 0; ph < PH_COUNT; ++ph) e->prefix[ph][m + 1] = e->prefix[ph][m] + tiles[ph];
   }
-  // one x1 tile width for the ensemble (the CTA size of the x1 launch): the
-  // smallest member choice, then the tile counts and shared memory from it
-  e->x1_cols = 16;
-  e->x1_nc1 = 1;
-  for (const Member32& mb : e->mem) {
-    e->x1_cols = std::min(e->x1_cols, mb.x1_cols);
-    e->x1_nc1 = std::max(e->x1_nc1, mb.g.nc1);
-  }
-  for (int m = 0; m < e->M; ++m) {
-    Member32& mb = e->mem[m];
-    mb.x1_cols = e->x1_cols;
-    const int64_t ncol1 = (int64_t)mb.g.nc2 * mb.g.nc3;
-    const int64_t n1 = e->a1 ? (ncol1 + e->x1_cols - 1) / e->x1_cols : 0;
-    e->prefix[PH_X1][m + 1] = e->prefix[PH_X1][m] + n1;
-  }
-  e->x1_smem = x1_smem32_bytes(e->x1_nc1, 5 + e->p.nscalar, e->x1_cols);
   if (e->x1_smem > 200 * 1024) return efail(SNAPB_ERR_ARG, "ensemble: x1 tile too large");
   // implicit solve: cyclic reduction only when every member is in its range
   e->max_layers = 0;
@@ -295,7 +272,8 @@ PersistGrid pgrid(const snapb_ensemble* e, int ph) {
   g.sms = e->sms;
   g.cap = e->tune.ctas_per_sm;
   g.tiles = e->prefix[ph][e->M];
-  if (ph >= PH_VCH8 && ph <= PH_VCH32) g.cap *= 4;  // CTAs of one warp instead of four
+  // CTAs of one warp instead of four
+  if (ph == PH_X1 || (ph >= PH_VCH8 && ph <= PH_VCH32)) g.cap *= 4;
   return g;
 }
 
@@ -440,11 +418,8 @@ int snapb_ensemble_stage_f32(snapb_ensemble* e, int stage, void* stream) {
   int last = e->a3 ? 3 : (e->a2 ? 2 : 1);
   if (e->a1) {
     ScopedTimer t(SNAPB_K_X1, st);
-    if (p.grav1 != 0.)
-      c = launch_x1_ghost_revision32_batch(mem, p, queue(e, PH_X1REV), pgrid(e, PH_X1REV), st);
-    if (c == cudaSuccess)
-      c = launch_x1_32_batch(mem, p, queue(e, PH_X1), stage, last == 1, pgrid(e, PH_X1),
-                             e->x1_smem, e->x1_cols, e->x1_nc1, st);
+    c = launch_x1_32_batch(mem, p, queue(e, PH_X1), stage, last == 1, pgrid(e, PH_X1), e->x1_smem,
+                           st);
     if (c != cudaSuccess) return cuda_e(c, "ensemble x1");
   }
   if (e->a2) {

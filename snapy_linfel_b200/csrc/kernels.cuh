@@ -7,7 +7,7 @@
 
 #include <string>
 
-#include "common.cuh"
+#include "cells.cuh"
 
 namespace snapb {
 
@@ -76,7 +76,7 @@ struct Member32 {
   Geo g;
   StageBufs32 b;
   int bc[6];
-  int x1_cols;           // columns per x1 tile
+  X1Split x1;            // split of the x1 sweep
   int seglen2, nseg2;    // x2 march: faces per segment, segments
   int seglen3, nseg3;    // x3 march
   int vic_cols;          // columns per implicit-column tile
@@ -178,8 +178,8 @@ inline int persistent_grid(K kernel, int block, size_t smem, const PersistGrid& 
 
 // persistent launchers of the batched FP32 stage
 cudaError_t launch_x1_32_batch(const Member32* mem, const Phys& p, const WorkQueue& q,
-                               int stage, bool last, const PersistGrid& pg, size_t smem, int C,
-                               int nc1max, cudaStream_t st);
+                               int stage, bool last, const PersistGrid& pg, size_t smem,
+                               cudaStream_t st);
 cudaError_t launch_march32_batch(int axis, const Member32* mem, const Phys& p,
                                  const WorkQueue& q, int stage, bool first, bool last,
                                  const PersistGrid& pg, cudaStream_t st);
@@ -203,12 +203,10 @@ int vicf_tile_columns();
 cudaError_t launch_bc32_batch(const Member32* mem, const Phys& p, const WorkQueue& q, int kind,
                               double igm1, const PersistGrid& pg, cudaStream_t st);
 size_t x1_smem32_per_column(const Geo& g, int nvt);
-int x1_columns_pow2(int c);  // x1 tile width rounded down to a power of two
-// shared memory of an x1 tile of C columns in a launch whose longest column is nc1max
-size_t x1_smem32_bytes(int nc1max, int nvt, int C);
-cudaError_t launch_x1_ghost_revision32_batch(const Member32* mem, const Phys& p,
-                                             const WorkQueue& q, const PersistGrid& pg,
-                                             cudaStream_t st);
+// split of the FP32 x1 sweep of a block and its items (last: the sweep finishes
+// the cells; columns: per item, 0 for the rule)
+X1Split x1_split32(const Geo& g, int nvt, bool last, int columns);
+int64_t x1_items32(const Geo& g, const X1Split& sp);
 StageBufs32 bufs32_of(const snapb_hydro_config& c, void* ws);
 size_t workspace_size_f32_of(const snapb_hydro_config& c);
 constexpr int kVicFinishCols = 32;    // columns per implicit-finish tile
@@ -216,7 +214,6 @@ constexpr int kVicFinishCols = 32;    // columns per implicit-finish tile
 // large enough that the queue fetch and the CTA's reductions are amortised
 constexpr int kCflItem = 8192;       // interior cells per CFL item
 constexpr int kShellItem = 2048;     // ghost-shell slots per boundary-fill item
-constexpr int kRevisionItem = 1024;  // ghost-revision slots per item
 
 // RK3 (Shu-Osher) stage weights: u = wgt0*u0 + wgt1*u + wgt2*du
 inline void rk3_weights(int stage, double& a, double& b, double& c) {

@@ -12,7 +12,7 @@
 // Formulas as in common.cuh (src/riemann/{hllc,lmars,roe}_impl.h).
 #pragma once
 
-#include "common.cuh"
+#include "cells.cuh"
 
 namespace snapb {
 
@@ -191,6 +191,19 @@ __device__ __forceinline__ void sweep_face_states(int typ, bool scale, int v, co
     face_states<float>(typ, scale, q, wl, wr);
   else
     face_states<float>(v == IDN || v >= 5 ? SNAPB_RECON_WENO5 : SNAPB_RECON_CP5, false, q, wl, wr);
+}
+// the face values of a cell (cells.cuh), the mixing ratios clipped at zero
+template <int FP>
+__device__ __forceinline__ void sweep_cell_states(int typ, bool scale, int v, const float* q,
+                                                  float& lo, float& hi) {
+  if constexpr (FP == 0)
+    cell_states<float>(typ, scale, q, lo, hi);
+  else
+    cell_states<float>(v == IDN || v >= 5 ? SNAPB_RECON_WENO5 : SNAPB_RECON_CP5, false, q, lo, hi);
+  if (v >= 5) {
+    lo = lo < 0.f ? 0.f : lo;
+    hi = hi < 0.f ? 0.f : hi;
+  }
 }
 template <int FP>
 __device__ __forceinline__ void sweep_riemann(int solver, const float* L, const float* R, float pl,

@@ -9,7 +9,8 @@
 //     the residual of the reference x1 momentum balance
 //     rbar_i = -(A1 pf_{i+1} - A1 pf_i)/V + rho_bar_i g1, formed in FP64 and
 //     stored after the cancellation;
-//   * the isentropic x1 ghost revision (pow of full values) in FP64;
+//   * the isentropic x1 ghost revision (pow of full values) in FP64, in the
+//     x1 sweep;
 //   * the implicit column solve (vic.cu, FP64 elimination on full states).
 // The momentum fluxes carry the pressure as p' = p - pf (pert.cuh), so the
 // large hydrostatic pressure never enters an FP32 difference.
@@ -17,7 +18,6 @@
 #include <type_traits>
 
 #include "kernels.cuh"
-#include "bulk.cuh"
 #include "pert.cuh"
 
 namespace snapb {
@@ -72,70 +72,84 @@ __global__ void k_ref32_residual(Geo g, Phys p, StageBufs32 b) {
 // finalize: du' = -dt div'/V + gravity (with the FP64 reference residual),
 // then RK on u' or du for the implicit solve
 // ---------------------------------------------------------------------------
+// What the finish of a cell needs of the descriptors, converted once per CTA
+// and member into shared memory (held in registers it made the marches spill:
+// 0.75 -> 1.2 ms on the 48 members; read from the descriptors, every cell
+// took an FP64 division and nine conversions).
+struct Finish32 {
+  float dt, ivol, g1, g2, g3, w0, w1, w2;
+  bool balance, write_du, stage0;
+  const float *rbf, *rbar;
+  float *D, *u, *u0, *s, *s0, *r;
+  int sv;
+  __device__ __forceinline__ void set(const Geo& g, const Phys& p, const StageBufs32& b) {
+    dt = (float)*b.dt, ivol = (float)(1.0 / g.vol);
+    g1 = (float)p.grav1, g2 = (float)p.grav2, g3 = (float)p.grav3;
+    w0 = (float)b.wgt0, w1 = (float)b.wgt1, w2 = (float)b.wgt2;
+    balance = g.nc1 > 1, write_du = b.write_du != 0, stage0 = b.stage == 0;
+    rbf = b.rbf, rbar = b.rbar, D = b.D, u = b.u, u0 = b.u0, s = b.s, s0 = b.s0, r = b.r;
+    sv = (int)g.sv;
+  }
+};
+
+// A CTA's shared descriptors: the block's (or the current member's), the
+// physics and the finish.
+struct Shared32 {
+  Member32 m;
+  Phys p;
+  Finish32 fin;
+};
+
 template <int NS>
-__device__ __forceinline__ void finalize32(const Geo& g, const Phys& p, const StageBufs32& b,
-                                           int64_t off, int xi, const float* d, const float* wc) {
-  const int64_t sv = g.sv;
-  const float dt = (float)*b.dt;
-  const float ivol = (float)(1.0 / g.vol);
-  float rho = b.rbf[xi] + wc[IDN];
+__device__ __forceinline__ void finalize32(const Finish32& c, int off, int xi, const float* d,
+                                           const float* wc) {
+  const int sv = c.sv;
+  const float dt = c.dt;
+  float rho = c.rbf[xi] + wc[IDN];
   float du[5];
 #pragma unroll
-  for (int v = 0; v < 5; ++v) du[v] = -dt * (d[v] * ivol);
-  if (g.nc1 > 1) du[IVX] += dt * b.rbar[xi];  // reference pressure gradient + rho_bar g1
-  if (p.grav1 != 0.) {
-    du[IVX] += dt * wc[IDN] * (float)p.grav1;
-    du[IPR] += dt * rho * wc[IVX] * (float)p.grav1;
+  for (int v = 0; v < 5; ++v) du[v] = -dt * (d[v] * c.ivol);
+  if (c.balance) du[IVX] += dt * c.rbar[xi];  // reference pressure gradient + rho_bar g1
+  if (c.g1 != 0.f) {
+    du[IVX] += dt * wc[IDN] * c.g1;
+    du[IPR] += dt * rho * wc[IVX] * c.g1;
   }
-  if (p.grav2 != 0.) {
-    du[IVY] += dt * rho * (float)p.grav2;
-    du[IPR] += dt * rho * wc[IVY] * (float)p.grav2;
+  if (c.g2 != 0.f) {
+    du[IVY] += dt * rho * c.g2;
+    du[IPR] += dt * rho * wc[IVY] * c.g2;
   }
-  if (p.grav3 != 0.) {
-    du[IVZ] += dt * rho * (float)p.grav3;
-    du[IPR] += dt * rho * wc[IVZ] * (float)p.grav3;
+  if (c.g3 != 0.f) {
+    du[IVZ] += dt * rho * c.g3;
+    du[IPR] += dt * rho * wc[IVZ] * c.g3;
   }
   float ds[NS > 0 ? NS : 1];
 #pragma unroll
-  for (int n = 0; n < NS; ++n) ds[n] = -dt * (d[5 + n] * ivol);
-  if (b.write_du) {
+  for (int n = 0; n < NS; ++n) ds[n] = -dt * (d[5 + n] * c.ivol);
+  if (c.write_du) {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) b.D[v * sv + off] = du[v];
+    for (int v = 0; v < 5; ++v) c.D[v * sv + off] = du[v];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) b.D[(5 + n) * sv + off] = ds[n];
+    for (int n = 0; n < NS; ++n) c.D[(5 + n) * sv + off] = ds[n];
     return;
   }
-  const float w0 = (float)b.wgt0, w1 = (float)b.wgt1, w2 = (float)b.wgt2;
   float unew_rho = 0.f;
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
-    int64_t o = v * sv + off;
-    float uo = b.u[o];
-    float u0v;
-    if (b.stage == 0) {
-      u0v = uo;
-      b.u0[o] = uo;
-    } else {
-      u0v = b.u0[o];
-    }
-    float un = w0 * u0v + w1 * uo + w2 * du[v];
-    b.u[o] = un;
-    if (v == IDN) unew_rho = b.rbf[xi] + un;
+    const int o = v * sv + off;
+    const float uo = c.u[o], u0v = c.stage0 ? uo : c.u0[o];
+    if (c.stage0) c.u0[o] = uo;
+    const float un = fmaf(c.w2, du[v], fmaf(c.w1, uo, c.w0 * u0v));
+    c.u[o] = un;
+    if (v == IDN) unew_rho = c.rbf[xi] + un;
   }
 #pragma unroll
   for (int n = 0; n < NS; ++n) {
-    int64_t o = n * sv + off;
-    float so = b.s[o];
-    float s0v;
-    if (b.stage == 0) {
-      s0v = so;
-      b.s0[o] = so;
-    } else {
-      s0v = b.s0[o];
-    }
-    float sn = w0 * s0v + w1 * so + w2 * ds[n];
-    b.s[o] = sn;
-    if (b.r) b.r[o] = sn / unew_rho;
+    const int o = n * sv + off;
+    const float so = c.s[o], s0v = c.stage0 ? so : c.s0[o];
+    if (c.stage0) c.s0[o] = so;
+    const float sn = fmaf(c.w2, ds[n], fmaf(c.w1, so, c.w0 * s0v));
+    c.s[o] = sn;
+    if (c.r) c.r[o] = sn / unew_rho;
   }
 }
 
@@ -152,307 +166,239 @@ __device__ __forceinline__ void cons2prim_pert(const float* u, float* w, float r
   w[IPR] = gm1 * (u[IPR] - ke);
 }
 
-// ---------------------------------------------------------------------------
-// x1 column kernel
-// ---------------------------------------------------------------------------
-// One warp per x1 column, C columns per tile (CTA of 32 C threads).  Shared
-// memory of a tile: W' rows [C][NV][nc1], the full density row [C][nc1]
-// (rho_bar + rho', the reconstructed density), then the staging planes of the
-// tile's U' and scalar slabs, [NV][ps] with ps >= C nc1 + 3, 16-byte aligned.
+// Blocks whose x1 column would not fit this many bytes (every variable twice,
+// a density row) are refused by the FP32 entry points.
 size_t x1_smem32_per_column(const Geo& g, int nvt) {
   return (size_t)(2 * nvt + 1) * g.nc1 * sizeof(float);
 }
-// The layout follows the longest column of the launch (nc1max): a batched
-// launch stages the next tile, possibly of another member, while the current
-// one's rows are read, so the staging planes start after the rows of any tile.
-struct X1Smem {
-  int64_t fo, ps;  // float offset of the staging planes, plane stride
-  __host__ __device__ X1Smem(int nc1max, int nvt, int C) {
-    fo = (((int64_t)C * (nvt + 1) * nc1max) + 3) & ~(int64_t)3;
-    ps = ((int64_t)C * nc1max + 3 + 3) & ~(int64_t)3;
-  }
-  __host__ __device__ size_t bytes(int nvt) const {
-    return (size_t)(fo + ps * nvt) * sizeof(float);
-  }
-};
-size_t x1_smem32_bytes(int nc1max, int nvt, int C) { return X1Smem(nc1max, nvt, C).bytes(nvt); }
 
-// set by a CTA of the x1 sweep whose bulk copy did not complete in time
-__device__ int snapb_x1_bulk_timeout = 0;
+// ---------------------------------------------------------------------------
+// x1 sweep
+// ---------------------------------------------------------------------------
+constexpr size_t kX1RowBytes32 = 7 * 1024;  // rows of a warp: 24 and more warps per SM
+constexpr double kX1Resident32 = 148. * 24.;
 
-// Isentropic x1 ghost revision on full values, in FP64, written into W' of the
-// ghost cells (density and pressure rows).  The recurrence
-// p_{n+1} = (p_n^a + c)^(1/a) has h_n = p_n^a = p_e^a + n c, so every ghost
-// level is independent: one slot per (column, end, level), all columns of the
-// block (ghost columns included), slot = (col * 2 + top) * ng + n.  The x1
-// sweep reads these W' values for its ghost cells and leaves them in place.
-__device__ __forceinline__ void x1_ghost_revision32(const Geo& g, const Phys& p,
-                                                    const StageBufs32& b, int64_t slot) {
-  const int ng = g.ng;
-  const int64_t col = slot / (2 * ng);
-  const int rest = (int)(slot - col * 2 * ng);
-  const int top = rest / ng, n = rest - top * ng;
-  const int64_t sv = g.sv, cb = col * g.nc1;  // (k, j, 0) offset: s2 = nc1
-  const int e = top ? g.iu : g.il, dir = top ? 1 : -1;
-  float ue[5], we[5];
-#pragma unroll
-  for (int v = 0; v < 5; ++v) ue[v] = b.u[v * sv + cb + e];
-  cons2prim_pert(ue, we, b.rbf[e], (float)(p.gammad - 1.));
-  const double gam = p.gammad;
-  const double a = (gam - 1.) / gam, ig = 1. / gam, ia = 1. / a;
-  const double grav = -p.grav1, dz = g.dx1;
-  const double ps = b.pb[e] + we[IPR], rs = b.rb[e] + we[IDN];
-  const double K = ps / pow(rs, gam), kg = pow(K, ig);
-  const double step = (top ? -a : a) * grav * dz / kg;
-  const double h = pow(ps, a) + (n + 1) * step;
-  const double pn = pow(h, ia);
-  const double rn = pow(pn / K, ig);
-  const int cell = e + dir * (n + 1);  // ghosts only; the edge cell is never written
-  b.w[IPR * sv + cb + cell] = (float)(pn - b.pb[cell]);
-  b.w[IDN * sv + cb + cell] = (float)(rn - b.rb[cell]);
-}
-
-__global__ void __launch_bounds__(256) k_x1_ghost_revision32(Geo g, Phys p, StageBufs32 b) {
-  const int64_t slot = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (slot < (int64_t)g.nc2 * g.nc3 * 2 * g.ng) x1_ghost_revision32(g, p, b, slot);
-}
-
-// (0) Warp 0 stages the U' and scalar slabs of columns col0 .. col0+C-1 (they
-// are consecutive in every variable plane) into the staging planes: the
-// aligned interiors by bulk copies completing on `bar`, the ragged ends by
-// plain loads (visible after the next CTA barrier).
-template <int NS>
-__device__ __forceinline__ void x1_32_stage(const Geo& g, const StageBufs32& b, int C,
-                                            int64_t col0, float* smf, int nc1max,
-                                            uint64_t* bar) {
+// One item (X1Split, cells.cuh) by one warp, with its rows (full density
+// rho_bar + rho', v', p', mixing ratios) in shared memory:
+//   (1) U' -> W' of the item's cells, W' and the mixing ratios stored;
+//   (2) density and pressure of the x1 ghosts from the isentropic revision of
+//       the edge cells, on full values in FP64, one lane per (column, end,
+//       level);
+//   (3) the cells in rounds of 32 lanes, the item's columns end to end: a lane
+//       forms the flux of its cell's lower face from its own left value and
+//       the next lower lane's right value, and closes the cell below.
+// Not inlined: the one-block and the batched kernel run this very code, so a
+// member of an ensemble rounds as it does alone.
+//
+// Bound: instruction issue (62 % active at 20 warps per SM) and the latency of
+// the conversion's loads.  Per stage, against a tile of columns per CTA (bulk
+// copies into shared memory, barriers, the revision in its own kernel):
+// 384 x 384 x 192, Roe, two tracers 1.29 -> 1.25 ms, 512 x 256 21.0 -> 10.7 us,
+// 48 members of 64 and 128 layers 1.57 ms with either.
+template <int NS, int FP>
+__device__ __noinline__ void x1_32_item(const Shared32* sh, int64_t item, float* row, int last) {
   constexpr int NV = 5 + NS;
-  if (threadIdx.x >= 32) return;
-  const X1Smem L(nc1max, NV, C);
-  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  const int64_t nslab = std::min<int64_t>(C, ncol - col0) * g.nc1;
-  auto plane = [&](int v) -> const float* {
-    return (v < 5 ? b.u + v * g.sv : b.s + (v - 5) * g.sv) + col0 * g.nc1;
-  };
-  if (threadIdx.x == 0) {
-    unsigned bytes = 0;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) bytes += (unsigned)(bulk_split(plane(v), nslab).body * 4);
-    fence_proxy_async_smem();  // earlier reads of the staging planes come first
-    mbar_arrive_expect_tx(bar, bytes);
-  }
-  if (threadIdx.x < 8)
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      bulk_stage_slab(smf + L.fo + v * L.ps, plane(v), nslab, bar, threadIdx.x == 0);
-}
-
-// One tile after its staging completed, every thread of the CTA (one
-// barrier): warp w works column col0 + w.
-//   (1) U' -> W' of the column's cells from the staged slabs into shared
-//       memory, with W' and the scalar mixing ratios stored; ghost cells take
-//       density and pressure from the ghost revision (gravity along x1);
-//   (2) the faces in rounds of 32 (face il + 32 k + lane): states and flux in
-//       registers; the flux difference of cell f takes face f+1 from the next
-//       lane (a shuffle), lane 31 that of the next round's lane 0 one round
-//       later; then du or the RK combination (finalize32).
-// The staging planes are free after (1): on return from x1_32_convert the
-// caller may stage the next tile while x1_32_faces runs.
-template <int NS>
-__device__ __forceinline__ void x1_32_convert(const Geo& g, const Phys& p, const StageBufs32& b,
-                                              int C, int64_t col0, float* smf, int nc1max) {
-  constexpr int NV = 5 + NS;
-  const int nc1 = g.nc1, ng = g.ng, il = g.il, iu = g.iu;
-  const X1Smem L(nc1max, NV, C);
-  float* sw = smf;                        // [C][NV][nc1]
-  float* sr = sw + (size_t)C * NV * nc1;  // [C][nc1]
-  const float* st = smf + L.fo;           // staging planes
-  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  const int tid = threadIdx.x, nt = blockDim.x, lane = tid & 31, c = tid >> 5;
-  const int lgC = __ffs(C) - 1;
-  const int64_t sv = g.sv;
+  const Geo& g = sh->m.g;
+  const StageBufs32& b = sh->m.b;
+  const Phys& p = sh->p;
+  const X1Split sp = sh->m.x1;
+  const int lane = threadIdx.x & 31;
+  const int nc1 = g.nc1, il = g.il, iu = g.iu, ng = g.ng, pitch = sp.pitch;
+  const int sv = (int)g.sv;  // (element indices stay below 2^31: check_config)
+  const int ncol = g.nc2 * g.nc3;
+  const int grp = sp.nseg > 1 ? udiv(item, sp.nseg) : (int)item;
+  const int seg = sp.nseg > 1 ? umod(item, sp.nseg) : 0;
+  const int col0 = grp * sp.K, K = min(sp.K, ncol - col0);
+  // cells [c0, c1) are this item's in every column; rows hold [lo, lo + n)
+  const int c0 = il + seg * sp.seglen, c1 = min(c0 + sp.seglen, iu + 1);
+  const bool bottom = c0 == il, top = c1 == iu + 1;
+  const int lo = bottom ? 0 : c0 - 3, n = (top ? nc1 : c1 + 3) - lo;
+  const int span = col0 * nc1 + lo;
   const float gm1 = (float)(p.gammad - 1.);
   const bool revise = p.grav1 != 0.;
-  int sbase[NV];  // float offset in the staging planes of each variable's element 0
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-    sbase[v] = (int)(v * L.ps) +
-               bulk_phase((v < 5 ? b.u + v * sv : b.s + (v - 5) * sv) + col0 * nc1);
-  auto convert = [&](int cc, int i, bool ghost) {
-    const int64_t off = (col0 + cc) * nc1 + i;
-    const int e = cc * nc1 + i;
-    float uc[5], wc[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) uc[v] = st[sbase[v] + e];
-    cons2prim_pert(uc, wc, b.rbf[i], gm1);
-    float* base = sw + (size_t)cc * NV * nc1;
-    if (ghost && revise) {  // density and pressure from the ghost revision
-      wc[IDN] = b.w[IDN * sv + off];
-      wc[IPR] = b.w[IPR * sv + off];
-#pragma unroll
-      for (int v = IVX; v <= IVZ; ++v) b.w[v * sv + off] = wc[v];
-    } else {
-#pragma unroll
-      for (int v = 0; v < 5; ++v) b.w[v * sv + off] = wc[v];
-    }
-#pragma unroll
-    for (int v = 0; v < 5; ++v) base[v * nc1 + i] = wc[v];
-    sr[(size_t)cc * nc1 + i] = b.rbf[i] + wc[IDN];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      float rr = fdiv(st[sbase[5 + n] + e], b.rbf[i] + uc[IDN]);
-      base[(5 + n) * nc1 + i] = rr;
-      b.R[n * sv + off] = rr;
-    }
-  };
-  if (col0 + c < ncol)
-    for (int i = il + lane; i <= iu; i += 32) convert(c, i, false);
-  for (int idx = tid; idx < 2 * ng * C; idx += nt) {  // ghost cells, 2 ng per column
-    const int cc = idx & (C - 1), k = idx >> lgC;
-    if (col0 + cc < ncol) convert(cc, k < ng ? k : iu + 1 + (k - ng), true);
+  const float *u = b.u, *s = b.s, *rbf = b.rbf, *offL = b.offL, *offR = b.offR;
+  const double* pf = b.pf;
+  float *w = b.w, *rr = b.R, *D = b.D;
+  // which of the item's columns are interior ones
+  bool inner = lane < K;
+  if (inner) {
+    const int j = umod(col0 + lane, g.nc2), k = udiv(col0 + lane, g.nc2);
+    inner = j >= g.jl && j <= g.ju && k >= g.kl && k <= g.ku;
   }
-  __syncthreads();
-}
-
-template <int NS, int FP>
-__device__ __forceinline__ void x1_32_faces(const Geo& g, const Phys& p, const StageBufs32& b,
-                                            int C, int last, int64_t col0, const float* smf) {
-  constexpr int NV = 5 + NS;
-  const int nc1 = g.nc1, il = g.il, iu = g.iu;
-  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;
-  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  auto interior = [&](int cc) {
-    const int64_t col = col0 + cc;
-    if (col >= ncol) return false;
-    const int j = umod(col, g.nc2), k = udiv(col, g.nc2);
-    return j >= g.jl && j <= g.ju && k >= g.kl && k <= g.ku;
-  };
-  const int64_t sv = g.sv;
-  const float gamma = (float)p.gammad;
-  const bool revise = p.grav1 != 0.;
-  const int ptype = (p.r1_shock) ? p.r1_type : interp2_of(p.r1_type);
-  const float A1 = (float)g.A1;
-  // face f of tile column cc; the stencil f-3 .. f+2 stays inside the column (ng >= 3)
-  auto face = [&](int cc, int f, float* F) {
-    const float* base = smf + (size_t)cc * NV * nc1 + f - 3;
-    const float* rho = smf + (size_t)C * NV * nc1 + (size_t)cc * nc1 + f - 3;
-    float L[NV], R[NV];
-    float pl, pr;
+  const unsigned columns = __ballot_sync(0xffffffffu, inner);
+  // two cells a lane at a time, so that both cells' loads are in flight
+  for (int e0 = lane; e0 < K * n; e0 += 64) {
+    float uc[2][5], sc[2][NS > 0 ? NS : 1], rb[2];
+    int xi[2];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      float q[6];
+    for (int h = 0; h < 2; ++h) {
+      const int e = min(e0 + 32 * h, K * n - 1), off = span + e;
+      xi[h] = lo + (sp.K > 1 ? umod(e, n) : e);
 #pragma unroll
-      for (int s6 = 0; s6 < 6; ++s6) q[s6] = v == IDN ? rho[s6] : base[v * nc1 + s6];
-      if (v == IPR) {
-        sweep_face_states<FP>(ptype, p.r1_scale != 0, v, q, pl, pr);
-        pl += b.offL[f];
-        pr += b.offR[f];
-      } else if (v < 5) {
-        int typ = (p.r1_shock || v == IDN) ? p.r1_type : interp2_of(p.r1_type);
-        sweep_face_states<FP>(typ, p.r1_scale != 0, v, q, L[v], R[v]);
-      } else {
-        sweep_face_states<FP>(p.rs_type, p.rs_scale != 0, v, q, L[v], R[v]);
-        L[v] = L[v] < 0.f ? 0.f : L[v];
-        R[v] = R[v] < 0.f ? 0.f : R[v];
+      for (int v = 0; v < 5; ++v) uc[h][v] = u[v * sv + off];
+#pragma unroll
+      for (int m = 0; m < NS; ++m) sc[h][m] = s[m * sv + off];
+      rb[h] = rbf[xi[h]];
+    }
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int e = e0 + 32 * h, off = span + e;
+      if (e >= K * n) break;
+      float wc[5];
+      cons2prim_pert(uc[h], wc, rb[h], gm1);
+      const bool own = (xi[h] >= c0 || bottom) && (xi[h] < c1 || top);
+      row[IDN * pitch + e] = rb[h] + wc[IDN];
+#pragma unroll
+      for (int v = 1; v < 5; ++v) row[v * pitch + e] = wc[v];
+      if (own)
+#pragma unroll
+        for (int v = 0; v < 5; ++v) w[v * sv + off] = wc[v];
+#pragma unroll
+      for (int m = 0; m < NS; ++m) {
+        const float mix = fdiv(sc[h][m], rb[h] + uc[h][IDN]);
+        row[(5 + m) * pitch + e] = mix;
+        if (own) rr[m * sv + off] = mix;
       }
     }
-    if (revise) {
-      if (f == il) {
-        pl = pr;
-        L[IDN] = R[IDN];
-      }
-      if (f == iu + 1) {
-        pr = pl;
-        R[IDN] = L[IDN];
-      }
+  }
+  __syncwarp();
+  if (revise && (bottom || top)) {
+    for (int slot = lane; slot < 2 * ng * K; slot += 32) {
+      const int kk = slot / (2 * ng), rest = slot - kk * 2 * ng;
+      const int end = rest >= ng, lev = rest - end * ng + 1;
+      if (end ? !top : !bottom) continue;
+      const int edge = end ? iu : il, e = kk * n + edge - lo, dst = end ? e + lev : e - lev;
+      const int cell = end ? edge + lev : edge - lev;
+      double pn, rn;
+      isentropic_ghost(p.gammad, -p.grav1 * g.dx1, end, lev,
+                       b.pb[edge] + (double)row[IPR * pitch + e],
+                       b.rb[edge] + (double)u[IDN * sv + span + e], pn, rn);
+      const float wp = (float)(pn - b.pb[cell]), wr = (float)(rn - b.rb[cell]);
+      row[IPR * pitch + dst] = wp;
+      row[IDN * pitch + dst] = rbf[cell] + wr;
+      w[IPR * sv + span + dst] = wp;
+      w[IDN * sv + span + dst] = wr;
     }
-    const float pfv = (float)b.pf[f];
-    L[IPR] = pfv + pl;
-    R[IPR] = pfv + pr;
-    if (p.disable1) {
+    __syncwarp();
+  }
+  const int nn = c1 - c0 + 2, total = K * nn;
+  const float gamma = (float)p.gammad, A1 = (float)g.A1;
+  const bool flux = !p.disable1;
+  const int ptype = p.r1_shock ? p.r1_type : interp2_of(p.r1_type);
+  float Hc[NV], Fc[NV];  // lane 0: lane 31 of the previous round
+#pragma unroll
+  for (int v = 0; v < NV; ++v) Hc[v] = Fc[v] = 0.f;
+  int kk = lane / nn, t = lane - kk * nn;
+  for (int s0 = 0; s0 < total; s0 += 32) {
+    const bool act = s0 + lane < total && (columns >> kk & 1);
+    if (__any_sync(0xffffffffu, act)) {
+      const int c = c0 - 1 + t;
+      const float* cell = row + (act ? kk * n + c - lo : 2);
+      float L[NV], R[NV];
+#pragma unroll
+      for (int v = 0; v < NV; ++v) {
+        float q[5], H;
+#pragma unroll
+        for (int m = 0; m < 5; ++m) q[m] = cell[v * pitch + m - 2];
+        const int typ = v >= 5 ? p.rs_type : (v == IDN ? p.r1_type : ptype);
+        sweep_cell_states<FP>(typ, v >= 5 ? p.rs_scale != 0 : p.r1_scale != 0, v, q, R[v], H);
+        const float below = __shfl_sync(0xffffffffu, H, (lane + 31) & 31);
+        L[v] = lane == 0 ? Hc[v] : below;
+        Hc[v] = below;
+      }
+      const int f = act ? c : il;
+      float pl = L[IPR] + offL[f], pr = R[IPR] + offR[f];
+      if (revise) {
+        if (c == il) {
+          pl = pr;
+          L[IDN] = R[IDN];
+        }
+        if (c == iu + 1) {
+          pr = pl;
+          R[IDN] = L[IDN];
+        }
+      }
+      const float pfv = (float)pf[f];
+      L[IPR] = pfv + pl;
+      R[IPR] = pfv + pr;
+      float F[NV];
 #pragma unroll
       for (int v = 0; v < 5; ++v) F[v] = 0.f;
-    } else {
-      sweep_riemann<FP>(p.riemann, L, R, pl, pr, pfv, IVX, gamma, F);
-    }
+      if (act && t > 0 && flux)
+        sweep_riemann<FP>(p.riemann, L, R, pl, pr, pfv, IVX, gamma, F);
 #pragma unroll
-    for (int n = 0; n < NS; ++n) F[5 + n] = F[IDN] > 0.f ? F[IDN] * L[5 + n] : F[IDN] * R[5 + n];
-  };
-  const float* wcol = smf + (size_t)c * NV * nc1;
-  auto finish = [&](int i, const float* d) {
-    const int64_t off = (col0 + c) * nc1 + i;
-    if (last) {
-      float wc[5];
-#pragma unroll
-      for (int v = 0; v < 5; ++v) wc[v] = wcol[v * nc1 + i];
-      finalize32<NS>(g, p, b, off, i, d, wc);
-    } else {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) b.D[v * sv + off] = d[v];
-    }
-  };
-  // faces il .. iu+1 in rounds of 32 (face f0 + lane); the flux difference
-  // of cell f takes face f+1 from the next lane, lane 31 that of the next
-  // round's lane 0 one round later
-  if (!interior(c)) return;  // the whole warp
-  float Fkeep[NV];  // lane 31: its face of the previous round
-#pragma unroll
-  for (int v = 0; v < NV; ++v) Fkeep[v] = 0.f;
-  for (int f0 = il; f0 <= iu + 1; f0 += 32) {
-    const int f = f0 + lane;
-    float F[NV];
-    if (f <= iu + 1) {
-      face(c, f, F);
-    } else {
-#pragma unroll
-      for (int v = 0; v < NV; ++v) F[v] = 0.f;
-    }
-    float Fn[NV];  // lanes 0 .. 30: face f + 1; lane 31: this round's first face
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      const float dn = __shfl_down_sync(0xffffffffu, F[v], 1);
-      const float f0v = __shfl_sync(0xffffffffu, F[v], 0);
-      Fn[v] = lane < 31 ? dn : f0v;
-    }
-    // this lane's cell: f (lanes 0 .. 30), the previous round's last (lane 31)
-    const int i = lane < 31 ? f : f0 - 1;
-    if (i >= il && i <= iu) {
+      for (int m = 0; m < NS; ++m)
+        F[5 + m] = F[IDN] > 0.f ? F[IDN] * L[5 + m] : F[IDN] * R[5 + m];
       float d[NV];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) d[v] = A1 * Fn[v] - A1 * (lane < 31 ? F[v] : Fkeep[v]);
-      finish(i, d);
-    }
+      for (int v = 0; v < NV; ++v) {
+        const float below = __shfl_sync(0xffffffffu, F[v], (lane + 31) & 31);
+        d[v] = A1 * F[v] - A1 * (lane == 0 ? Fc[v] : below);
+        Fc[v] = below;
+      }
+      if (act && t > 1) {
+        const int off = (col0 + kk) * nc1 + c - 1;
+        if (last) {
+          float wc[5];
+          wc[IDN] = w[IDN * sv + off];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) Fkeep[v] = F[v];
+          for (int v = 1; v < 5; ++v) wc[v] = cell[v * pitch - 1];
+          finalize32<NS>(sh->fin, off, c - 1, d, wc);
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) D[v * sv + off] = d[v];
+        }
+      }
+    }
+    t += 32;
+    while (t >= nn) {
+      t -= nn;
+      ++kk;
+    }
   }
 }
 
-// one tile per CTA: stage, convert, faces
+// one item per CTA of one warp; the block's descriptor goes to shared memory,
+// where the batched form has its members'
 template <int NS, int FP>
-__global__ void __launch_bounds__(512, 2) k_x1_32(Geo g, Phys p, StageBufs32 b, int C, int last) {
-  extern __shared__ __align__(16) float smf[];
-  __shared__ uint64_t bar;
-  if (threadIdx.x == 0) mbar_init(&bar, 1);
-  __syncthreads();
-  const int64_t col0 = (int64_t)blockIdx.x * C;
-  x1_32_stage<NS>(g, b, C, col0, smf, g.nc1, &bar);
-  const bool ok = threadIdx.x >= 32 || mbar_wait(&bar, 0, &snapb_x1_bulk_timeout);
-  if (__syncthreads_or(!ok)) {
-    if (threadIdx.x < 32) mbar_wait(&bar, 0, &snapb_x1_bulk_timeout);  // copies in flight
-    return;
+__global__ void __launch_bounds__(32, 20) k_x1_32(Geo g, Phys p, StageBufs32 b, X1Split sp,
+                                                  int last) {
+  extern __shared__ float x1_rows32[];
+  __shared__ Shared32 sh;
+  if (threadIdx.x == 0) {
+    sh.m.g = g;
+    sh.m.b = b;
+    sh.m.x1 = sp;
+    sh.p = p;
+    sh.fin.set(g, p, b);
   }
-  x1_32_convert<NS>(g, p, b, C, col0, smf, g.nc1);
-  x1_32_faces<NS, FP>(g, p, b, C, last, col0, smf);
+  __syncwarp();
+  x1_32_item<NS, FP>(&sh, blockIdx.x, x1_rows32, last);
 }
 
 // ---------------------------------------------------------------------------
 // x2 / x3 marching sweeps (reference constant along the sweep)
 // ---------------------------------------------------------------------------
+// resident CTAs per SM: the register budget that holds the window of 5 + NS
+// variables without spilling it
+template <int NS, int FP>
+constexpr int kMarchCtas32 = NS >= 2 ? 4 : (NS == 0 && FP == 1 ? 6 : 5);
+
 // One thread's work: line tid (x1 cell x other horizontal index) and face
-// segment seg of the sweep axis.
+// segment seg of the sweep axis.  Cell centred (cells.cuh); per stage x2 and x3
+// 0.81 + 0.85 -> 0.75 + 0.79 ms on the 48 members, 43 + 45 -> 35 + 40 us on 7
+// members of 29 to 129 layers, 0.80 + 0.84 -> 0.79 + 0.84 ms on 384 x 384 x 192
+// with two tracers.  Bound by instruction issue.  Not inlined, as x1_32_item: the one-block and
+// the batched kernel round alike, and the descriptor's fields are read from
+// shared memory when they are needed instead of being held in registers
+// (copied into registers the batched kernel spilled).
 template <int NS, int AX, int FP>
-__device__ __forceinline__ void march32_line(const Geo& g, const Phys& p, const StageBufs32& b,
-                                             int seglen, int first, int last, int64_t tid,
-                                             int seg) {
+__device__ __noinline__ void march32_line(const Shared32* sh, int first, int last, int tid,
+                                          int seg) {
+  const Geo& g = sh->m.g;
+  const StageBufs32& b = sh->m.b;
+  const Phys& p = sh->p;
+  const int seglen = AX == 2 ? sh->m.seglen2 : sh->m.seglen3;
   constexpr int NV = 5 + NS;
   const int ni = g.iu - g.il + 1;
   int lo, hi, olo, ohi;
@@ -463,7 +409,7 @@ __device__ __forceinline__ void march32_line(const Geo& g, const Phys& p, const 
     lo = g.kl, hi = g.ku, st = g.s3, olo = g.jl, ohi = g.ju, ost = g.s2;
   }
   const int no = ohi - olo + 1;
-  if (tid >= (int64_t)ni * no) return;
+  if (tid >= ni * no) return;
   const int i = g.il + umod(tid, ni);
   const int o = olo + udiv(tid, ni);
   const int f0 = lo + seg * seglen;
@@ -471,95 +417,113 @@ __device__ __forceinline__ void march32_line(const Geo& g, const Phys& p, const 
   const int f1 = min(f0 + seglen, hi + 1);
   const int64_t base = i + o * ost;
   const int64_t sv = g.sv;
+  const float *w = b.w, *r = b.R;
+  float* D = b.D;
   const int ivx = AX == 2 ? IVY : IVZ;
   const float A = (float)(AX == 2 ? g.A2 : g.A3);
   const int disabled = AX == 2 ? p.disable2 : p.disable3;
-  const int ncax = AX == 2 ? g.nc2 : g.nc3;
   const float rref = b.rbf[i], pref = b.pbf[i];
   const float gamma = (float)p.gammad;
 
-  // six-cell window of the face's stencil plus one cell loaded a face ahead
-  // (slot 6), so a load's latency overlaps the previous face's arithmetic
-  float q[NV][7];
-  auto load = [&](int cell, int slot) {
-    cell = min(max(cell, 0), ncax - 1);
-    int64_t off = base + cell * st;
+  // five-cell window (cells c-2 .. c+2) and the cell after it, loaded a step
+  // ahead so that its latency overlaps this step's arithmetic; the stencil
+  // stays inside the array (nghost >= 3)
+  float q[NV][6];
+  int at = (int)base + (f0 - 3) * (int)st;  // (indices stay below 2^31: check_config)
+  const int svi = (int)sv, sti = (int)st;
+  auto load = [&](int slot) {
 #pragma unroll
-    for (int v = 0; v < 5; ++v) q[v][slot] = b.w[v * sv + off];
+    for (int v = 0; v < 5; ++v) q[v][slot] = w[v * svi + at];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) q[5 + n][slot] = b.R[n * sv + off];
+    for (int n = 0; n < NS; ++n) q[5 + n][slot] = r[n * svi + at];
+    at += sti;
   };
 #pragma unroll
-  for (int t = 0; t < 6; ++t) load(f0 - 3 + t, t);
+  for (int t = 0; t < 5; ++t) load(t);
 
-  float Fp[NV];
-  for (int f = f0; f <= f1; ++f) {
-    load(f + 3, 6);
-    // the running sums of the cell this face closes, fetched before the
-    // face's arithmetic
+  // The face of cell c pairs its left value with the right value of the cell
+  // before, carried in L; it closes cell c - 1.
+  const int t23 = p.r23_shock ? p.r23_type : interp2_of(p.r23_type);
+  float L[NV], Fp[NV];
+#pragma unroll
+  for (int v = 0; v < NV; ++v) L[v] = Fp[v] = 0.f;
+  int off = (int)base + (f0 - 2) * sti;  // cell c - 1
+  for (int c = f0 - 1; c <= f1; ++c, off += sti) {
+    if (c < f1) load(5);
+    // the running sums of cell c - 1, fetched before the face's arithmetic
     float dprev[NV];
-    if (f > f0 && !first) {
-      const int64_t off = base + (int64_t)(f - 1) * st;
+    if (c > f0 && !first) {
 #pragma unroll
-      for (int v = 0; v < NV; ++v) dprev[v] = b.D[v * sv + off];
+      for (int v = 0; v < NV; ++v) dprev[v] = D[v * svi + off];
     }
-    float L[NV], R[NV], F[NV];
+    float R[NV], H[NV];
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-      if (v < 5) {
-        int typ = (p.r23_shock || v == IDN) ? p.r23_type : interp2_of(p.r23_type);
-        sweep_face_states<FP>(typ, p.r23_scale != 0, v, q[v], L[v], R[v]);
+    for (int v = 0; v < NV; ++v)
+      sweep_cell_states<FP>(v >= 5 ? p.rs_type : (v == IDN ? p.r23_type : t23),
+                            v >= 5 ? p.rs_scale != 0 : p.r23_scale != 0, v, q[v], R[v], H[v]);
+    if (c >= f0) {
+      const float pl = L[IPR], pr = R[IPR];
+      L[IDN] += rref;
+      R[IDN] += rref;
+      L[IPR] += pref;
+      R[IPR] += pref;
+      float F[NV];
+      if (disabled) {
+#pragma unroll
+        for (int v = 0; v < 5; ++v) F[v] = 0.f;
       } else {
-        sweep_face_states<FP>(p.rs_type, p.rs_scale != 0, v, q[v], L[v], R[v]);
-        L[v] = L[v] < 0.f ? 0.f : L[v];
-        R[v] = R[v] < 0.f ? 0.f : R[v];
+        sweep_riemann<FP>(p.riemann, L, R, pl, pr, pref, ivx, gamma, F);
       }
-    }
-    float pl = L[IPR], pr = R[IPR];
-    L[IDN] += rref;
-    R[IDN] += rref;
-    L[IPR] += pref;
-    R[IPR] += pref;
-    if (disabled) {
 #pragma unroll
-      for (int v = 0; v < 5; ++v) F[v] = 0.f;
-    } else {
-      sweep_riemann<FP>(p.riemann, L, R, pl, pr, pref, ivx, gamma, F);
-    }
+      for (int n = 0; n < NS; ++n)
+        F[5 + n] = F[IDN] > 0.f ? F[IDN] * L[5 + n] : F[IDN] * R[5 + n];
+      if (c > f0) {
+        float d[NV];
 #pragma unroll
-    for (int n = 0; n < NS; ++n) F[5 + n] = F[IDN] > 0.f ? F[IDN] * L[5 + n] : F[IDN] * R[5 + n];
-    if (f > f0) {
-      const int64_t off = base + (int64_t)(f - 1) * st;
-      float d[NV];
+        for (int v = 0; v < NV; ++v) {
+          d[v] = A * F[v] - A * Fp[v];
+          if (!first) d[v] = dprev[v] + d[v];
+        }
+        if (last) {
+          float wc[5];
 #pragma unroll
-      for (int v = 0; v < NV; ++v) {
-        d[v] = A * F[v] - A * Fp[v];
-        if (!first) d[v] = dprev[v] + d[v];
+          for (int v = 0; v < 5; ++v) wc[v] = q[v][1];
+          finalize32<NS>(sh->fin, off, i, d, wc);
+        } else {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) D[v * svi + off] = d[v];
+        }
       }
-      if (last) {
-        float wc[5];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) wc[v] = q[v][2];
-        finalize32<NS>(g, p, b, off, i, d, wc);
-      } else {
-#pragma unroll
-        for (int v = 0; v < NV; ++v) b.D[v * sv + off] = d[v];
-      }
+      for (int v = 0; v < NV; ++v) Fp[v] = F[v];
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-      Fp[v] = F[v];
+      L[v] = H[v];
 #pragma unroll
-      for (int t = 0; t < 6; ++t) q[v][t] = q[v][t + 1];
+      for (int t = 0; t < 5; ++t) q[v][t] = q[v][t + 1];
     }
   }
 }
 
 template <int NS, int AX, int FP>
-__global__ void __launch_bounds__(128) k_march32(Geo g, Phys p, StageBufs32 b, int seglen,
-                                                 int first, int last) {
-  march32_line<NS, AX, FP>(g, p, b, seglen, first, last,
-                       (int64_t)blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>) k_march32(Geo g, Phys p, StageBufs32 b, int seglen,
+                                                    int first, int last) {
+  __shared__ Shared32 sh;
+  // (each of the copies by its own warp: they are one after the other's latency
+  // otherwise)
+  if (threadIdx.x == 0) {
+    sh.m.g = g;
+    sh.m.seglen2 = sh.m.seglen3 = seglen;
+  } else if (threadIdx.x == 32) {
+    sh.m.b = b;
+  } else if (threadIdx.x == 64) {
+    sh.p = p;
+  } else if (threadIdx.x == 96) {
+    sh.fin.set(g, p, b);
+  }
+  __syncthreads();
+  march32_line<NS, AX, FP>(&sh, first, last, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -716,106 +680,64 @@ __global__ void k_cfl32(Geo g, double gammad, int use1, int use2, int use3, cons
 // ---------------------------------------------------------------------------
 // persistent batched kernels: every CTA pulls (member, tile) items
 // ---------------------------------------------------------------------------
-// Persistent batched x1 sweep (CTA of 32 C threads, C the ensemble's tile
-// width): tiles are taken from the queue one ahead, so warp 0 stages the next
-// tile's slabs by bulk copies while the current tile's faces are computed.
+// Persistent batched x1 sweep: CTAs of one warp, the next item claimed while the
+// current one is worked on
 template <int NS, int FP>
-__global__ void __launch_bounds__(512, 2) k_x1_32_batch(const Member32* __restrict__ mem, Phys p,
-                                                        WorkQueue q, int stage, int last,
-                                                        int nc1max) {
-  extern __shared__ __align__(16) float smf[];
-  __shared__ Member32 s_mem[2];  // descriptors of the current and the next tile's member
-  __shared__ uint64_t bar;       // completion of a tile's bulk copies
-  __shared__ unsigned long long s_item;
-  const int tid = threadIdx.x;
-  // Thread 0 claims work items one tile ahead of their use: the claim of the
-  // item after next is issued while the next one is being staged, so the
-  // atomic's latency overlaps a whole tile.
-  unsigned long long ahead = 0;
-  if (tid == 0) {
-    mbar_init(&bar, 1);
-    s_item = atomicAdd(q.counter, 1ULL);
-    ahead = atomicAdd(q.counter, 1ULL);
+__global__ void __launch_bounds__(32, 20)
+    k_x1_32_batch(const Member32* __restrict__ mem, Phys p, WorkQueue q, int stage, int last) {
+  extern __shared__ float x1_rows32[];
+  __shared__ Shared32 sh;
+  const int lane = threadIdx.x;
+  unsigned long long item = 0, ahead = 0;
+  if (lane == 0) {
+    sh.p = p;
+    item = atomicAdd(q.counter, 1ULL);
   }
-  __syncthreads();
-  int m;
-  int64_t tile;
-  if (!queue_find(q, (int64_t)s_item, m, tile)) return;
-  if (tid < 32) {
-    load_member_warp(s_mem[0], mem, m);
-    if (tid == 0) set_stage32(s_mem[0].b, stage);
-    __syncwarp();
-    x1_32_stage<NS>(s_mem[0].g, s_mem[0].b, s_mem[0].x1_cols, tile * s_mem[0].x1_cols, smf,
-                    nc1max, &bar);
-  }
-  __syncthreads();
-  int buf = 0;
-  unsigned parity = 0;
+  item = __shfl_sync(0xffffffffu, item, 0);
+  int m = -1;
   while (true) {
-    const Member32& cur = s_mem[buf];
-    const int C = cur.x1_cols;
-    const int64_t col0 = tile * C;
-    bool ok = true;
-    if (tid < 32) ok = mbar_wait(&bar, parity, &snapb_x1_bulk_timeout);
-    if (tid == 0) s_item = ahead;  // the next item, claimed a tile ago
-    if (__syncthreads_or(!ok)) {
-      if (tid < 32) mbar_wait(&bar, parity, &snapb_x1_bulk_timeout);  // copies in flight
-      return;
-    }
     int nm;
-    int64_t ntile;
-    const bool more = queue_find(q, (int64_t)s_item, nm, ntile);
-    // the next tile's descriptor: the current one when the member is the same
-    const int nbuf = more && nm != m ? buf ^ 1 : buf;
-    x1_32_convert<NS>(cur.g, p, cur.b, C, col0, smf, nc1max);  // (ends with a CTA barrier)
-    if (more && tid < 32) {  // stage the next tile while this one's faces run
-      Member32& nxt = s_mem[nbuf];
-      if (nbuf != buf) {
-        load_member_warp(nxt, mem, nm);
-        if (tid == 0) set_stage32(nxt.b, stage);
-        __syncwarp();
+    int64_t tile;
+    if (!queue_find(q, (int64_t)item, nm, tile)) return;
+    if (lane == 0) ahead = atomicAdd(q.counter, 1ULL);
+    __syncwarp();  // the last item's rows and descriptor are read
+    if (nm != m) {
+      load_member_warp(sh.m, mem, nm);
+      if (lane == 0) {
+        set_stage32(sh.m.b, stage);
+        sh.fin.set(sh.m.g, p, sh.m.b);
       }
-      x1_32_stage<NS>(nxt.g, nxt.b, nxt.x1_cols, ntile * nxt.x1_cols, smf, nc1max, &bar);
-      if (tid == 0) ahead = atomicAdd(q.counter, 1ULL);  // the item after next
+      __syncwarp();
+      m = nm;
     }
-    x1_32_faces<NS, FP>(cur.g, p, cur.b, C, last, col0, smf);
-    if (!more) return;
-    __syncthreads();  // this tile's rows are read; the next descriptor is in place
-    buf = nbuf;
-    m = nm;
-    parity ^= 1;
-    tile = ntile;
-  }
-}
-
-// the x1 ghost revision of every member, kRevisionItem slots per tile
-__global__ void __launch_bounds__(256) k_x1_ghost_revision32_batch(const Member32* __restrict__ mem,
-                                                                   Phys p, WorkQueue q) {
-  int m;
-  int64_t tile;
-  while (queue_next(q, m, tile)) {
-    const Geo& g = mem[m].g;
-    const int64_t n = (int64_t)g.nc2 * g.nc3 * 2 * g.ng, s0 = tile * kRevisionItem;
-    for (int64_t slot = s0 + threadIdx.x; slot < min(s0 + kRevisionItem, n); slot += blockDim.x)
-      x1_ghost_revision32(g, p, mem[m].b, slot);
+    x1_32_item<NS, FP>(&sh, tile, x1_rows32, last);
+    item = __shfl_sync(0xffffffffu, ahead, 0);
   }
 }
 
 template <int NS, int AX, int FP>
-__global__ void __launch_bounds__(128, 6) k_march32_batch(const Member32* __restrict__ mem, Phys p,
+__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>)
+    k_march32_batch(const Member32* __restrict__ mem, Phys p,
                                                        WorkQueue q, int stage, int first,
                                                        int last) {
-  int m;
+  __shared__ Shared32 sh;
+  if (threadIdx.x == 0) sh.p = p;
+  int m, have = -1;
   int64_t tile;
-  while (queue_next(q, m, tile)) {
-    const Geo g = mem[m].g;
-    StageBufs32 b = mem[m].b;
-    set_stage32(b, stage);
-    const int seglen = AX == 2 ? mem[m].seglen2 : mem[m].seglen3;
-    const int nseg = AX == 2 ? mem[m].nseg2 : mem[m].nseg3;
-    const int64_t blk = tile / nseg;
-    const int seg = (int)(tile - blk * nseg);
-    march32_line<NS, AX, FP>(g, p, b, seglen, first, last, blk * blockDim.x + threadIdx.x, seg);
+  while (queue_next(q, m, tile)) {  // (starts with a barrier: the last tile is done)
+    if (m != have) {
+      load_member(sh.m, mem, m);
+      if (threadIdx.x == 0) {
+        set_stage32(sh.m.b, stage);
+        sh.fin.set(sh.m.g, p, sh.m.b);
+      }
+      __syncthreads();
+      have = m;
+    }
+    const int nseg = AX == 2 ? sh.m.nseg2 : sh.m.nseg3;
+    const int blk = udiv(tile, nseg);
+    march32_line<NS, AX, FP>(&sh, first, last, blk * blockDim.x + threadIdx.x,
+                             (int)tile - blk * nseg);
   }
 }
 
@@ -876,24 +798,15 @@ static cudaError_t with_ns_profile(int ns, int fp, F&& f) {
 }
 
 cudaError_t launch_x1_32_batch(const Member32* mem, const Phys& p, const WorkQueue& q,
-                               int stage, bool last, const PersistGrid& pg, size_t smem, int C,
-                               int nc1max, cudaStream_t st) {
-  const int nt = 32 * C;  // one warp per column of a tile
+                               int stage, bool last, const PersistGrid& pg, size_t smem,
+                               cudaStream_t st) {
   return with_ns_profile(p.nscalar, face_profile32(p, 1), [&](auto ns, auto fp) {
     constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
     raise_smem_limit(k_x1_32_batch<NS, FP>, 200 * 1024);
-    const int grid = persistent_grid(k_x1_32_batch<NS, FP>, nt, smem, pg);
-    k_x1_32_batch<NS, FP><<<grid, nt, smem, st>>>(mem, p, q, stage, last ? 1 : 0, nc1max);
+    const int grid = persistent_grid(k_x1_32_batch<NS, FP>, 32, smem, pg);
+    k_x1_32_batch<NS, FP><<<grid, 32, smem, st>>>(mem, p, q, stage, last ? 1 : 0);
     return cudaGetLastError();
   });
-}
-
-cudaError_t launch_x1_ghost_revision32_batch(const Member32* mem, const Phys& p,
-                                             const WorkQueue& q, const PersistGrid& pg,
-                                             cudaStream_t st) {
-  k_x1_ghost_revision32_batch<<<persistent_grid(k_x1_ghost_revision32_batch, 256, 0, pg), 256, 0,
-                                st>>>(mem, p, q);
-  return cudaGetLastError();
 }
 
 cudaError_t launch_march32_batch(int axis, const Member32* mem, const Phys& p,
@@ -928,46 +841,36 @@ cudaError_t launch_ref32(const Geo& g, const Phys& p, const double* rb, const do
   return cudaGetLastError();
 }
 
-// columns per x1 tile: a power of two (one warp per column), 8 by default
-// (the fastest measured) within about 96 KB of shared memory
-int x1_columns_pow2(int c) {
-  c = std::max(1, std::min(c, 16));  // CTAs of at most 512 threads
-  while (c & (c - 1)) c &= c - 1;
-  return c;
+// the split of the x1 sweep of one block; columns > 0 asks for that many per
+// item (as far as the shared memory goes).  A 1-D block's cells are finished by
+// the sweep itself, so its column is not cut into segments whose halos another
+// warp would be updating.
+X1Split x1_split32(const Geo& g, int nvt, bool last, int columns) {
+  X1Split sp = x1_split(g, nvt, sizeof(float), kX1RowBytes32, kX1Resident32, last);
+  if (columns > 0) {
+    const int fit = (int)((48 * 1024) / ((size_t)nvt * g.nc1 * sizeof(float)));
+    if (fit >= 1 || last) {
+      const int K = std::max(1, std::min(columns, fit));
+      sp = X1Split{K, 1, g.nx1, K * g.nc1};
+    }
+  }
+  return sp;
 }
-int x1_columns_per_cta32(const Geo& g, int nvt) {
-  size_t per = x1_smem32_per_column(g, nvt);
-  return x1_columns_pow2((int)std::min<size_t>(8, std::max<size_t>(1, (96 * 1024) / per)));
-}
-
-cudaError_t launch_x1_ghost_revision32(const Geo& g, const Phys& p, const StageBufs32& b,
-                                       cudaStream_t st) {
-  if (p.grav1 == 0.) return cudaSuccess;
-  const int64_t n = (int64_t)g.nc2 * g.nc3 * 2 * g.ng;
-  k_x1_ghost_revision32<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(g, p, b);
-  return cudaGetLastError();
-}
-
-template <int NS, int FP>
-static cudaError_t launch_x1_32t(const Geo& g, const Phys& p, const StageBufs32& b, bool last,
-                                 cudaStream_t st) {
-  const int nvt = 5 + NS;
-  int C = x1_columns_per_cta32(g, nvt);
-  size_t smem = x1_smem32_bytes(g.nc1, nvt, C);
-  if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
-  raise_smem_limit(k_x1_32<NS, FP>, 200 * 1024);
-  cudaError_t e = launch_x1_ghost_revision32(g, p, b, st);
-  if (e != cudaSuccess) return e;
-  int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  k_x1_32<NS, FP><<<(unsigned)((ncol + C - 1) / C), 32 * C, smem, st>>>(g, p, b, C,
-                                                                      last ? 1 : 0);
-  return cudaGetLastError();
+int64_t x1_items32(const Geo& g, const X1Split& sp) {
+  return ((int64_t)g.nc2 * g.nc3 + sp.K - 1) / sp.K * sp.nseg;
 }
 
 cudaError_t launch_x1_32(const Geo& g, const Phys& p, const StageBufs32& b, bool last,
                          cudaStream_t st) {
+  const int nvt = 5 + p.nscalar;
+  const X1Split sp = x1_split32(g, nvt, last, 0);
+  const size_t smem = (size_t)sp.pitch * nvt * sizeof(float);
+  if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
   return with_ns_profile(p.nscalar, face_profile32(p, 1), [&](auto ns, auto fp) {
-    return launch_x1_32t<decltype(ns)::value, decltype(fp)::value>(g, p, b, last, st);
+    constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
+    raise_smem_limit(k_x1_32<NS, FP>, 200 * 1024);
+    k_x1_32<NS, FP><<<(unsigned)x1_items32(g, sp), 32, smem, st>>>(g, p, b, sp, last ? 1 : 0);
+    return cudaGetLastError();
   });
 }
 
@@ -1039,14 +942,5 @@ cudaError_t launch_cfl32(const Geo& g, const Phys& p, const float* w, const floa
 
 }  // namespace snapb
 
-extern "C" int snapb_bulk_copy_timeouts(void) {
-  int v = 0;
-  if (cudaMemcpyFromSymbol(&v, snapb::snapb_x1_bulk_timeout, sizeof(int)) != cudaSuccess)
-    return -1;
-  if (v) {
-    const int z = 0;
-    if (cudaMemcpyToSymbol(snapb::snapb_x1_bulk_timeout, &z, sizeof(int)) != cudaSuccess)
-      return -1;
-  }
-  return v;
-}
+// No kernel waits on bulk copies any more; kept for the callers of the ABI.
+extern "C" int snapb_bulk_copy_timeouts(void) { return 0; }

@@ -21,6 +21,7 @@
 
 #include <type_traits>
 
+#include "cells.cuh"
 #include "kernels.cuh"
 #include "ring.cuh"
 
@@ -99,77 +100,6 @@ __device__ __forceinline__ void finalize_cell(const Geo& g, const Phys& p, const
     double sn = b.wgt0 * s0v + b.wgt1 * so + b.wgt2 * ds[n];
     b.s[o] = sn;
     if (b.r) b.r[o] = sn / unew_rho;
-  }
-}
-
-// ---------------------------------------------------------------------------
-// Cell-centred reconstruction: from the cells c-2 .. c+2 (q[0..4]) the value
-// at the cell's left face (wr of face c) and at its right face (wl of face
-// c+1).  The same formulas as face_states (common.cuh); for WENO5 the two
-// sides share the three smoothness measures.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ void cell_states(int type, bool scale, const double* q, double& lo,
-                                            double& hi) {
-  switch (type) {
-    case SNAPB_RECON_WENO5: {
-      double a = q[0], b = q[1], c = q[2], d = q[3], e = q[4], vs = 1.;
-      if (scale) {
-        vs = (fabs(a) + fabs(b) + fabs(c) + fabs(d) + fabs(e)) / 5.;
-        if (vs == 0.) {
-          lo = hi = 0.;
-          return;
-        }
-        const double iv = 1. / vs;
-        a *= iv, b *= iv, c *= iv, d *= iv, e *= iv;
-      }
-      const double c16 = 1. / 6., c56 = 5. / 6., c13 = 1. / 3., c116 = 11. / 6., c76 = 7. / 6.,
-                   c1312 = 13. / 12.;
-      const double s0 = sqr(c1312 * sqr(a - 2. * b + c) + 0.25 * sqr(a - 4. * b + 3. * c) + 1e-6);
-      const double s1 = sqr(c1312 * sqr(b - 2. * c + d) + 0.25 * sqr(d - b) + 1e-6);
-      const double s2 = sqr(c1312 * sqr(c - 2. * d + e) + 0.25 * sqr(3. * c - 4. * d + e) + 1e-6);
-      // alpha_k = d_k / s_k over the common denominator s0 s1 s2
-      const double s12 = s1 * s2, s01 = s0 * s1, n1 = 0.6 * (s0 * s2);
-      const double m01 = c56 * b + c13 * c, m10 = c13 * b + c56 * c;  // shared candidate parts
-      const double m23 = c56 * c + c13 * d, m32 = c13 * c + c56 * d;
-      {
-        const double n0 = 0.3 * s12, n2 = 0.1 * s01;
-        lo = vs * ((n0 * (m01 - c16 * a) + n1 * (m10 - c16 * d) +
-                    n2 * (c116 * c - c76 * d + c13 * e)) / (n0 + n1 + n2));
-      }
-      {
-        const double n0 = 0.3 * s01, n2 = 0.1 * s12;
-        hi = vs * ((n0 * (m32 - c16 * e) + n1 * (m23 - c16 * b) +
-                    n2 * (c116 * c - c76 * b + c13 * a)) / (n0 + n1 + n2));
-      }
-      break;
-    }
-    case SNAPB_RECON_CP5: {
-      const double a = -1. / 20., b = 9. / 20., c = 47. / 60., d = -13. / 60., e = 1. / 30.;
-      lo = a * q[0] + b * q[1] + c * q[2] + d * q[3] + e * q[4];
-      hi = a * q[4] + b * q[3] + c * q[2] + d * q[1] + e * q[0];
-      break;
-    }
-    case SNAPB_RECON_WENO3:
-      lo = weno3_face(q[1], q[2], q[3], scale);
-      hi = weno3_face(q[3], q[2], q[1], scale);
-      break;
-    case SNAPB_RECON_CP3: {
-      const double a = 1. / 3., b = 5. / 6., c = -1. / 6.;
-      lo = a * q[1] + b * q[2] + c * q[3];
-      hi = a * q[3] + b * q[2] + c * q[1];
-      break;
-    }
-    case SNAPB_RECON_PLM: {
-      // harmonic-mean slope with FLT_MIN guard, zeroed across extrema
-      const double dl = q[2] - q[1], dr = q[3] - q[2], d2 = dl * dr;
-      double m = 2. * d2 / (dl + dr + 1.1754943508222875e-38);
-      m = d2 >= 0. ? m : 0.;
-      lo = q[2] - 0.5 * m;
-      hi = q[2] + 0.5 * m;
-      break;
-    }
-    default:  // donor cell
-      lo = hi = q[2];
   }
 }
 
@@ -327,33 +257,11 @@ __global__ void __launch_bounds__(kMarchThreads, 4)
 // ---------------------------------------------------------------------------
 // x1 sweep
 // ---------------------------------------------------------------------------
-// Split of the x1 sweep over warps: an item is either K whole columns
-// (consecutive, so their cells are one contiguous span per variable) or one of
-// nseg segments of seglen cells of a single column.
-struct X1Split {
-  int K, nseg, seglen;
-  int pitch;  // doubles per variable row in the warp's shared memory
-};
-
-// Isentropic density and pressure of ghost level n (1 = next to the interior)
-// from the edge cell's: with a = (gamma - 1) / gamma the recurrence
-// p_{n+1}^a = p_n^a +- a g dz / K^(1/gamma) is linear in p^a, so every level
-// follows from the edge directly.  With q = p_e^(1/gamma) the other powers
-// are quotients (p_e^a = p_e / q, K^(1/gamma) = q / rho_e,
-// p^(1/gamma) = p / p^a), which leaves two pow calls per level.
-__device__ __forceinline__ void isentropic_ghost(double gamma, double gdz, int top, int n,
-                                                 double pe, double re, double& pn, double& rn) {
-  const double a = (gamma - 1.) / gamma, q = pow(pe, 1. / gamma);
-  const double h = (pe + (top ? -n : n) * a * gdz * re) / q;
-  pn = pow(h, 1. / a);
-  rn = pn / h * (re / q);
-}
-
 // Bound: FP64 issue, as the marches.  One warp per item with its own rows in
 // shared memory leaves no CTA barrier (the earlier kernel, one CTA per 16
 // columns, waited at four of them and kept face fluxes in shared memory too).
-// 384 x 384 x 192, Roe, two tracers: 4.79 -> 2.49 ms a stage; 128^3, LMARS:
-// 0.202 -> 0.106 ms; a 1-D block of 1024 cells: 43 -> 6 us.
+// 384 x 384 x 192, Roe, two tracers: 4.79 -> 2.03 ms a stage; 128^3, LMARS:
+// 0.202 -> 0.093 ms; a 1-D block of 1024 cells: 43 -> 6 us.
 template <int NS, int RP, int SV>
 __global__ void __launch_bounds__(128, 4)
     k_x1(Geo g, Phys p, StageBufs b, X1Split sp, int64_t items) {
@@ -375,25 +283,38 @@ __global__ void __launch_bounds__(128, 4)
   double* row = x1_rows + (size_t)(threadIdx.x >> 5) * NV * sp.pitch;
   const int64_t span = col0 * nc1 + lo;  // flat offset of the rows' first cell
 
-  // (1) U -> W of the item's cells (ghosts included)
-  for (int e = lane; e < K * n; e += 32) {
-    const int64_t off = span + e;
-    double uc[5], wc[5];
+  // (1) U -> W of the item's cells (ghosts included), two cells a lane at a
+  // time so that both cells' loads are in flight
+  for (int e0 = lane; e0 < K * n; e0 += 64) {
+    double uc[2][5], sc[2][NS > 0 ? NS : 1];
 #pragma unroll
-    for (int v = 0; v < 5; ++v) uc[v] = b.u[v * sv + off];
-    cons2prim_cell(uc, wc, p.gammad - 1.);
-    const int i = lo + (sp.nseg > 1 ? e : umod(e, n));
-    const bool own = (i >= c0 || bottom) && (i < c1 || top);
+    for (int h = 0; h < 2; ++h) {
+      const int64_t off = span + min(e0 + 32 * h, K * n - 1);
 #pragma unroll
-    for (int v = 0; v < 5; ++v) {
-      row[v * sp.pitch + e] = wc[v];
-      if (own) b.w[v * sv + off] = wc[v];
+      for (int v = 0; v < 5; ++v) uc[h][v] = b.u[v * sv + off];
+#pragma unroll
+      for (int m = 0; m < NS; ++m) sc[h][m] = b.s[m * sv + off];
     }
 #pragma unroll
-    for (int m = 0; m < NS; ++m) {
-      const double rr = b.s[m * sv + off] / uc[IDN];
-      row[(5 + m) * sp.pitch + e] = rr;
-      if (own) b.R[m * sv + off] = rr;
+    for (int h = 0; h < 2; ++h) {
+      const int e = e0 + 32 * h;
+      if (e >= K * n) break;
+      const int64_t off = span + e;
+      double wc[5];
+      cons2prim_cell(uc[h], wc, p.gammad - 1.);
+      const int i = lo + (sp.K > 1 ? umod(e, n) : e);
+      const bool own = (i >= c0 || bottom) && (i < c1 || top);
+#pragma unroll
+      for (int v = 0; v < 5; ++v) {
+        row[v * sp.pitch + e] = wc[v];
+        if (own) b.w[v * sv + off] = wc[v];
+      }
+#pragma unroll
+      for (int m = 0; m < NS; ++m) {
+        const double rr = sc[h][m] / uc[h][IDN];
+        row[(5 + m) * sp.pitch + e] = rr;
+        if (own) b.R[m * sv + off] = rr;
+      }
     }
   }
   __syncwarp();
@@ -426,14 +347,17 @@ __global__ void __launch_bounds__(128, 4)
   double Hc[NV], Fc[NV], rc = 0.;  // lane 0: lane 31 of the previous round
 #pragma unroll
   for (int v = 0; v < NV; ++v) Hc[v] = Fc[v] = 0.;
+  // which of the item's columns are interior ones
+  bool inner = lane < K;
+  if (inner) {
+    const int j = umod(col0 + lane, g.nc2), k = udiv(col0 + lane, g.nc2);
+    inner = j >= g.jl && j <= g.ju && k >= g.kl && k <= g.ku;
+  }
+  const unsigned columns = __ballot_sync(0xffffffffu, inner);
   int kk = lane / nn, t = lane - kk * nn;
   const int total = K * nn;
   for (int s0 = 0; s0 < total; s0 += 32) {
-    bool act = s0 + lane < total;
-    if (act) {
-      const int j = umod(col0 + kk, g.nc2), k = udiv(col0 + kk, g.nc2);
-      act = j >= g.jl && j <= g.ju && k >= g.kl && k <= g.ku;
-    }
+    const bool act = s0 + lane < total && (columns >> kk & 1);
     if (__any_sync(0xffffffffu, act)) {
       const int c = c0 - 1 + t;
       const double* cell = row + (act ? kk * n + c - lo : 2);
