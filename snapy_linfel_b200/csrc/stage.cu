@@ -40,80 +40,83 @@ __global__ void k_c2p_r(Geo g, Phys p, StageBufs b) {
 // ---------------------------------------------------------------------------
 // diffusion (src/forcing/diffusion.cpp:152-240), uniform Cartesian
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ int64_t axis_stride(const Geo& g, int a) {
-  return a == 0 ? (int64_t)1 : (a == 1 ? g.s2 : g.s3);
-}
-__device__ __forceinline__ double axis_dx(const Geo& g, int a) {
-  return a == 0 ? g.dx1 : (a == 1 ? g.dx2 : g.dx3);
-}
-__device__ __forceinline__ bool axis_active(const Geo& g, int a) {
-  return a == 0 ? g.nc1 > 1 : (a == 1 ? g.nc2 > 1 : g.nc3 > 1);
-}
-
-__device__ double div_vel(const Geo& g, const double* w, int64_t t) {
-  double dv = 0.;
-  for (int a = 0; a < 3; ++a) {
-    if (!axis_active(g, a)) continue;
-    int64_t s = axis_stride(g, a);
-    const double* v = w + (IVX + a) * g.sv;
-    dv += (v[t + s] - v[t - s]) / (2. * axis_dx(g, a));
+// Isotropic viscosity and heat conduction of the block's active axes (AXES, a
+// bit mask), one thread per cell.  With the axes known at compile time every
+// loop unrolls, the velocity gradients and temperatures that the cell's faces
+// share are formed once, and the spacings enter as reciprocals.  Bound: loads
+// in flight (34 of the neighbourhood) and FP64 issue.  1024 x 128 cells: 20.4
+// us with run-time axes and quotients -> 8.6 us.
+template <int AXES>
+struct DiffCell {
+  const double* w;
+  int64_t sv, st[3];
+  double i1[3], i2[3];  // 1 / dx, 1 / (2 dx)
+  static constexpr bool on(int a) { return AXES >> a & 1; }
+  __device__ __forceinline__ double slope(int v, int a, int64_t t) const {
+    return (w[v * sv + t + st[a]] - w[v * sv + t - st[a]]) * i2[a];
   }
-  return dv;
-}
-
-// viscous + conductive flux at the face between t - s_a and t
-__device__ void diff_face(const Geo& g, const Phys& p, const double* w, int a, int64_t t,
-                          double* F) {
-  const int64_t sv = g.sv;
-  const int64_t s = axis_stride(g, a);
-  const double dxa = axis_dx(g, a);
-  const double* rho = w + IDN * sv;
+  __device__ __forceinline__ double div(int64_t t) const {
+    double d = 0.;
 #pragma unroll
-  for (int v = 0; v < 5; ++v) F[v] = 0.;
-  double rho_face = 0.5 * (rho[t] + rho[t - s]);
-  if (p.nu > 0.) {
-    double div_face = 0.5 * (div_vel(g, w, t) + div_vel(g, w, t - s));
-    const double* va = w + (IVX + a) * sv;
-    for (int bb = 0; bb < 3; ++bb) {
-      const double* vb = w + (IVX + bb) * sv;
-      double stress = (vb[t] - vb[t - s]) / dxa;
-      if (bb == a) {
-        stress = 2. * stress - (2. / 3.) * div_face;
-      } else if (axis_active(g, bb)) {
-        int64_t sb = axis_stride(g, bb);
-        double dxb = axis_dx(g, bb);
-        double d0 = (va[t + sb] - va[t - sb]) / (2. * dxb);
-        double d1 = (va[t - s + sb] - va[t - s - sb]) / (2. * dxb);
-        stress += 0.5 * (d0 + d1);
+    for (int a = 0; a < 3; ++a)
+      if (on(a)) d += slope(IVX + a, a, t);
+    return d;
+  }
+  // viscous + conductive flux at the face between t - s_a and t
+  __device__ __forceinline__ void face(const Phys& p, int a, int64_t t, double div0, double div1,
+                                       double T0, double T1, double cv, double* F) const {
+    const int64_t s = st[a];
+    const double rho0 = w[IDN * sv + t], rho1 = w[IDN * sv + t - s];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) F[v] = 0.;
+    const double rho_face = 0.5 * (rho0 + rho1);
+    if (p.nu > 0.) {
+      const double div_face = 0.5 * (div0 + div1);
+#pragma unroll
+      for (int bb = 0; bb < 3; ++bb) {
+        const double v0 = w[(IVX + bb) * sv + t], v1 = w[(IVX + bb) * sv + t - s];
+        double stress = (v0 - v1) * i1[a];
+        if (bb == a)
+          stress = 2. * stress - (2. / 3.) * div_face;
+        else if (on(bb))
+          stress += 0.5 * (slope(IVX + a, bb, t) + slope(IVX + a, bb, t - s));
+        const double m = -p.nu * rho_face * stress;
+        F[IVX + bb] = m;
+        F[IPR] += 0.5 * (v0 + v1) * m;
       }
-      double m = -p.nu * rho_face * stress;
-      F[IVX + bb] = m;
-      F[IPR] += 0.5 * (vb[t] + vb[t - s]) * m;
     }
+    if (p.kappa > 0.) F[IPR] -= p.kappa * (0.5 * (rho0 * cv + rho1 * cv)) * ((T0 - T1) * i1[a]);
   }
-  if (p.kappa > 0.) {
-    const double* pr = w + IPR * sv;
-    double cv = p.rgas / (p.gammad - 1.);
-    double T0 = pr[t] / (rho[t] * p.rgas), T1 = pr[t - s] / (rho[t - s] * p.rgas);
-    F[IPR] -= p.kappa * (0.5 * (rho[t] * cv + rho[t - s] * cv)) * ((T0 - T1) / dxa);
-  }
-}
+};
 
-__global__ void k_diff(Geo g, Phys p, StageBufs b) {
+template <int AXES>
+__global__ void __launch_bounds__(128) k_diff(Geo g, Phys p, StageBufs b) {
   const int ni = g.iu - g.il + 1, nj = g.ju - g.jl + 1, nk = g.ku - g.kl + 1;
-  int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (tid >= (int64_t)ni * nj * nk) return;
-  int i = g.il + umod(tid, ni);
-  int j = g.jl + umod(udiv(tid, ni), nj);
-  int k = g.kl + udiv(tid, (int64_t)ni * nj);
-  int64_t t = (int64_t)k * g.s3 + (int64_t)j * g.s2 + i;
+  const int i = g.il + umod(tid, ni);
+  const int j = g.jl + umod(udiv(tid, ni), nj);
+  const int k = g.kl + udiv(tid, (int64_t)ni * nj);
+  const int64_t t = (int64_t)k * g.s3 + (int64_t)j * g.s2 + i;
+  using D = DiffCell<AXES>;
+  D c;
+  c.w = b.w;
+  c.sv = g.sv;
+  c.st[0] = 1, c.st[1] = g.s2, c.st[2] = g.s3;
+  const double dx[3] = {g.dx1, g.dx2, g.dx3}, A[3] = {g.A1, g.A2, g.A3};
+#pragma unroll
+  for (int a = 0; a < 3; ++a) c.i1[a] = 1. / dx[a], c.i2[a] = 1. / (2. * dx[a]);
+  const double cv = p.rgas / (p.gammad - 1.);
+  auto temp = [&](int64_t o) { return b.w[IPR * g.sv + o] / (b.w[IDN * g.sv + o] * p.rgas); };
+  const double dc = c.div(t), Tc = temp(t);
   double acc[5] = {0., 0., 0., 0., 0.};
-  const double A[3] = {g.A1, g.A2, g.A3};
+#pragma unroll
   for (int a = 0; a < 3; ++a) {
-    if (!axis_active(g, a)) continue;
+    if (!D::on(a)) continue;
+    const int64_t s = c.st[a];
     double Fm[5], Fp[5];
-    diff_face(g, p, b.w, a, t, Fm);
-    diff_face(g, p, b.w, a, t + axis_stride(g, a), Fp);
+    c.face(p, a, t, dc, c.div(t - s), Tc, temp(t - s), cv, Fm);
+    c.face(p, a, t + s, c.div(t + s), dc, temp(t + s), Tc, cv, Fp);
 #pragma unroll
     for (int v = 0; v < 5; ++v) acc[v] += A[a] * Fp[v] - A[a] * Fm[v];
   }
@@ -309,8 +312,18 @@ cudaError_t launch_march(int axis, const Geo& g, const Phys& p, const StageBufs&
 }
 
 cudaError_t launch_diffusion(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
-  int64_t n = (int64_t)(g.iu - g.il + 1) * (g.ju - g.jl + 1) * (g.ku - g.kl + 1);
-  k_diff<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(g, p, b);
+  const int64_t n = (int64_t)(g.iu - g.il + 1) * (g.ju - g.jl + 1) * (g.ku - g.kl + 1);
+  const unsigned grid = (unsigned)((n + 127) / 128);
+  switch ((g.nc1 > 1 ? 1 : 0) | (g.nc2 > 1 ? 2 : 0) | (g.nc3 > 1 ? 4 : 0)) {
+    case 0: k_diff<0><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 1: k_diff<1><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 2: k_diff<2><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 3: k_diff<3><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 4: k_diff<4><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 5: k_diff<5><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 6: k_diff<6><<<grid, 128, 0, st>>>(g, p, b); break;
+    case 7: k_diff<7><<<grid, 128, 0, st>>>(g, p, b); break;
+  }
   return cudaGetLastError();
 }
 

@@ -105,3 +105,12 @@ def test_fp32_sweeps_match_fp64(nx, riemann, nscalar):
         sa, sb = m32.scalar_s.double().cpu().numpy(), m64.scalar_s.cpu().numpy()
         assert_finite(sa)
         assert np.max(np.abs(sa - sb)) < 1e-5 * np.max(np.abs(sb))
+
+
+@pytest.mark.parametrize("nu,kappa", [(0.02, 0.0), (0.0, 0.03), (0.02, 0.03)])
+@pytest.mark.parametrize("nx", [(40, 1, 1), (1, 33, 1), (9, 17, 1), (1, 1, 21), (11, 1, 13),
+                                (1, 9, 12), (12, 7, 19)])
+def test_diffusion_axes(oracle, nx, nu, kappa):
+    """every set of active axes of the diffusive fluxes"""
+    _check(oracle, nx, nu_iso=nu, kappa_iso=kappa,
+           bc=("reflecting",) * 2 + ("periodic",) * 4)
