@@ -103,124 +103,54 @@ cudaError_t launch_bc(const Geo& g, const snapb_hydro_config& c, double* var, in
 }
 
 // ---------------------------------------------------------------------------
-// CFL limit (src/hydro/hydro.cpp:118-180).  slots[0..2] receive the per-axis
-// minima as ordered 64-bit patterns (all candidates are positive doubles).
+// CFL limit (src/hydro/hydro.cpp:118-180).  A thread keeps the largest signal
+// speed per axis and divides once (cfl32_speeds, kernels.cuh: the quotient is
+// monotone, so the minimum is the same to the bit).  Bound: HBM (70 % of the
+// copy rate); 384 x 384 x 192: 386 us with a division per cell and axis -> 246.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ double warp_min(double x) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) x = fmin(x, __shfl_xor_sync(0xffffffffu, x, o));
-  return x;
+__global__ void __launch_bounds__(256) k_cfl(Geo g, double gammad, CflUse use, const double* w,
+                                             unsigned long long* slots, double* dt_out) {
+  double a1 = 0., a2 = 0., a3 = 0.;
+  cfl_cells(g, [&](int64_t o, int) {
+    const double rho = w[IDN * g.sv + o], pr = w[IPR * g.sv + o];
+    const double cs = sqrt(gammad * pr / rho);
+    if (use.use1) a1 = fmax(a1, fabs(w[IVX * g.sv + o]) + cs);
+    if (use.use2) a2 = fmax(a2, fabs(w[IVY * g.sv + o]) + cs);
+    if (use.use3) a3 = fmax(a3, fabs(w[IVZ * g.sv + o]) + cs);
+  });
+  cfl_finish(use, fmin(DBL_MAX, g.dx1 / a1), fmin(DBL_MAX, g.dx2 / a2), fmin(DBL_MAX, g.dx3 / a3),
+             slots, dt_out);
 }
 
-__global__ void k_cfl(Geo g, double gammad, int use1, int use2, int use3, const double* w,
-                      unsigned long long* slots) {
-  const int ni = g.iu - g.il + 1, nj = g.ju - g.jl + 1, nk = g.ku - g.kl + 1;
-  const int64_t n = (int64_t)ni * nj * nk;
-  double m1 = DBL_MAX, m2 = DBL_MAX, m3 = DBL_MAX;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    int i = g.il + umod(t, ni);
-    int j = g.jl + umod(udiv(t, ni), nj);
-    int k = g.kl + udiv(t, (int64_t)ni * nj);
-    int64_t o = (int64_t)k * g.s3 + (int64_t)j * g.s2 + i;
-    double rho = w[IDN * g.sv + o], pr = w[IPR * g.sv + o];
-    double cs = sqrt(gammad * pr / rho);
-    if (use1) m1 = fmin(m1, g.dx1 / (fabs(w[IVX * g.sv + o]) + cs));
-    if (use2) m2 = fmin(m2, g.dx2 / (fabs(w[IVY * g.sv + o]) + cs));
-    if (use3) m3 = fmin(m3, g.dx3 / (fabs(w[IVZ * g.sv + o]) + cs));
+CflUse cfl_use(const Geo& g, const Phys& p) {
+  const int scheme = p.implicit_scheme;
+  CflUse u{g.nc1 > 1, g.nc2 > 1, g.nc3 > 1, -1.};
+  if (scheme != 0) {
+    u.use1 = u.use1 && (!(scheme & 1) || (g.nc3 == 1 && g.nc2 == 1));
+    u.use2 = u.use2 && !((scheme >> 1) & 1);
+    u.use3 = u.use3 && !((scheme >> 2) & 1);
   }
-  __shared__ double red[3][32];
-  m1 = warp_min(m1);
-  m2 = warp_min(m2);
-  m3 = warp_min(m3);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) {
-    red[0][wid] = m1;
-    red[1][wid] = m2;
-    red[2][wid] = m3;
+  const double coeff = fmax(p.nu, p.kappa);
+  if (coeff > 0.) {
+    int ndim = 0;
+    double dxm = DBL_MAX;
+    if (g.nc1 > 1) ++ndim, dxm = fmin(dxm, g.dx1);
+    if (g.nc2 > 1) ++ndim, dxm = fmin(dxm, g.dx2);
+    if (g.nc3 > 1) ++ndim, dxm = fmin(dxm, g.dx3);
+    if (ndim > 0) u.dt_diff = dxm * dxm / (2. * ndim * coeff);
   }
-  __syncthreads();
-  if (wid == 0) {
-    int nw = blockDim.x >> 5;
-    m1 = lane < nw ? red[0][lane] : DBL_MAX;
-    m2 = lane < nw ? red[1][lane] : DBL_MAX;
-    m3 = lane < nw ? red[2][lane] : DBL_MAX;
-    m1 = warp_min(m1);
-    m2 = warp_min(m2);
-    m3 = warp_min(m3);
-    if (lane == 0) {
-      atomicMin(&slots[0], (unsigned long long)__double_as_longlong(m1));
-      atomicMin(&slots[1], (unsigned long long)__double_as_longlong(m2));
-      atomicMin(&slots[2], (unsigned long long)__double_as_longlong(m3));
-    }
-  }
-}
-
-__global__ void k_cfl_final(const unsigned long long* slots, int use1, int use2, int use3,
-                            double dt_diff, double* dt_out) {
-  double d1 = use1 ? __longlong_as_double((long long)slots[0]) : 1.e9;
-  double d2 = use2 ? __longlong_as_double((long long)slots[1]) : 1.e9;
-  double d3 = use3 ? __longlong_as_double((long long)slots[2]) : 1.e9;
-  double dt = fmin(d1, fmin(d2, d3));
-  if (dt_diff > 0.) dt = fmin(dt, dt_diff);
-  *dt_out = dt;
-}
-
-__global__ void k_fill_ull(unsigned long long* p, int n, unsigned long long v) {
-  if ((int)threadIdx.x < n) p[threadIdx.x] = v;
+  return u;
 }
 
 cudaError_t launch_cfl(const Geo& g, const Phys& p, const double* w, double* slots,
                        double* dt_out, cudaStream_t st) {
-  int scheme = p.implicit_scheme;
-  int use1 = g.nc1 > 1, use2 = g.nc2 > 1, use3 = g.nc3 > 1;
-  if (scheme != 0) {
-    use1 = use1 && (!(scheme & 1) || (g.nc3 == 1 && g.nc2 == 1));
-    use2 = use2 && !((scheme >> 1) & 1);
-    use3 = use3 && !((scheme >> 2) & 1);
-  }
-  double dt_diff = -1.;
-  double coeff = fmax(p.nu, p.kappa);
-  if (coeff > 0.) {
-    int ndim = 0;
-    double dxm = DBL_MAX;
-    if (g.nc1 > 1) ++ndim, dxm = fmin(dxm, g.dx1);
-    if (g.nc2 > 1) ++ndim, dxm = fmin(dxm, g.dx2);
-    if (g.nc3 > 1) ++ndim, dxm = fmin(dxm, g.dx3);
-    if (ndim > 0) dt_diff = dxm * dxm / (2. * ndim * coeff);
-  }
   auto* sl = reinterpret_cast<unsigned long long*>(slots);
-  double big = DBL_MAX;
-  unsigned long long big_bits;
-  std::memcpy(&big_bits, &big, sizeof(big));
-  k_fill_ull<<<1, 32, 0, st>>>(sl, 3, big_bits);
-  int64_t n = (int64_t)(g.iu - g.il + 1) * (g.ju - g.jl + 1) * (g.ku - g.kl + 1);
-  int blocks = (int)std::min<int64_t>((n + 255) / 256, 148 * 8);
-  k_cfl<<<blocks, 256, 0, st>>>(g, p.gammad, use1, use2, use3, w, sl);
-  k_cfl_final<<<1, 1, 0, st>>>(sl, use1, use2, use3, dt_diff, dt_out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_cfl_final(const Geo& g, const Phys& p, unsigned long long* slots,
-                             double* dt_out, cudaStream_t st) {
-  int scheme = p.implicit_scheme;
-  int use1 = g.nc1 > 1, use2 = g.nc2 > 1, use3 = g.nc3 > 1;
-  if (scheme != 0) {
-    use1 = use1 && (!(scheme & 1) || (g.nc3 == 1 && g.nc2 == 1));
-    use2 = use2 && !((scheme >> 1) & 1);
-    use3 = use3 && !((scheme >> 2) & 1);
+  const int blocks = cfl_blocks(g);
+  if (blocks > 1) {
+    const cudaError_t e = cudaMemsetAsync(sl, 0xff, 4 * sizeof(*sl), st);
+    if (e != cudaSuccess) return e;
   }
-  double dt_diff = -1.;
-  double coeff = fmax(p.nu, p.kappa);
-  if (coeff > 0.) {
-    int ndim = 0;
-    double dxm = DBL_MAX;
-    if (g.nc1 > 1) ++ndim, dxm = fmin(dxm, g.dx1);
-    if (g.nc2 > 1) ++ndim, dxm = fmin(dxm, g.dx2);
-    if (g.nc3 > 1) ++ndim, dxm = fmin(dxm, g.dx3);
-    if (ndim > 0) dt_diff = dxm * dxm / (2. * ndim * coeff);
-  }
-  k_cfl_final<<<1, 1, 0, st>>>(slots, use1, use2, use3, dt_diff, dt_out);
+  k_cfl<<<blocks, 256, 0, st>>>(g, p.gammad, cfl_use(g, p), w, sl, dt_out);
   return cudaGetLastError();
 }
 

@@ -114,3 +114,32 @@ def test_diffusion_axes(oracle, nx, nu, kappa):
     """every set of active axes of the diffusive fluxes"""
     _check(oracle, nx, nu_iso=nu, kappa_iso=kappa,
            bc=("reflecting",) * 2 + ("periodic",) * 4)
+
+
+@pytest.mark.parametrize("nx", [(3, 1, 1), (300, 1, 1), (16, 16, 16), (17, 241, 1), (64, 65, 1),
+                                (5, 60, 41), (129, 7, 9), (200, 90, 80)])
+def test_time_step_reduction(nx):
+    """the CFL limit by one CTA, by many, and over several rounds of the grid;
+    a cell without a finite speed does not count.  FP64: the same operations in
+    the same order, within 2 ulp; FP32 speeds: within 4 FP32 ulp."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from snapy_linfel_b200.mesh import MeshBlock, MeshBlockF32
+
+    cfg = make_config(nx1=nx[0], nx2=nx[1], nx3=nx[2], x1=(0.0, 0.1 * nx[0]),
+                      x2=(0.0, 0.13 * nx[1]), x3=(0.0, 0.17 * nx[2]))
+    opts = MeshBlockOptions(cfg, Integration(cfl=1.0))
+    w = random_prim(np.random.default_rng(sum(nx)), cfg.shape)
+    m64, m32 = MeshBlock(opts), MeshBlockF32(opts)
+    m64.initialize(w)
+    m32.initialize(w, reference=None)
+    k, j, i = (n // 2 for n in w.shape[1:])
+    w[0, k, j, i] = np.nan
+    ng = [(n - m) // 2 for n, m in zip(w.shape[1:], nx[::-1])]
+    v = w[(slice(None),) + tuple(slice(g, n - g) for g, n in zip(ng, w.shape[1:]))]
+    cs = np.sqrt(cfg.gammad * v[4] / v[0])
+    dt = min(np.nanmin(d / (np.abs(v[1 + a]) + cs))
+             for a, (d, n) in enumerate(zip((0.1, 0.13, 0.17), nx)) if n > 1)
+    for m, tol in ((m64, 5e-16), (m32, 5e-7)):
+        m.hydro_w.copy_(torch.from_numpy(w))
+        assert abs(float(m.max_time_step()) / dt - 1.0) < tol
