@@ -18,7 +18,7 @@ OUT = os.path.join(HERE, "libsnapb.so")
 BUILD = os.path.join(HERE, "_build")
 SOURCES = ["capi.cu", "stage.cu", "vic.cu", "aux.cu", "stage32.cu", "capi32.cu", "adjoint.cu", "ensemble.cu", "totals.cu", "halo.cu", "vicf.cu", "vic_cr.cu",
            "vic_chunk.cu", "vic_pair5.cu",
-           "vadj_chunk.cu"]
+           "vadj_chunk.cu", "adj_march.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
          "-Xptxas", "-warn-spills"]

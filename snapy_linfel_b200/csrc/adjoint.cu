@@ -43,6 +43,8 @@
 
 #include "dual.cuh"
 #include "kernels.cuh"
+#include "adj_bufs.cuh"
+#include "cells_adj.cuh"
 #include "vadj_chunk.cuh"
 #include "ring.cuh"
 #include "riemann_adj.cuh"
@@ -254,63 +256,6 @@ __global__ void k_mask_interior(Geo g, const double* src, double* dst, int nv) {
 // Local reverse maps
 // ---------------------------------------------------------------------------
 
-// WENO5-JS face value (weno5_face) reversed by hand: g * d out / d (a..e),
-// accumulated into gx[0..4].  With omega_k = alpha_k / sum(alpha):
-//   d out / d p_k = omega_k,  d out / d beta_k = -2 omega_k (p_k - out) / (beta_k + eps);
-// the mean-|phi| scaling adds sign(x_i)/5 * (W - sum_j y_j dW/dy_j).
-__device__ __forceinline__ void weno5_face_vjp(double a, double b, double c, double d, double e,
-                                               bool scale, double g, double* gx) {
-  double x[5] = {a, b, c, d, e};
-  double vs = 1.;
-  if (scale) {
-    vs = (fabs(a) + fabs(b) + fabs(c) + fabs(d) + fabs(e)) / 5.;
-    if (vs == 0.) return;  // the forward returns the constant 0
-    double iv = 1. / vs;
-#pragma unroll
-    for (int q = 0; q < 5; ++q) x[q] *= iv;
-  }
-  const double c16 = 1. / 6., c56 = 5. / 6., c13 = 1. / 3.;
-  const double c116 = 11. / 6., c76 = 7. / 6., c1312 = 13. / 12.;
-  double y0 = x[0], y1 = x[1], y2 = x[2], y3 = x[3], y4 = x[4];
-  double p0 = -c16 * y0 + c56 * y1 + c13 * y2;
-  double p1 = c13 * y1 + c56 * y2 - c16 * y3;
-  double p2 = c116 * y2 - c76 * y3 + c13 * y4;
-  double u0 = y0 - 2. * y1 + y2, v0 = y0 - 4. * y1 + 3. * y2;
-  double u1 = y1 - 2. * y2 + y3, v1 = y3 - y1;
-  double u2 = y2 - 2. * y3 + y4, v2 = 3. * y2 - 4. * y3 + y4;
-  double b0 = c1312 * u0 * u0 + 0.25 * v0 * v0;
-  double b1 = c1312 * u1 * u1 + 0.25 * v1 * v1;
-  double b2 = c1312 * u2 * u2 + 0.25 * v2 * v2;
-  double e0 = b0 + 1e-6, e1 = b1 + 1e-6, e2 = b2 + 1e-6;
-  double a0 = 0.3 / (e0 * e0), a1 = 0.6 / (e1 * e1), a2 = 0.1 / (e2 * e2);
-  double is = 1. / (a0 + a1 + a2);
-  double o0 = a0 * is, o1 = a1 * is, o2 = a2 * is;
-  double W = o0 * p0 + o1 * p1 + o2 * p2;
-  double gb0 = -2. * o0 * (p0 - W) / e0;
-  double gb1 = -2. * o1 * (p1 - W) / e1;
-  double gb2 = -2. * o2 * (p2 - W) / e2;
-  const double k13 = 13. / 6.;
-  double gy[5];
-  gy[0] = -c16 * o0 + gb0 * (k13 * u0 + 0.5 * v0);
-  gy[1] = c56 * o0 + c13 * o1 + gb0 * (-2. * k13 * u0 - 2. * v0) + gb1 * (k13 * u1 - 0.5 * v1);
-  gy[2] = c13 * o0 + c56 * o1 + c116 * o2 + gb0 * (k13 * u0 + 1.5 * v0) +
-          gb1 * (-2. * k13 * u1) + gb2 * (k13 * u2 + 1.5 * v2);
-  gy[3] = -c16 * o1 - c76 * o2 + gb1 * (k13 * u1 + 0.5 * v1) + gb2 * (-2. * k13 * u2 - 2. * v2);
-  gy[4] = c13 * o2 + gb2 * (k13 * u2 + 0.5 * v2);
-  if (!scale) {
-#pragma unroll
-    for (int q = 0; q < 5; ++q) gx[q] += g * gy[q];
-    return;
-  }
-  double ydw = 0.;
-#pragma unroll
-  for (int q = 0; q < 5; ++q) ydw += x[q] * gy[q];
-  double corr = (W - ydw) / 5.;
-  double raw[5] = {a, b, c, d, e};
-#pragma unroll
-  for (int q = 0; q < 5; ++q) gx[q] += g * (gy[q] + (raw[q] < 0. ? -corr : corr));
-}
-
 // g_L * dL/dq + g_R * dR/dq of face_states over the six-cell window
 __device__ __forceinline__ void face_states_vjp(int type, bool scale, const double* q, double gl,
                                                 double gr, double* gq) {
@@ -371,86 +316,10 @@ __device__ __forceinline__ void face_states_vjp(int type, bool scale, const doub
   }
 }
 
-// Reverse of one face: window q (cells f-3 .. f+2) of the nvar primitives and
-// the ns mixing ratios, the cotangent gFin of its nvar + ns fluxes; adds the
-// window cotangents into gq.  rev_l / rev_r: the x1 hydrostatic face
-// revisions (left state takes the right state's p, rho at the lower boundary
-// face, and the converse at the upper one).
-template <int NS>
-__device__ __forceinline__ void face_vjp(const Phys& p, int rtype, int rshock, int rscale, int ivx,
-                                         bool disabled, bool rev_l, bool rev_r,
-                                         const double (&q)[5 + NS][6],
-                                         const double (&gFin)[5 + NS], double (&gq)[5 + NS][6]) {
-  constexpr int NV = 5 + NS;
-  double L[NV], R[NV], Lraw[NV > 5 ? NV : 6], Rraw[NV > 5 ? NV : 6];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (v < 5) {
-      int typ = (rshock || v == IDN) ? rtype : interp2_of(rtype);
-      face_states(typ, rscale != 0, q[v], L[v], R[v]);
-    } else {
-      face_states(p.rs_type, p.rs_scale != 0, q[v], Lraw[v], Rraw[v]);
-      L[v] = Lraw[v] < 0. ? 0. : Lraw[v];
-      R[v] = Rraw[v] < 0. ? 0. : Rraw[v];
-    }
-  }
-  if (rev_l) {
-    L[IPR] = R[IPR];
-    L[IDN] = R[IDN];
-  }
-  if (rev_r) {
-    R[IPR] = L[IPR];
-    R[IDN] = L[IDN];
-  }
-  double gL[NV], gR[NV];
-#pragma unroll
-  for (int v = 0; v < NV; ++v) gL[v] = gR[v] = 0.;
-  if (!disabled) {
-    double F[5];
-    riemann_flux(p.riemann, L, R, ivx, p.gammad, F);
-    double gF[5];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) gF[v] = gFin[v];
-    // scalar upwind flux F_s = F[IDN] * (F[IDN] > 0 ? r_L : r_R)
-#pragma unroll
-    for (int n = 0; n < NS; ++n) {
-      double gs = gFin[5 + n];
-      if (F[IDN] > 0.) {
-        gF[IDN] += gs * L[5 + n];
-        gL[5 + n] = gs * F[IDN];
-      } else {
-        gF[IDN] += gs * R[5 + n];
-        gR[5 + n] = gs * F[IDN];
-      }
-    }
-    riemann_vjp_rev(p.riemann, L, R, ivx, p.gammad, gF, gL, gR);
-  }
-  if (rev_l) {
-    gR[IPR] += gL[IPR];
-    gL[IPR] = 0.;
-    gR[IDN] += gL[IDN];
-    gL[IDN] = 0.;
-  }
-  if (rev_r) {
-    gL[IPR] += gR[IPR];
-    gR[IPR] = 0.;
-    gL[IDN] += gR[IDN];
-    gR[IDN] = 0.;
-  }
-#pragma unroll
-  for (int v = 0; v < NV; ++v) {
-    if (v < 5) {
-      int typ = (rshock || v == IDN) ? rtype : interp2_of(rtype);
-      face_states_vjp(typ, rscale != 0, q[v], gL[v], gR[v], gq[v]);
-    } else {
-      double gl = Lraw[v] < 0. ? 0. : gL[v];
-      double gr = Rraw[v] < 0. ? 0. : gR[v];
-      face_states_vjp(p.rs_type, p.rs_scale != 0, q[v], gl, gr, gq[v]);
-    }
-  }
-}
-
-// The same reverse for an x1 face whose window lives in shared memory (wb:
+// Reverse of one x1 face (the cotangent gFin of its nvar + ns fluxes; rev_l /
+// rev_r: the hydrostatic face revisions, where the left state takes the right
+// state's p, rho at the lower boundary face, and the converse at the upper
+// one) whose window lives in shared memory (wb:
 // the column's NV rows of nc1 cells); the window cotangents are added into the
 // column's shared accumulator gb with shared-memory atomics, so no per-face
 // array of contributions is held in registers.
@@ -536,103 +405,6 @@ __device__ __forceinline__ void face_vjp_smem(const Phys& p, int rtype, int rsho
   }
 }
 
-// Buffers of the stage adjoint (all [var][sv], FP64)
-struct AdjBufs {
-  const double* dt;
-  const double* u;   // stage-start state (ghosts filled)
-  const double* s;
-  const double* W;   // primitives of u with the x1 ghost revision (recomputed)
-  const double* R;   // mixing ratios s / rho (recomputed)
-  const double* D;   // explicit du (recomputed; implicit solve only)
-  double* GD;        // cotangent of du (nvar + ns); rows replaced by the VIC adjoint
-  double* GW;        // cotangent of w (nvar) and r (ns), accumulated
-  double* gu;        // out: += cotangent of u
-  double* gs;        // out: += cotangent of s
-  double* vic;       // VIC adjoint scratch
-};
-
-// ---------------------------------------------------------------------------
-// x2 / x3 faces: one thread per (x1 cell, other index) and segment of faces
-// ---------------------------------------------------------------------------
-template <int NS, int AX>
-__global__ void __launch_bounds__(128) k_march_adj(Geo g, Phys p, AdjBufs b, int seglen) {
-  constexpr int NV = 5 + NS;
-  const int ni = g.iu - g.il + 1;
-  int lo, hi, olo, ohi;
-  int64_t st, ost;
-  if (AX == 2) {
-    lo = g.jl, hi = g.ju, st = g.s2, olo = g.kl, ohi = g.ku, ost = g.s3;
-  } else {
-    lo = g.kl, hi = g.ku, st = g.s3, olo = g.jl, ohi = g.ju, ost = g.s2;
-  }
-  const int no = ohi - olo + 1;
-  const int64_t tid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (tid >= (int64_t)ni * no) return;
-  const int i = g.il + umod(tid, ni);
-  const int o = olo + udiv(tid, ni);
-  const int f0 = lo + blockIdx.y * seglen;
-  if (f0 > hi + 1) return;
-  const int f1 = min(f0 + seglen - 1, hi + 1);
-  const int64_t base = i + o * ost;
-  const int64_t sv = g.sv;
-  const int ivx = AX == 2 ? IVY : IVZ;
-  const double A = AX == 2 ? g.A2 : g.A3;
-  const int disabled = AX == 2 ? p.disable2 : p.disable3;
-  const double cf = *b.dt * A / g.vol;
-
-  double q[NV][6], acc[NV][6];
-  auto load = [&](int cell, int slot) {
-    int64_t off = base + (int64_t)cell * st;
-#pragma unroll
-    for (int v = 0; v < 5; ++v) q[v][slot] = b.W[v * sv + off];
-#pragma unroll
-    for (int n = 0; n < NS; ++n) q[5 + n][slot] = b.R[n * sv + off];
-  };
-  auto gd = [&](int cell, double* out) {
-    bool in = cell >= lo && cell <= hi;
-    int64_t off = base + (int64_t)cell * st;
-#pragma unroll
-    for (int v = 0; v < NV; ++v) out[v] = in ? b.GD[v * sv + off] : 0.;
-  };
-  auto flush = [&](int cell, int slot) {
-    int64_t off = base + (int64_t)cell * st;
-#pragma unroll
-    for (int v = 0; v < NV; ++v)
-      if (acc[v][slot] != 0.) atomicAdd(&b.GW[v * sv + off], acc[v][slot]);
-  };
-#pragma unroll
-  for (int t = 0; t < 5; ++t) load(f0 - 3 + t, t);
-#pragma unroll
-  for (int v = 0; v < NV; ++v)
-#pragma unroll
-    for (int t = 0; t < 6; ++t) acc[v][t] = 0.;
-  double gm[NV], gp[NV];
-  gd(f0 - 1, gm);
-  for (int f = f0; f <= f1; ++f) {
-    load(f + 2, 5);
-    gd(f, gp);
-    double gF[NV];
-#pragma unroll
-    for (int v = 0; v < NV; ++v) gF[v] = cf * (gp[v] - gm[v]);
-    face_vjp<NS>(p, p.r23_type, p.r23_shock, p.r23_scale, ivx, disabled != 0, false, false, q, gF,
-                 acc);
-    // cell f-3 is complete
-    flush(f - 3, 0);
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-#pragma unroll
-      for (int t = 0; t < 5; ++t) {
-        q[v][t] = q[v][t + 1];
-        acc[v][t] = acc[v][t + 1];
-      }
-      acc[v][5] = 0.;
-      gm[v] = gp[v];
-    }
-  }
-  // after the shift, slot t holds cell f1 - 2 + t
-#pragma unroll
-  for (int t = 0; t < 5; ++t) flush(f1 - 2 + t, t);
-}
 
 // ---------------------------------------------------------------------------
 // x1: one CTA per group of columns (every column: the U->W reverse covers the
@@ -1661,25 +1433,10 @@ template <int NS>
 static cudaError_t launch_sweeps_adj_ns(const Geo& g, const Phys& p, const AdjBufs& b,
                                         cudaStream_t st) {
   const bool a1 = g.nc1 > 1, a2 = g.nc2 > 1, a3 = g.nc3 > 1;
-  const int ni = g.iu - g.il + 1;
   for (int ax = 3; ax >= 2; --ax) {
     if ((ax == 3 && !a3) || (ax == 2 && !a2)) continue;
     ScopedTimer tm(SNAPB_K_ADJ_X23, st);
-    int nax = ax == 2 ? g.nx2 : g.nx3;
-    int no = ax == 2 ? (g.ku - g.kl + 1) : (g.ju - g.jl + 1);
-    int64_t lines = (int64_t)ni * no;
-    // enough (line, segment) pairs for ~4 waves of 148 SMs x 4 CTAs of 128
-    int64_t want = 148LL * 4 * 128 * 4;
-    int nseg = (int)std::min<int64_t>(std::max<int64_t>(1, want / std::max<int64_t>(lines, 1)),
-                                      (nax + 1 + 7) / 8);
-    int seglen = (nax + 1 + nseg - 1) / nseg;
-    nseg = (nax + 1 + seglen - 1) / seglen;
-    dim3 grid((unsigned)((lines + 127) / 128), (unsigned)nseg);
-    if (ax == 2)
-      k_march_adj<NS, 2><<<grid, 128, 0, st>>>(g, p, b, seglen);
-    else
-      k_march_adj<NS, 3><<<grid, 128, 0, st>>>(g, p, b, seglen);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = launch_march_adj(ax, g, p, b, st);
     if (e != cudaSuccess) return e;
   }
   ScopedTimer tm(SNAPB_K_ADJ_X1, st);
