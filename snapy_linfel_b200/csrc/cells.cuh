@@ -26,9 +26,12 @@ __device__ __forceinline__ void cell_states(int type, bool scale, const T* q, T&
         hi = weno5_face(q[4], q[3], q[2], q[1], q[0], scale);
         break;
       } else {
+        // Written so that the reversed window gives lo and hi exchanged, to the
+        // bit: at a reflecting wall both sides of the face then hold mirrored
+        // states, and its mass flux is zero instead of a rounding error.
         T a = q[0], b = q[1], c = q[2], d = q[3], e = q[4], vs = T(1);
         if (scale) {
-          vs = (fabs(a) + fabs(b) + fabs(c) + fabs(d) + fabs(e)) / T(5);
+          vs = (((fabs(a) + fabs(e)) + (fabs(b) + fabs(d))) + fabs(c)) / T(5);
           if (vs == T(0)) {
             lo = hi = T(0);
             return;
@@ -36,33 +39,43 @@ __device__ __forceinline__ void cell_states(int type, bool scale, const T* q, T&
           const T iv = T(1) / vs;
           a *= iv, b *= iv, c *= iv, d *= iv, e *= iv;
         }
-        const T c16 = T(1. / 6.), c56 = T(5. / 6.), c13 = T(1. / 3.), c116 = T(11. / 6.),
-                c76 = T(7. / 6.), c1312 = T(13. / 12.), eps = T(1e-6), q4 = T(0.25);
-        const T s0 = sqr(c1312 * sqr(a - T(2) * b + c) + q4 * sqr(a - T(4) * b + T(3) * c) + eps);
-        const T s1 = sqr(c1312 * sqr(b - T(2) * c + d) + q4 * sqr(d - b) + eps);
-        const T s2 = sqr(c1312 * sqr(c - T(2) * d + e) + q4 * sqr(T(3) * c - T(4) * d + e) + eps);
+        auto M = [](T x, T y) { return __dmul_rn(x, y); };
+        auto S = [](T x, T y) { return __dadd_rn(x, y); };
+        const T c16 = 1. / 6., c56 = 5. / 6., c13 = 1. / 3., c116 = 11. / 6., c76 = 7. / 6.,
+                c1312 = 13. / 12.;
+        auto measure = [&](T u, T w) {
+          const T t = fma(M(c1312, u), u, fma(M(T(0.25), w), w, T(1e-6)));
+          return M(t, t);
+        };
+        const T s0 = measure(S(fma(T(-2), b, a), c), fma(T(3), c, fma(T(-4), b, a)));
+        const T s1 = measure(fma(T(-2), c, S(b, d)), S(d, -b));
+        const T s2 = measure(S(fma(T(-2), d, e), c), fma(T(3), c, fma(T(-4), d, e)));
         // weights over the common denominator s0 s1 s2: one division a side
-        const T s12 = s1 * s2, s01 = s0 * s1, n1 = T(0.6) * (s0 * s2);
-        const T m01 = c56 * b + c13 * c, m10 = c13 * b + c56 * c;  // shared candidate parts
-        const T m23 = c56 * c + c13 * d, m32 = c13 * c + c56 * d;
-        {
-          const T n0 = T(0.3) * s12, n2 = T(0.1) * s01;
-          lo = vs * ((n0 * (m01 - c16 * a) + n1 * (m10 - c16 * d) +
-                      n2 * (c116 * c - c76 * d + c13 * e)) / (n0 + n1 + n2));
-        }
-        {
-          const T n0 = T(0.3) * s01, n2 = T(0.1) * s12;
-          hi = vs * ((n0 * (m32 - c16 * e) + n1 * (m23 - c16 * b) +
-                      n2 * (c116 * c - c76 * b + c13 * a)) / (n0 + n1 + n2));
-        }
+        const T s12 = M(s1, s2), s01 = M(s0, s1), n1 = M(T(0.6), M(s0, s2));
+        const T k13 = M(c13, c), k56 = M(c56, c), k116 = M(c116, c);
+        auto side = [&](T n0, T n2, T x0, T x1, T x3, T x4) {
+          const T p0 = fma(-c16, x0, fma(c56, x1, k13)), p1 = fma(-c16, x3, fma(c13, x1, k56));
+          const T p2 = fma(c13, x4, fma(-c76, x3, k116));
+          return M(vs, fma(n2, p2, fma(n1, p1, M(n0, p0))) / S(S(n0, n1), n2));
+        };
+        lo = side(M(T(0.3), s12), M(T(0.1), s01), a, b, d, e);
+        hi = side(M(T(0.3), s01), M(T(0.1), s12), e, d, b, a);
         break;
       }
     }
     case SNAPB_RECON_CP5: {
       const T a = T(-1. / 20.), b = T(9. / 20.), c = T(47. / 60.), d = T(-13. / 60.),
               e = T(1. / 30.);
-      lo = a * q[0] + b * q[1] + c * q[2] + d * q[3] + e * q[4];
-      hi = a * q[4] + b * q[3] + c * q[2] + d * q[1] + e * q[0];
+      if constexpr (sizeof(T) == 8) {  // (mirrored to the bit, as above)
+        auto side = [&](T x0, T x1, T x3, T x4) {
+          return fma(e, x4, fma(d, x3, fma(c, q[2], fma(b, x1, __dmul_rn(a, x0)))));
+        };
+        lo = side(q[0], q[1], q[3], q[4]);
+        hi = side(q[4], q[3], q[1], q[0]);
+      } else {
+        lo = a * q[0] + b * q[1] + c * q[2] + d * q[3] + e * q[4];
+        hi = a * q[4] + b * q[3] + c * q[2] + d * q[1] + e * q[0];
+      }
       break;
     }
     case SNAPB_RECON_WENO3:

@@ -143,3 +143,25 @@ def test_time_step_reduction(nx):
     for m, tol in ((m64, 5e-16), (m32, 5e-7)):
         m.hydro_w.copy_(torch.from_numpy(w))
         assert abs(float(m.max_time_step()) / dt - 1.0) < tol
+
+
+@pytest.mark.parametrize("riemann", ["lmars", "hllc", "roe"])
+@pytest.mark.parametrize("kw", [{}, dict(shock1=True, shock23=True),
+                                dict(scale1=True, scale23=True)])
+def test_no_mass_through_walls(riemann, kw):
+    """a face on a reflecting wall has exactly mirrored states on its sides, so
+    no mass crosses it: the mass of a closed block changes by the rounding of
+    its own updates only (cells x 2^-53 x 3 stages of the mean cell mass)"""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from snapy_linfel_b200.mesh import MeshBlock
+
+    cfg = make_config(nx1=12, nx2=9, nx3=7, x1=(0.0, 1.2), x2=(0.0, 0.9), x3=(0.0, 0.7),
+                      riemann=riemann, bc=("reflecting",) * 6, **kw)
+    mb = MeshBlock(MeshBlockOptions(cfg, Integration(cfl=0.3)))
+    mb.initialize(random_prim(np.random.default_rng(8), cfg.shape))
+    it = (0,) + cfg.interior()
+    m0 = mb.hydro_u[it].sum().item()
+    mb.step(0.01)
+    m1 = mb.hydro_u[it].sum().item()
+    assert abs(m1 - m0) < m0 * 3 * 2.0 ** -53 * np.sqrt(12 * 9 * 7)
