@@ -12,7 +12,8 @@
 // and the kernels run its pieces backwards:
 //   k_adj_combine   BC^T (a gather over each interior cell's ghost images)
 //                   and the RK weights;
-//   VIC adjoint     k_vadj_assemble / k_vadj_sweep / k_vadj_contract: the
+//   VIC adjoint     k_vadj_chunk (vadj_chunk.cu), or k_vadj_assemble /
+//                   k_vadj_sweep, then k_vadj_contract: the
 //                   forward elimination is repeated, the transposed
 //                   block-tridiagonal system T^T t = g_delta is solved with the
 //                   same factors, and the dependence of the blocks on w is
@@ -20,8 +21,8 @@
 //                   x = delta_k - delta_{k-1}, interface k contributes
 //                   A hiv * d(y^T |A|(w_{k-1}, w_k) x) and cell m contributes
 //                   A hiv * d((t_{m+1} - t_{m-1})^T J(w_m) delta_m);
-//   k_march_adj     x2 / x3 faces: Riemann + reconstruction VJPs, a six-cell
-//                   register window of cotangent accumulators per thread;
+//   k_march_adj     x2 / x3 faces (adj_march.cu): Riemann + reconstruction
+//                   VJPs, cell by cell;
 //   k_x1_adj        x1 faces of a column in shared memory, gravity, the
 //                   ghost-revision VJP and the U->W VJP into g_u, g_s.
 //
