@@ -166,12 +166,17 @@ int plan(snapb_ensemble* e) {
     warps += ((int64_t)(mb.g.ju - mb.g.jl + 1) * (mb.g.ku - mb.g.kl + 1) + cw - 1) / cw;
   }
   const int chunk_groups = (int)std::min<int64_t>(8, std::max<int64_t>(1, warps / (e->sms * 64)));
+  // An x1 item is sized for the member's part of the chip: cut as if each member
+  // had all of it, 16 members of 40 to 100 cells a side took 186 us a stage
+  // instead of 134, the 48 members 1.57 ms instead of 1.47.
+  double cells = 0.;  // of all members
+  for (const Member32& mb : e->mem) cells += (double)mb.g.sv;
   for (int m = 0; m < e->M; ++m) {
     Member32& mb = e->mem[m];
     const Geo& g = mb.g;
     const int nvt = 5 + e->p.nscalar;
     // x1: one warp per item
-    mb.x1 = x1_split32(g, nvt, !e->a2 && !e->a3, t.x1_columns);
+    mb.x1 = x1_split32(g, nvt, !e->a2 && !e->a3, t.x1_columns, (double)g.sv / cells);
     e->x1_smem = std::max(e->x1_smem, (size_t)mb.x1.pitch * nvt * sizeof(float));
     // march: 128 lines per tile, segments of seglen faces
     int ni = g.iu - g.il + 1;

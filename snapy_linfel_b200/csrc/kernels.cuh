@@ -204,8 +204,9 @@ cudaError_t launch_bc32_batch(const Member32* mem, const Phys& p, const WorkQueu
                               double igm1, const PersistGrid& pg, cudaStream_t st);
 size_t x1_smem32_per_column(const Geo& g, int nvt);
 // split of the FP32 x1 sweep of a block and its items (last: the sweep finishes
-// the cells; columns: per item, 0 for the rule)
-X1Split x1_split32(const Geo& g, int nvt, bool last, int columns);
+// the cells; columns: per item, 0 for the rule; share: the block's part of the
+// work that the launch gives the chip)
+X1Split x1_split32(const Geo& g, int nvt, bool last, int columns, double share);
 int64_t x1_items32(const Geo& g, const X1Split& sp);
 StageBufs32 bufs32_of(const snapb_hydro_config& c, void* ws);
 size_t workspace_size_f32_of(const snapb_hydro_config& c);

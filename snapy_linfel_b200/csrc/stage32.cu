@@ -194,7 +194,7 @@ constexpr double kX1Resident32 = 148. * 24.;
 // the conversion's loads.  Per stage, against a tile of columns per CTA (bulk
 // copies into shared memory, barriers, the revision in its own kernel):
 // 384 x 384 x 192, Roe, two tracers 1.29 -> 1.25 ms, 512 x 256 21.0 -> 10.7 us,
-// 48 members of 64 and 128 layers 1.57 ms with either.
+// 48 members of 64 and 128 layers 1.57 -> 1.47 ms.
 template <int NS, int FP>
 __device__ __noinline__ void x1_32_item(const Shared32* sh, int64_t item, float* row, int last) {
   constexpr int NV = 5 + NS;
@@ -810,8 +810,8 @@ cudaError_t launch_ref32(const Geo& g, const Phys& p, const double* rb, const do
 // item (as far as the shared memory goes).  A 1-D block's cells are finished by
 // the sweep itself, so its column is not cut into segments whose halos another
 // warp would be updating.
-X1Split x1_split32(const Geo& g, int nvt, bool last, int columns) {
-  X1Split sp = x1_split(g, nvt, sizeof(float), kX1RowBytes32, kX1Resident32, last);
+X1Split x1_split32(const Geo& g, int nvt, bool last, int columns, double share) {
+  X1Split sp = x1_split(g, nvt, sizeof(float), kX1RowBytes32, kX1Resident32 * share, last);
   if (columns > 0) {
     const int fit = (int)((48 * 1024) / ((size_t)nvt * g.nc1 * sizeof(float)));
     if (fit >= 1 || last) {
@@ -828,7 +828,7 @@ int64_t x1_items32(const Geo& g, const X1Split& sp) {
 cudaError_t launch_x1_32(const Geo& g, const Phys& p, const StageBufs32& b, bool last,
                          cudaStream_t st) {
   const int nvt = 5 + p.nscalar;
-  const X1Split sp = x1_split32(g, nvt, last, 0);
+  const X1Split sp = x1_split32(g, nvt, last, 0, 1.);
   const size_t smem = (size_t)sp.pitch * nvt * sizeof(float);
   if (smem > 200 * 1024) return cudaErrorInvalidConfiguration;
   return with_ns_profile(p.nscalar, face_profile32(p, 1), [&](auto ns, auto fp) {
