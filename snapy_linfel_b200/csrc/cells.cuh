@@ -1,8 +1,9 @@
 // cells.cuh — what the cell-centred sweeps of both forms share: the face values
-// of a cell, the isentropic x1 ghosts, and the split of the x1 sweep.
+// of a cell and the isentropic x1 ghosts.
 #pragma once
 
 #include "common.cuh"
+#include "x1_split.cuh"
 
 namespace snapb {
 
@@ -102,14 +103,6 @@ __device__ __forceinline__ void cell_states(int type, bool scale, const T* q, T&
   }
 }
 
-// Split of the x1 sweep over warps: an item is either K whole columns
-// (consecutive, so their cells are one contiguous span per variable) or one of
-// nseg segments of seglen cells of a single column.
-struct X1Split {
-  int K, nseg, seglen;
-  int pitch;  // doubles per variable row in the warp's shared memory
-};
-
 // Isentropic density and pressure of ghost level n (1 = next to the interior)
 // from the edge cell's: with a = (gamma - 1) / gamma the recurrence
 // p_{n+1}^a = p_n^a +- a g dz / K^(1/gamma) is linear in p^a, so every level
@@ -123,9 +116,5 @@ __device__ __forceinline__ void isentropic_ghost(double gamma, double gdz, int t
   pn = pow(h, 1. / a);
   rn = pn / h * (re / q);
 }
-
-// The split for a block: rows of at most row_bytes a warp where some split has
-// them, `resident` warps on the GPU at once (whole: no segments).
-X1Split x1_split(const Geo& g, int nvt, size_t item, size_t row_bytes, double resident, bool whole);
 
 }  // namespace snapb

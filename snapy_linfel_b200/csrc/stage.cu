@@ -10,8 +10,6 @@
 // solvers (src/riemann/*_impl.h), divergence (src/coord/coordinate.cpp:352-396),
 // gravity (src/forcing/const_gravity.cpp:26-45), hydrostatic revisions
 // (src/hydro/hydro.cpp:217-269), ScalarImpl::forward (src/scalar/scalar.cpp:50-132).
-#include <algorithm>
-
 #include "sweep64.cuh"
 
 namespace snapb {
@@ -224,43 +222,9 @@ cudaError_t launch_finalize(const Geo& g, const Phys& p, const StageBufs& b,
   return cudaGetLastError();
 }
 
-// How the x1 sweep is split over warps.  A warp's time is about one unit per
-// round of 32 cells, a third of one per 32 cells converted, and a start-up;
-// the FP64 form's 16 warps per SM are resident when a warp's rows stay within
-// 14 KB.  Packing
-// K short columns end to end fills the last round of each column (64 layers
-// alone: 66 cells in 3 rounds, 69 %; five columns: 330 in 11, 94 %);
-// segments of a column spread a few long columns over the SMs (1024 cells of
-// a 1-D block: one CTA took 43 us).
-X1Split x1_split(const Geo& g, int nvt, size_t item, size_t row_bytes, double resident,
-                 bool whole) {
-  const int64_t ncol = (int64_t)g.nc2 * g.nc3;
-  X1Split best{1, 1, g.nx1, g.nc1};
-  double best_cost = 0.;
-  size_t best_bytes = 0;
-  auto consider = [&](X1Split s, int n, int nn) {
-    const int64_t items = (ncol + s.K - 1) / s.K * s.nseg;
-    const size_t bytes = (size_t)s.pitch * nvt * item;
-    const double waves = std::max(1., items / resident + 0.5);
-    const double cost = waves * (1. + (s.K * nn + 31) / 32 + ((s.K * n + 31) / 32) / 3.);
-    const bool fits = bytes <= row_bytes, best_fits = best_bytes <= row_bytes;
-    if (best_bytes == 0 || (fits && !best_fits) ||
-        (fits == best_fits && (fits ? cost < best_cost : bytes < best_bytes))) {
-      best = s;
-      best_cost = cost;
-      best_bytes = bytes;
-    }
-  };
-  for (int K = 1; K <= 8; ++K) consider({K, 1, g.nx1, K * g.nc1}, g.nc1, g.nx1 + 2);
-  for (int want = 2; !whole && want <= (g.nx1 + 29) / 30; ++want) {
-    const int S = (g.nx1 + want - 1) / want, nseg = (g.nx1 + S - 1) / S;
-    if (nseg > 1) consider({1, nseg, S, S + g.ng + 3}, S + 6, S + 2);
-  }
-  return best;
-}
-
 cudaError_t launch_x1(const Geo& g, const Phys& p, const StageBufs& b, cudaStream_t st) {
-  const X1Split sp = x1_split(g, 5 + p.nscalar, sizeof(double), 14 * 1024, 148. * 16., false);
+  const X1Split sp = x1_split(g.nx1, g.ng, (int64_t)g.nc2 * g.nc3, 5 + p.nscalar, sizeof(double),
+                              14 * 1024, 148. * 16., false);
   const int64_t items = ((int64_t)g.nc2 * g.nc3 + sp.K - 1) / sp.K * sp.nseg;
   const size_t per = (size_t)sp.pitch * (5 + p.nscalar) * sizeof(double);
   // warps per CTA: four, fewer when the items would not reach every SM

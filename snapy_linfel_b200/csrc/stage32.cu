@@ -811,7 +811,8 @@ cudaError_t launch_ref32(const Geo& g, const Phys& p, const double* rb, const do
 // the sweep itself, so its column is not cut into segments whose halos another
 // warp would be updating.
 X1Split x1_split32(const Geo& g, int nvt, bool last, int columns, double share) {
-  X1Split sp = x1_split(g, nvt, sizeof(float), kX1RowBytes32, kX1Resident32 * share, last);
+  X1Split sp = x1_split(g.nx1, g.ng, (int64_t)g.nc2 * g.nc3, nvt, sizeof(float), kX1RowBytes32,
+                        kX1Resident32 * share, last);
   if (columns > 0) {
     const int fit = (int)((48 * 1024) / ((size_t)nvt * g.nc1 * sizeof(float)));
     if (fit >= 1 || last) {

@@ -165,3 +165,61 @@ def test_no_mass_through_walls(riemann, kw):
     mb.step(0.01)
     m1 = mb.hydro_u[it].sum().item()
     assert abs(m1 - m0) < m0 * 3 * 2.0 ** -53 * np.sqrt(12 * 9 * 7)
+
+
+# lengths that segments of 30 cells leave one or two cells over of
+SHORT_REST = [842, 871, 872, 901, 1022]
+
+
+@pytest.mark.parametrize("nx", [(n, 1, 1) for n in SHORT_REST] +
+                         [(842, 4, 1), (871, 4, 1), (871, 20, 1), (901, 4, 4), (872, 1, 4)])
+@pytest.mark.parametrize("nghost", [3, 4])
+def test_short_last_segment_under_gravity(oracle, nx, nghost):
+    """the segment below a wall's reads no ghost cell: only the wall's own
+    segment revises them"""
+    _check(oracle, nx, nghost=nghost, nscalar=1, scalar_recon="weno5",
+           bc=("reflecting",) * 4 + ("periodic",) * 2)
+
+
+@pytest.mark.parametrize("nx", [(842, 4, 1), (871, 20, 1), (901, 3, 3)])
+def test_fp32_short_last_segment_under_gravity(nx):
+    """as above in the FP32 form (only its 2-D and 3-D columns are cut), against
+    the FP64 form, and in an ensemble with a larger member, where a member is cut
+    for its share of the chip: bit for bit the one-block run"""
+    test_fp32_sweeps_match_fp64(nx, "lmars", 0)
+    from snapy_linfel_b200.ensemble import Ensemble
+    from snapy_linfel_b200.mesh import MeshBlockF32
+
+    members = []
+    for n in (nx, (60, 40, 30) if nx[2] > 1 else (200, 300, 1)):
+        cfg = make_config(nx1=n[0], nx2=n[1], nx3=n[2], x1=(0.0, 0.1 * n[0]),
+                          x2=(0.0, 0.1 * n[1]), x3=(0.0, 0.1 * n[2]), grav=(-0.2, 0.0, 0.0),
+                          bc=("reflecting",) * 4 + ("periodic",) * 2)
+        members.append((MeshBlockOptions(cfg, Integration(cfl=0.3)),
+                        random_prim(np.random.default_rng(n[0]), cfg.shape), None))
+    ens = Ensemble(members)
+    ens.step()
+    for (opts, w, r), b in zip(members, ens.blocks):
+        mb = MeshBlockF32(opts)
+        mb.initialize(w, r)
+        mb.step()
+        assert torch.equal(mb.hydro_u, b.hydro_u)
+
+
+def test_no_mass_through_segments():
+    """the two warps that form the face between their segments form the same
+    flux: the mass of a closed block with gravity changes by the rounding of its
+    own updates only (the bound of test_no_mass_through_walls)"""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from snapy_linfel_b200.mesh import MeshBlock
+
+    cfg = make_config(nx1=871, nx2=4, x1=(0.0, 87.1), x2=(0.0, 0.4), grav=(-0.2, 0.0, 0.0),
+                      bc=("reflecting",) * 6)
+    mb = MeshBlock(MeshBlockOptions(cfg, Integration(cfl=0.3)))
+    mb.initialize(random_prim(np.random.default_rng(8), cfg.shape))
+    it = (0,) + cfg.interior()
+    m0 = mb.hydro_u[it].sum().item()
+    mb.step(0.01)
+    m1 = mb.hydro_u[it].sum().item()
+    assert abs(m1 - m0) < m0 * 3 * 2.0 ** -53 * np.sqrt(871 * 4)
