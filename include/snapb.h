@@ -295,9 +295,10 @@ typedef struct snapb_member_f32 {
   size_t workspace_bytes;
 } snapb_member_f32;
 
-/* tile shapes and kernel variants; 0 = default.  x1_columns: columns per x1
- * tile (a power of two); march_segment: faces per x2/x3 segment; ctas_per_sm:
- * persistent CTAs per SM cap (of 128 threads); vic_kernel: the implicit solve
+/* tile shapes and kernel variants; 0 = default.  x1_columns: whole x1
+ * columns per work item of the x1 sweep (any number; at most 32 of them, and as
+ * many as 48 KB of rows hold, are taken); march_segment: faces per x2/x3
+ * segment; ctas_per_sm: persistent CTAs per SM cap (of 128 threads); vic_kernel: the implicit solve
  * (0 one warp per group of columns for 3x3 blocks and columns of at most 1216
  * layers, else the column kernel + finish kernel; 1 block cyclic reduction,
  * one CTA per column, where it applies: 3x3 blocks and columns of at most 256

@@ -807,19 +807,14 @@ cudaError_t launch_ref32(const Geo& g, const Phys& p, const double* rb, const do
 }
 
 // the split of the x1 sweep of one block; columns > 0 asks for that many per
-// item (as far as the shared memory goes).  A 1-D block's cells are finished by
+// item (as far as a warp and its shared memory go).  A 1-D block's cells are finished by
 // the sweep itself, so its column is not cut into segments whose halos another
 // warp would be updating.
 X1Split x1_split32(const Geo& g, int nvt, bool last, int columns, double share) {
   X1Split sp = x1_split(g.nx1, g.ng, (int64_t)g.nc2 * g.nc3, nvt, sizeof(float), kX1RowBytes32,
                         kX1Resident32 * share, last);
-  if (columns > 0) {
-    const int fit = (int)((48 * 1024) / ((size_t)nvt * g.nc1 * sizeof(float)));
-    if (fit >= 1 || last) {
-      const int K = std::max(1, std::min(columns, fit));
-      sp = X1Split{K, 1, g.nx1, K * g.nc1};
-    }
-  }
+  if (columns > 0)
+    sp = x1_split_columns(sp, g.nx1, g.ng, nvt, sizeof(float), columns, last);
   return sp;
 }
 int64_t x1_items32(const Geo& g, const X1Split& sp) {

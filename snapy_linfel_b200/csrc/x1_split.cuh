@@ -60,4 +60,19 @@ inline X1Split x1_split(int nx1, int ng, int64_t ncol, int nvt, size_t item, siz
   return best;
 }
 
+// Most whole columns of an item: a warp marks the interior ones of them in one
+// word, a bit each.
+constexpr int kX1MaxColumns = 32;
+
+// `columns` whole columns per item instead of the rule's split, as many of them
+// as an item takes and 48 KB of rows hold; the rule's where not one fits (whole:
+// one all the same).
+inline X1Split x1_split_columns(const X1Split& rule, int nx1, int ng, int nvt, size_t item,
+                                int columns, bool whole) {
+  const int nc1 = nx1 + 2 * ng, fit = (int)((48 * 1024) / ((size_t)nvt * nc1 * item));
+  if (fit < 1 && !whole) return rule;
+  const int K = std::max(1, std::min({columns, fit, kX1MaxColumns}));
+  return X1Split{K, 1, nx1, K * nc1};
+}
+
 }  // namespace snapb

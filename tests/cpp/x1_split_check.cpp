@@ -1,6 +1,7 @@
 // Host check of csrc/x1_split.cuh over every column length up to the longest
 // that a block may have, the column counts of lines, planes and boxes, both
-// forms' limits and the shares of the chip that an ensemble's members get.
+// forms' limits, the shares of the chip that an ensemble's members get and the
+// columns per item that a caller may ask for.
 // Prints "splits <n> faults <n>" and the first faults.
 #include <cstdio>
 
@@ -50,7 +51,13 @@ int main() {
           for (double share : {1., 0.3, 0.02})
             check(x1_split(nx1, ng, ncol, nvt, 4, 7 * 1024, 148. * 24. * share, false), nx1, ng,
                   ncol);
-          check(x1_split(nx1, ng, ncol, nvt, 4, 7 * 1024, 148. * 24., true), nx1, ng, ncol);
+          for (bool whole : {false, true}) {
+            const X1Split rule = x1_split(nx1, ng, ncol, nvt, 4, 7 * 1024, 148. * 24., whole);
+            check(rule, nx1, ng, ncol);
+            if (ncol != 1030) continue;
+            for (int columns : {1, 2, 7, 16, 31, 32, 33, 64, 1000})
+              check(x1_split_columns(rule, nx1, ng, nvt, 4, columns, whole), nx1, ng, ncol);
+          }
         }
   printf("splits %ld faults %ld\n", splits, faults);
   return 0;

@@ -165,3 +165,14 @@ def test_cyclic_reduction_agrees_with_block_thomas(dev):
             scale = float(b[v].abs().max())
             err = float((a[v] - b[v]).abs().max())
             assert err <= 1e-5 * max(scale, 1e-30), f"member {k} var {v}: {err} vs {scale}"
+
+
+@pytest.mark.parametrize("columns", [16, 32, 33, 64, 1000])
+def test_any_number_of_x1_columns_is_exact(dev, columns):
+    """more columns per item than a warp has lanes are accepted and change no
+    result (members of 8 and 16 layers, 196 and more columns)"""
+    members = small_members(n=4, seed=23)
+    ref = singles(members, 2, dev)
+    _, got = batched(members, 2, dev, tuning={"x1_columns": columns})
+    for k, (a, b) in enumerate(zip(got, ref)):
+        assert torch.equal(a, b), f"member {k}: {float((a - b).abs().max())}"
