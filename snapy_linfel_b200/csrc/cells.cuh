@@ -106,15 +106,21 @@ __device__ __forceinline__ void cell_states(int type, bool scale, const T* q, T&
 // Isentropic density and pressure of ghost level n (1 = next to the interior)
 // from the edge cell's: with a = (gamma - 1) / gamma the recurrence
 // p_{n+1}^a = p_n^a +- a g dz / K^(1/gamma) is linear in p^a, so every level
-// follows from the edge directly.  With q = p_e^(1/gamma) the other powers
-// are quotients (p_e^a = p_e / q, K^(1/gamma) = q / rho_e,
-// p^(1/gamma) = p / p^a), which leaves two pow calls per level.
+// follows from the edge directly, and with y = p_n^a / p_e^a = 1 +- n a g dz
+// rho_e / p_e (K^(1/gamma) = p_e^(1/gamma) / rho_e and p_e^a p_e^(1/gamma) = p_e)
+// p_n = p_e y^(1/a), rho_n = rho_e y^(1/a) / y.  y is near one, so the rounding
+// of the exponent does not grow with log p as it does in powers of p itself:
+// against 45 digits the pressure is off by 1.7e-16 on average (8e-16 at most), by
+// 1.05e-15 (4.1e-15) from powers of p_e.
 __device__ __forceinline__ void isentropic_ghost(double gamma, double gdz, int top, int n,
                                                  double pe, double re, double& pn, double& rn) {
-  const double a = (gamma - 1.) / gamma, q = pow(pe, 1. / gamma);
-  const double h = (pe + (top ? -n : n) * a * gdz * re) / q;
-  pn = pow(h, 1. / a);
-  rn = pn / h * (re / q);
+  const double a = (gamma - 1.) / gamma;
+  // (a negative pressure or density has no adiabat)
+  const double y = pe < 0. || re < 0. ? __longlong_as_double(0x7ff8000000000000ll)
+                                      : 1. + (top ? -n : n) * a * gdz * re / pe;
+  const double z = pow(y, 1. / a);
+  pn = pe * z;
+  rn = re * z / y;
 }
 
 }  // namespace snapb

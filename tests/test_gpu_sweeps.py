@@ -223,3 +223,83 @@ def test_no_mass_through_segments():
     mb.step(0.01)
     m1 = mb.hydro_u[it].sum().item()
     assert abs(m1 - m0) < m0 * 3 * 2.0 ** -53 * np.sqrt(871 * 4)
+
+
+@pytest.mark.parametrize("gammad", [1.4, 5.0 / 3.0])
+@pytest.mark.parametrize("units", ["air", "giant"])
+def test_isentropic_ghosts_to_rounding(gammad, units):
+    """the density and pressure that an x1 ghost takes from the edge cell, against
+    45 digits.  With y = 1 +- n a g dz rho / p, p y^(1/a) and rho y^(1/a) / y: y
+    holds 1.6 units of 2^-53 (its sum, and six roundings of a term below 0.1),
+    1 / a <= 3.5 times that enters the power, which adds 4 (2 ulp), and the last
+    products one each: 11.6 units for the pressure, 15 for the density."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import ctypes
+    from decimal import Decimal as D, getcontext
+
+    from snapy_linfel_b200 import _lib
+
+    dz, grav = (100.0, -9.8) if units == "air" else (2000.0, -24.8)
+    cfg = make_config(nx1=12, nx2=70, x1=(0.0, 12 * dz), x2=(0.0, 7e3), gammad=gammad,
+                      grav=(grav, 0.0, 0.0), bc=("reflecting",) * 4 + ("periodic",) * 2)
+    rng = np.random.default_rng(4)
+    w = random_prim(rng, cfg.shape)
+    if units == "air":
+        w[4] = rng.uniform(1e4, 1.2e5, w[4].shape)
+        w[0] = w[4] / (287.0 * rng.uniform(200.0, 310.0, w[4].shape))
+    else:
+        w[4] = 10.0 ** rng.uniform(4.0, 6.0, w[4].shape)
+        w[0] = w[4] / (3700.0 * rng.uniform(150.0, 400.0, w[4].shape))
+    wg = torch.from_numpy(w).cuda()
+    ug, du = torch.empty_like(wg), torch.empty_like(wg)
+    L = _lib.lib()
+    ws = torch.empty(L.snapb_workspace_size(ctypes.byref(cfg)), dtype=torch.uint8, device="cuda")
+    dt = torch.tensor([1e-3], dtype=torch.float64, device="cuda")
+    P = _lib.ptr
+    _lib.check(L.snapb_prim2cons(ctypes.byref(cfg), P(wg), P(ug), _lib.stream_ptr()))
+    _lib.check(L.snapb_hydro_forward(ctypes.byref(cfg), P(dt), P(ug), P(wg), P(du), None, P(ws),
+                                     ctypes.c_size_t(ws.numel()), _lib.stream_ptr()))
+    got = wg.cpu().numpy()[:, 0]
+    getcontext().prec = 45
+    g, h = D(cfg.gammad), D(cfg.grav1) * (D(cfg.x1max) - D(cfg.x1min)) / cfg.nx1
+    a, ng = (g - 1) / g, cfg.nghost
+    worst = [0.0, 0.0]
+    for j in range(got.shape[1]):
+        for edge, up in ((ng, -1), (ng + cfg.nx1 - 1, 1)):
+            re, pe = D(float(got[0, j, edge])), D(float(got[4, j, edge]))
+            for n in range(1, ng + 1):
+                y = 1 + up * n * a * h * re / pe
+                z = (y.ln() / a).exp()
+                for q, (v, ref) in enumerate(((4, pe * z), (0, re * z / y))):
+                    x = D(float(got[v, j, edge + up * n]))
+                    worst[q] = max(worst[q], float(abs((x - ref) / ref)))
+    assert worst[0] < 11.6 * 2.0 ** -53 and worst[1] < 15 * 2.0 ** -53, worst
+
+
+@pytest.mark.parametrize("var", [0, 4])
+def test_ghosts_of_an_unphysical_edge_are_nan(var):
+    """a negative density or pressure in the edge cell has no isentropic ghosts"""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import ctypes
+
+    from snapy_linfel_b200 import _lib
+
+    cfg = make_config(nx1=12, nx2=5, x1=(0.0, 1.2), x2=(0.0, 0.5), grav=(-0.2, 0.0, 0.0),
+                      bc=("reflecting",) * 4 + ("periodic",) * 2)
+    w = random_prim(np.random.default_rng(4), cfg.shape)
+    ng = cfg.nghost
+    w[var, 0, ng + 2, ng] *= -1.0
+    wg = torch.from_numpy(w).cuda()
+    ug, du = torch.empty_like(wg), torch.empty_like(wg)
+    L = _lib.lib()
+    ws = torch.empty(L.snapb_workspace_size(ctypes.byref(cfg)), dtype=torch.uint8, device="cuda")
+    dt = torch.tensor([1e-3], dtype=torch.float64, device="cuda")
+    P = _lib.ptr
+    _lib.check(L.snapb_prim2cons(ctypes.byref(cfg), P(wg), P(ug), _lib.stream_ptr()))
+    _lib.check(L.snapb_hydro_forward(ctypes.byref(cfg), P(dt), P(ug), P(wg), P(du), None, P(ws),
+                                     ctypes.c_size_t(ws.numel()), _lib.stream_ptr()))
+    got = wg.cpu().numpy()[:, 0]
+    assert np.isnan(got[[0, 4], ng + 2, :ng]).all()
+    assert np.isfinite(got[[0, 4], ng + 1, :ng]).all()
