@@ -85,7 +85,10 @@ __device__ __forceinline__ void jac_col(const PairCell& c, int q, double gm1, do
 // large under the row weights `lg` (binary logarithms, added to the exponent;
 // the implicit scaling of the reference's LU, whose rows differ by powers of
 // the sound speed).  Rows are not swapped; a step that pivots elsewhere marks
-// its row as taken, and the solution is put in order at the end.
+// its row as taken, and the solution is put in order at the end.  Each group
+// chooses its own pivots; the warp's vote only decides whether the step is
+// written for the diagonal alone, so that a column's bits depend on no other
+// column's.
 __device__ __forceinline__ void group_solve(double (&X1)[5], double (&X2)[5], const int (&lg)[5]) {
   unsigned left = 31u;
   int perm[5];
@@ -101,7 +104,8 @@ __device__ __forceinline__ void group_solve(double (&X1)[5], double (&X2)[5], co
       if (left >> r & 1) best = max(best, mag[r]);
     }
     perm[j] = j;
-    if (__all_sync(0xffffffffu, (left >> j & 1) && mag[j] >= best - (3 << 20))) {
+    const bool diagonal = (left >> j & 1) && mag[j] >= best - (3 << 20);
+    if (__all_sync(0xffffffffu, diagonal)) {
       const double rp = 1. / col[j], x1p = X1[j] * rp, x2p = X2[j] * rp;
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
@@ -114,7 +118,7 @@ __device__ __forceinline__ void group_solve(double (&X1)[5], double (&X2)[5], co
       bool found = false;
 #pragma unroll
       for (int r = 0; r < 5; ++r) {
-        const bool take = !found && (left >> r & 1) && mag[r] >= best;
+        const bool take = diagonal ? r == j : !found && (left >> r & 1) && mag[r] >= best;
         found = found || take;
         perm[j] = take ? r : perm[j];
         piv = take ? col[r] : piv;

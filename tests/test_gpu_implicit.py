@@ -161,3 +161,33 @@ def test_adjoint_solver_matches_sweep(L, monkeypatch, nl, nx2, nx3, ns):
         assert torch.isfinite(a).all()
         for v in range(a.shape[0]):
             assert float((a[v] - b[v]).abs().max()) <= 1e-11 * float(b[v].abs().max()), v
+
+
+@pytest.mark.parametrize("dt", [0.05, 5.0, 500.0])
+@pytest.mark.parametrize("nl", [3, 6, 33, 64])
+def test_five_by_five_column_is_its_own(L, nl, dt):
+    """a column's result depends on no other column: the same bits when the
+    column beside it in the warp holds another state, and when that state is
+    not a number"""
+    c = _config(nl, 4, 1, 9)
+    rng = np.random.default_rng(nl)
+    w = random_prim(rng, c.shape)
+    du = 0.05 * (rng.random(c.shape) - 0.5)
+    ws = torch.empty(L.lib().snapb_workspace_size(ctypes.byref(c)), dtype=torch.uint8,
+                     device="cuda")
+    dtg = torch.tensor([dt], dtype=torch.float64, device="cuda")
+    ng, out = c.nghost, []
+    for beside in ("same", "supersonic", "nan"):
+        x = w.copy()
+        if beside == "supersonic":
+            x[1:4, :, ng + 1::2] *= 1e3
+        elif beside == "nan":
+            x[:, :, ng + 1::2] = np.nan
+        dug, wg = dev(du), dev(x)
+        call(L, "snapb_implicit_correction", ctypes.byref(c), L.ptr(dtg), L.ptr(dug), L.ptr(wg),
+             None, L.ptr(ws), ctypes.c_size_t(ws.numel()), L.stream_ptr())
+        got = dug.cpu().numpy()[:, 0, ng:ng + 4:2, ng:-ng]
+        assert_finite(got)
+        out.append(got)
+    for got in out[1:]:
+        assert np.array_equal(got, out[0])
