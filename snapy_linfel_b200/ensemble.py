@@ -158,6 +158,13 @@ class Ensemble:
                     dst.copy_(src)
 
     # ---- autotuner ----
+    def _column_kernel(self):
+        """whether vic_kernel 0 (or 1 where it falls back to 0) solves some
+        member by the column kernel: 5x5 blocks, and columns longer than the
+        one-warp solve takes"""
+        return any(b.cfg.implicit_scheme == 9 or (b.cfg.implicit_scheme and b.cfg.nx1 > 1216)
+                   for b in self.blocks)
+
     def set_tuning(self, **kw):
         t = Tuning()
         for k, v in self.tuning.as_dict().items():
@@ -179,35 +186,42 @@ class Ensemble:
         snap = self.save()
         results = []
         best = None
+
+        def measure(trial):
+            nonlocal best
+            try:
+                self.set_tuning(**trial)
+            except _lib.SnapbError:
+                return
+            self.restore(snap)
+            self.step_eager()  # warm
+            torch.cuda.synchronize()
+            e0 = torch.cuda.Event(enable_timing=True)
+            e1 = torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(steps):
+                self.step_eager()
+            e1.record()
+            torch.cuda.synchronize()
+            ms = e0.elapsed_time(e1) / steps
+            results.append((dict(trial), ms))
+            if log:
+                log(f"tune {trial} -> {ms:.3f} ms/step")
+            if best is None or ms < best[1]:
+                best = (dict(trial), ms)
+
         # coordinate descent: one parameter at a time, starting from the defaults
         current = self.tuning.as_dict()
         for key, values in cand.items():
-            if key in ("vic_block", "vic_regs") and current.get("vic_kernel", 0) != 0:
-                continue  # shapes of the column kernel, not in use
+            if key in ("vic_block", "vic_regs") and (
+                    current.get("vic_kernel", 0) == 2 or not self._column_kernel()):
+                continue  # shapes of the column kernel, which runs for no member
             for v in values:
-                trial = dict(current)
-                trial[key] = v
-                try:
-                    self.set_tuning(**trial)
-                except _lib.SnapbError:
-                    continue
-                self.restore(snap)
-                self.step_eager()  # warm
-                torch.cuda.synchronize()
-                e0 = torch.cuda.Event(enable_timing=True)
-                e1 = torch.cuda.Event(enable_timing=True)
-                e0.record()
-                for _ in range(steps):
-                    self.step_eager()
-                e1.record()
-                torch.cuda.synchronize()
-                ms = e0.elapsed_time(e1) / steps
-                results.append((dict(trial), ms))
-                if log:
-                    log(f"tune {trial} -> {ms:.3f} ms/step")
-                if best is None or ms < best[1]:
-                    best = (dict(trial), ms)
-            current = dict(best[0])
+                measure({**current, key: v})
+            if best is not None:
+                current = dict(best[0])
+        if best is None:  # nothing to choose: the tuning as it is
+            measure(current)
         self.set_tuning(**best[0])
         self.restore(snap)
         return {"best": best[0], "best_ms_per_step": best[1],

@@ -176,3 +176,20 @@ def test_any_number_of_x1_columns_is_exact(dev, columns):
     _, got = batched(members, 2, dev, tuning={"x1_columns": columns})
     for k, (a, b) in enumerate(zip(got, ref)):
         assert torch.equal(a, b), f"member {k}: {float((a - b).abs().max())}"
+
+
+def test_autotuner_times_only_what_the_members_use(dev):
+    """the shapes of the column kernel are trials where some member's solve runs
+    in it (5x5 blocks), and none where the one-warp solve takes every member"""
+    from snapy_linfel_b200.ensemble import Ensemble
+
+    cand = {"vic_block": [32, 64], "vic_regs": [0, 1]}
+    for scheme, trials in ((1, 1), (9, 4)):
+        members = small_members(n=3, seed=7, implicit_scheme=scheme)
+        ref = singles(members, 1, dev)
+        ens = Ensemble(members, device=dev)
+        table = ens.tune(steps=1, candidates=cand)
+        assert len(table["trials"]) == trials and table["best_ms_per_step"] > 0.0
+        ens.step()
+        for a, b in zip([b.hydro_u for b in ens.blocks], ref):
+            assert torch.equal(a, b)
