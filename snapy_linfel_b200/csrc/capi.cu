@@ -70,8 +70,7 @@ Layout ws_layout(const snapb_hydro_config& c) {
   L.D = o;
   o = align256(o + (size_t)(c.nvar + c.nscalar) * sv);
   L.RG = o;
-  bool need_rg = c.grav1 != 0. && p.has_grav && c.non_hydrostatic < 1.;
-  o = align256(o + (need_rg ? sv : 0));
+  o = align256(o + (uses_rho_grav(g, p) ? sv : 0));
   L.DD = o;
   bool diff = c.nu_iso > 0. || c.kappa_iso > 0.;
   o = align256(o + (diff ? (size_t)c.nvar * sv : 0));
@@ -145,7 +144,7 @@ int run_stage(const snapb_hydro_config* c, int stage, const double* dt, double* 
   b.s0 = s0;
   b.r = p.implicit_scheme != 0 ? r : nullptr;
   b.D = at<double>(ws, L.D);
-  b.RG = at<double>(ws, L.RG);
+  b.RG = uses_rho_grav(g, p) ? at<double>(ws, L.RG) : nullptr;
   b.DD = at<double>(ws, L.DD);
   b.R = at<double>(ws, L.R);
   b.M = p.implicit_scheme ? at<double>(ws, L.M) : nullptr;

@@ -70,7 +70,6 @@ struct Phys {
   int nvar, nscalar;
   int implicit_scheme;
   int disable1, disable2, disable3;
-  bool has_grav;  // a const-gravity section exists (any g != 0 or nh != 1)
 };
 
 inline Phys make_phys(const snapb_hydro_config& c) {
@@ -98,8 +97,13 @@ inline Phys make_phys(const snapb_hydro_config& c) {
   p.disable1 = c.disable_flux[0];
   p.disable2 = c.disable_flux[1];
   p.disable3 = c.disable_flux[2];
-  p.has_grav = c.grav1 != 0. || c.grav2 != 0. || c.grav3 != 0. || c.non_hydrostatic != 1.;
   return p;
+}
+
+// Whether the hydrostatic correction rho_grav enters: the x1 sweep forms it under
+// gravity along an active x1.  It is zero otherwise, with no array to read.
+__host__ __device__ __forceinline__ bool uses_rho_grav(const Geo& g, const Phys& p) {
+  return g.nc1 > 1 && p.grav1 != 0. && p.nh < 1.;
 }
 
 // Index arithmetic.  Every element, cell, column, line and slot index of a

@@ -22,7 +22,7 @@ struct StageBufs {
   double* s0;
   double* r;         // scalar_r of the previous stage (mass-correction term)
   double* D;         // [nvar + nscalar][sv] flux-difference sums, then du
-  double* RG;        // [sv] hydrostatic correction rho_grav
+  double* RG;        // [sv] hydrostatic correction rho_grav, or null (uses_rho_grav)
   double* DD;        // [nvar][sv] diffusion flux differences (undivided)
   double* R;         // [nscalar][sv] scalar mixing ratio of the stage input
   double* M;         // [nvar][sv] implicit mass correction (IDN row used)

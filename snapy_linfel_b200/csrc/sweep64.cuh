@@ -55,7 +55,7 @@ __device__ __forceinline__ void finalize_cell(const Geo& g, const Phys& p, const
 #pragma unroll
     for (int v = 0; v < 5; ++v) du[v] -= dtv * b.DD[v * sv + off];
   }
-  if (p.has_grav && p.nh < 1.) {
+  if (uses_rho_grav(g, p)) {
     double rg = b.RG[off];
     du[IVX] += dt * rg * (1. - p.nh);
     du[IPR] += dt * wc[IVX] * rg * (1. - p.nh);
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(128, 4)
   // the lower neighbour's right value (the next lower lane, the previous
   // round's last lane for lane 0) and closes cell c - 1.
   const int nn = c1 - c0 + 2;
-  const bool need_rg = p.grav1 != 0. && p.has_grav && p.nh < 1.;
+  const bool need_rg = uses_rho_grav(g, p);
   double Hc[NV], Fc[NV], rc = 0.;  // lane 0: lane 31 of the previous round
 #pragma unroll
   for (int v = 0; v < NV; ++v) Hc[v] = Fc[v] = 0.;

@@ -303,3 +303,21 @@ def test_ghosts_of_an_unphysical_edge_are_nan(var):
     got = wg.cpu().numpy()[:, 0]
     assert np.isnan(got[[0, 4], ng + 2, :ng]).all()
     assert np.isfinite(got[[0, 4], ng + 1, :ng]).all()
+
+
+@pytest.mark.parametrize("nx,grav", [((40, 1, 1), (0.0, 0.0, 0.0)), ((12, 9, 1), (0.0, 0.1, 0.0)),
+                                     ((9, 6, 5), (0.0, 0.0, -0.1)), ((1, 9, 12), (-0.2, 0.1, 0.0)),
+                                     ((1, 30, 1), (-0.2, 0.0, 0.0)), ((11, 7, 1), (-0.2, 0.1, 0.0))])
+def test_hydrostatic_correction_only_where_it_is_formed(oracle, nx, grav):
+    """non_hydrostatic < 1 without gravity along an active x1: the correction is
+    zero (it was read from workspace that nothing had written, or past its end)"""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    cfg = make_config(nx1=nx[0], nx2=nx[1], nx3=nx[2], x1=(0.0, 0.1 * nx[0]),
+                      x2=(0.0, 0.1 * nx[1]), x3=(0.0, 0.1 * nx[2]), grav=grav,
+                      non_hydrostatic=0.5, bc=("reflecting",) * 6)
+    opts = MeshBlockOptions(cfg, Integration(cfl=0.3))
+    w = random_prim(np.random.default_rng(5), cfg.shape)
+    mb, _ = _run_gpu(opts, w, None, 1, dts=[0.01])
+    u, _, _ = _run_oracle(oracle, opts, w, None, 1, dts=[0.01])
+    assert state_err(mb.hydro_u.cpu().numpy(), u, u) < 1e-12
