@@ -12,89 +12,122 @@
 
 namespace snapb {
 
+// The equations of one lane's chunk in one of the two passes: A delta = du / dt,
+// or (tr) A^T t = g_delta + (g_fix - V g_B) e_0.
+template <int NS>
+struct VadjColumn {
+  const Geo& g;
+  const VadjChunk& in;
+  const int cb, l0, m, sv, nl;
+  const bool tr;
+  double gb, gog, idt;
+  ChunkBlocks<double> blocks;
+  double raw[5], rawd[3], fix = 0., gi = 0., rc;
+  double sum_r2 = 0., sum_du = 0., sum_g = 0.;
+
+  __device__ __forceinline__ void load_w(int l, double (&x)[5]) const {
+    const int o = cb + min(l, nl);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) x[v] = in.W[v * sv + o];
+  }
+  __device__ __forceinline__ void load_d(int l) {
+    const int o = cb + min(l, nl - 1);
+    const double* src = tr ? in.GD : in.D;  // right-hand side rows
+#pragma unroll
+    for (int r = 0; r < 3; ++r) rawd[r] = src[sel<3>(r) * sv + o];
+    gi = in.GD[IDN * sv + o];
+    if (tr) {
+      fix = 0.;
+#pragma unroll
+      for (int n = 0; n < NS; ++n) fix += in.GD[(5 + n) * sv + o] * in.R[n * sv + o];
+    }
+  }
+  __device__ __forceinline__ void make(const double (&x)[5], ChunkCell<double>& c) const {
+    c.set(x[IDN], x[IVX], x[IVY], x[IVZ], x[IPR], gog);
+  }
+  __device__ __forceinline__ VadjColumn(const Geo& g_, const Phys& p, const VadjChunk& in_, int cb_,
+                                        int l0_, int m_, bool tr_, double gb_)
+      : g(g_), in(in_), cb(cb_), l0(l0_), m(m_), sv((int)g_.sv), nl(g_.nx1), tr(tr_), gb(gb_) {
+    idt = 1. / *in.dt, gog = p.gammad / (p.gammad - 1.);
+    blocks.gm1 = p.gammad - 1.;
+    blocks.s = g.A1 * (0.5 / g.vol);
+    blocks.idt = idt;
+    blocks.grav = p.grav1;
+    ChunkCell<double> below, cell;
+    load_w(l0 - 1, raw);
+    make(raw, below);
+    load_w(l0, raw);
+    make(raw, cell);
+    rc = raw[IDN];
+    load_w(l0 + 1, raw);
+    load_d(l0);
+    blocks.start(below, cell);
+  }
+  __device__ __forceinline__ void operator()(int j, double (&a)[3][3], double (&bl)[3][3],
+                                             double (&c)[3][3], double (&rhs)[3]) {
+    const int l = l0 + j;
+    ChunkCell<double> cn;
+    make(raw, cn);
+    const double rn = raw[IDN];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) rhs[r] = l < nl ? (tr ? rawd[r] : rawd[r] * idt) : 0.;
+    if (l < nl) {
+      if (tr) {
+        rhs[0] += fix - g.vol * gb;
+      } else {
+        sum_r2 += rc * rc;
+        sum_du += rawd[0];
+        sum_g += gi * rc * rc;
+      }
+    }
+    if (j < m - 1) {
+      load_w(l + 2, raw);
+      load_d(l + 1);
+    }
+    blocks.template next<true>(cn, l, nl, tr, a, bl, c);
+    rc = rn;
+  }
+};
+
+// (as chunk_again, vic_chunk.cuh)
 template <int G, int NS>
-__global__ void __launch_bounds__(32) k_vadj_chunk(Geo g, Phys p, VadjChunk in, int m) {
+__device__ __noinline__ void vadj_again(const Geo& g, const Phys& p, const VadjChunk& in, int cb,
+                                        int m, double* mine, bool tr, double gb, bool again) {
+  const int k = threadIdx.x & (G - 1);
+  VadjColumn<NS> column(g, p, in, cb, k * m, m, tr, gb);
+  chunk_sequence<G>(m, k, mine, again, column);
+}
+
+template <int G, int NS>
+__global__ void __launch_bounds__(32)
+    k_vadj_chunk(const __grid_constant__ Geo g, const __grid_constant__ Phys p,
+                 const __grid_constant__ VadjChunk in, int m) {
   extern __shared__ double chunk_sm[];
   constexpr int CW = 32 / G;
   const int lane = threadIdx.x & 31, k = lane & (G - 1), cw = lane / G;
-  const int sv = (int)g.sv, nl = g.nx1, l0 = k * m;
+  const int nl = g.nx1, l0 = k * m;
   const int64_t ncol = (int64_t)(g.ju - g.jl + 1) * (g.ku - g.kl + 1);
   const int64_t col0 = (int64_t)blockIdx.x * CW;
   const int cb = (int)column_base(g, min(col0 + cw, ncol - 1));
   double* mine = chunk_sm + lane;
-  const double dt = *in.dt, idt = 1. / dt, gog = p.gammad / (p.gammad - 1.), V = g.vol;
-  ChunkBlocks<double> blocks;
-  blocks.gm1 = p.gammad - 1.;
-  blocks.s = g.A1 * (0.5 / g.vol);
-  blocks.idt = idt;
-  blocks.grav = p.grav1;
-
-  auto load_w = [&](int l, double (&x)[5]) {
-    const int o = cb + min(l, nl);
+  double gb = 0.;
+  // (unrolled: with the passes told apart at run time the second solve's call cost
+  // registers, 512 x 256 with the contraction 84 -> 75 us)
 #pragma unroll
-    for (int v = 0; v < 5; ++v) x[v] = in.W[v * sv + o];
-  };
-  auto make = [&](const double (&x)[5], ChunkCell<double>& c) {
-    c.set(x[IDN], x[IVX], x[IVY], x[IVZ], x[IPR], gog);
-  };
-  double sum_r2 = 0., sum_du = 0., sum_g = 0., sum_x = 0., gb = 0.;
-#pragma unroll 1
   for (int pass = 0; pass < 2; ++pass) {
     const bool tr = pass == 1;
-    const double* src = tr ? in.GD : in.D;  // right-hand side rows
-    double raw[5], rawd[3], fix = 0., gi = 0., rc;
-    auto load_d = [&](int l) {
-      const int o = cb + min(l, nl - 1);
-#pragma unroll
-      for (int r = 0; r < 3; ++r) rawd[r] = src[sel<3>(r) * sv + o];
-      gi = in.GD[IDN * sv + o];
-      if (tr) {
-        fix = 0.;
-#pragma unroll
-        for (int n = 0; n < NS; ++n) fix += in.GD[(5 + n) * sv + o] * in.R[n * sv + o];
-      }
-    };
-    {
-      ChunkCell<double> below, cell;
-      load_w(l0 - 1, raw);
-      make(raw, below);
-      load_w(l0, raw);
-      make(raw, cell);
-      rc = raw[IDN];
-      load_w(l0 + 1, raw);
-      load_d(l0);
-      blocks.start(below, cell);
+    VadjColumn<NS> column(g, p, in, cb, l0, m, tr, gb);
+    double sum_x;
+    const bool again =
+        chunk_solve<G>(m, k, mine, kGrowthLimit<double>, column, [] {}, nl - l0, sum_x);
+    if (__any_sync(0xffffffffu, again)) {
+      vadj_again<G, NS>(g, p, in, cb, m, mine, tr, gb, again);
+      sum_x = chunk_sum(m, mine, nl - l0);
     }
-    auto equation = [&](int j, double (&a)[3][3], double (&bl)[3][3], double (&c)[3][3],
-                        double (&rhs)[3]) {
-      const int l = l0 + j;
-      ChunkCell<double> cn;
-      make(raw, cn);
-      const double rn = raw[IDN];
-#pragma unroll
-      for (int r = 0; r < 3; ++r) rhs[r] = l < nl ? (tr ? rawd[r] : rawd[r] * idt) : 0.;
-      if (l < nl) {
-        if (tr) {
-          rhs[0] += fix - V * gb;
-        } else {
-          sum_r2 += rc * rc;
-          sum_du += rawd[0];
-          sum_g += gi * rc * rc;
-        }
-      }
-      if (j < m - 1) {
-        load_w(l + 2, raw);
-        load_d(l + 1);
-      }
-      blocks.template next<true>(cn, l, nl, tr, a, bl, c);
-      rc = rn;
-    };
-    chunk_solve<G>(m, k, mine, equation, [] {},
-                   [&](int j, const double (&x)[3]) {
-                     if (!tr && l0 + j < nl) sum_x += x[0];
-                   });
     if (!tr) {
-      double lost = sum_du - sum_x;
+      const double V = g.vol;
+      double sum_r2 = column.sum_r2, sum_g = column.sum_g;
+      double lost = column.sum_du - sum_x;
 #pragma unroll
       for (int h = 1; h < G; h *= 2) {
         lost += __shfl_xor_sync(0xffffffffu, lost, h, G);

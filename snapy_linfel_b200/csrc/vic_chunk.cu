@@ -7,7 +7,9 @@ namespace snapb {
 // CTAs of one warp: nothing is shared between warps, and the shared memory of
 // a column length need not divide by more.
 template <int G, int NS, class B>
-__global__ void __launch_bounds__(32) k_vic_chunk(Geo g, Phys p, B b, int m) {
+__global__ void __launch_bounds__(32) k_vic_chunk(const __grid_constant__ Geo g,
+                                                       const __grid_constant__ Phys p,
+                                                       const __grid_constant__ B b, int m) {
   extern __shared__ double chunk_sm[];
   vic_chunk<G, NS, B>(g, p, b, (int64_t)blockIdx.x * (32 / G), m, chunk_sm);
 }
@@ -17,7 +19,8 @@ __global__ void __launch_bounds__(32) k_vic_chunk(Geo g, Phys p, B b, int m) {
 // the current one is worked on.
 template <int G, int NS>
 __global__ void __launch_bounds__(32)
-    k_vic_chunk_batch(const Member32* __restrict__ mem, Phys p, WorkQueue q, int stage) {
+    k_vic_chunk_batch(const Member32* __restrict__ mem, const __grid_constant__ Phys p, WorkQueue q,
+                      int stage) {
   extern __shared__ double chunk_sm[];
   __shared__ Member32 s_mem;
   constexpr int CW = 32 / G;

@@ -10,7 +10,8 @@
 //     x_0 = P - Q y - S y-                       (carried in registers)
 // The G last layers then form a block-tridiagonal system of their own, solved
 // by parallel cyclic reduction across the lanes (shuffles), and each lane
-// substitutes back.  Against the sequential sweep (one thread per column) a
+// substitutes back; columns that this would cost digits are solved again in
+// sequence (chunk_solve).  Against the sequential sweep (one thread per column) a
 // layer costs 3 to 4 times the FP64 operations, but its chain is m layers and
 // log2 G reductions long instead of nl layers, the reduced blocks (96 B a
 // layer, written and read back through HBM by the sweep) stay in shared
@@ -287,16 +288,46 @@ __device__ __forceinline__ void shfl3(const double (&x)[3], int d, double (&y)[3
     y[r] = __shfl_sync(0xffffffffu, x[r], d, G);
 }
 
+// Largest magnitude among the diagonal entries of matrices, as the high word of a
+// double (which orders as the value does).
+struct Growth {
+  int hi = 0;
+  __device__ __forceinline__ void note(const double (&X)[3][3]) {
+#pragma unroll
+    for (int r = 0; r < 3; ++r) hi = max(hi, __double2hiint(X[r][r]) & 0x7fffffff);
+  }
+};
+// The growth from which a column is solved in sequence (chunk_solve), as such a
+// word: 1.5 with blocks in FP64, 32 with blocks in FP32, whose own rounding is the
+// larger error below that.
+template <class BT>
+constexpr int kGrowthLimit = sizeof(BT) == 8 ? 0x3ff80000 : (1023 + 5) << 20;
+
 // Solve the block-tridiagonal system of a column, one lane per chunk of m
 // layers (lane k of the column's G): eq(j, a, bl, c, rhs), called for j = 0 ..
 // m - 1 in turn, gives the equation bl x_{l-1} + a x_l + c x_{l+1} = rhs of the
 // lane's j-th layer (bl zero at the column's first layer, c at its last, and
 // the identity past its end); mid() is called between the elimination and the
-// reduction; seen(j, x) for every layer of the lane.  The solution is left in
-// mine[(j * kChunkElems + r) * 32].
-template <int G, class Eq, class Mid, class Seen>
-__device__ __forceinline__ void chunk_solve(int m, int k, double* mine, Eq&& eq, Mid&& mid,
-                                            Seen&& seen) {
+// reduction.  The solution is left in mine[(j * kChunkElems + r) * 32], the sum of
+// its first row over the lane's first `left` layers in sum_x.
+//
+// Returns whether the column is to be solved again by chunk_sequence: chunks and
+// the cyclic reduction eliminate stretches of layers that are open at both ends.
+// Where a stretch traps a wave (vertical flow converging in it, at vertical
+// Courant numbers far above one) its block is nearly singular although the
+// column's system is not, and the entries that the elimination makes of it grow by
+// as much as its result loses in digits; the elimination from the lower wall up
+// meets no such stretch.  So a column goes there whose Q, S or first B and C have
+// diagonal entries above `limit`.  Error against 80-bit solutions, 6500 columns of 9
+// to 256 layers, Courant numbers 0.5 to 10^4, vertical Mach numbers 3e-4 to 1.5: of
+// the columns that stay 1.15 times the sequential solve's in the mean, 3.3 times in
+// the worst hundredth, 26 at most; of those that go up to 10^11 times.  None goes at
+// Courant numbers up to 10 below Mach 0.1, nor up to 100 below Mach 0.01.  (Watching
+// every layer and every level as well kept no better and cost 7 % of the solve.)
+template <int G, class Eq, class Mid>
+__device__ __forceinline__ bool chunk_solve(int m, int k, double* mine, int limit, Eq&& eq,
+                                            Mid&& mid, int left, double& sum_x) {
+  Growth growth;
   // ---- elimination inside the chunk ----
   double Ap[3][3] = {}, f[3][3] = {}, pv[3] = {};           // A', f, p of the layer below
   double Q[3][3] = {}, S[3][3] = {}, P[3] = {};             // first layer's relation
@@ -370,6 +401,10 @@ __device__ __forceinline__ void chunk_solve(int m, int k, double* mine, Eq&& eq,
     neg_mul3(inv, t33, Bm);
     mul3(c, Qn, t33);
     neg_mul3(inv, t33, Cm);
+    growth.note(Q);
+    growth.note(S);
+    growth.note(Bm);
+    growth.note(Cm);
   }
   // y_k + B y_{k-h} + C y_{k+h} = r, strides h = 1, 2, 4, ...: a chunk without
   // a neighbour at that distance has a zero block there, so the values that the
@@ -416,7 +451,7 @@ __device__ __forceinline__ void chunk_solve(int m, int k, double* mine, Eq&& eq,
     x[r] = y[r];
     mine[((size_t)(m - 1) * kChunkElems + r) * 32] = x[r];
   }
-  seen(m - 1, x);
+  sum_x = m - 1 < left ? x[0] : 0.;
   for (int j = m - 2; j >= 0; --j) {
     double* at = mine + (size_t)j * kChunkElems * 32;
     double t[3];
@@ -430,8 +465,178 @@ __device__ __forceinline__ void chunk_solve(int m, int k, double* mine, Eq&& eq,
     }
 #pragma unroll
     for (int r = 0; r < 3; ++r) at[r * 32] = x[r] = t[r];
-    seen(j, x);
+    if (j < left) sum_x += x[0];
   }
+  const unsigned grown = __ballot_sync(0xffffffffu, growth.hi >= limit);
+  return grown >> (threadIdx.x & (32 - G)) & (0xffffffffu >> (32 - G));
+}
+
+// The same system of the columns that `again` is set for, layer after layer: the
+// column's lanes take turns, from the lower wall up and back.  A layer costs a
+// whole warp's issue: with every column of the block here, 512 of 256 layers 19 ->
+// 189 us (one thread a column, in the column sweep, 239), 16384 of 128 layers 155
+// -> 1816 (296).  From both walls at once with the blocks formed beforehand it took
+// 1163 us there, but lost a supersonic column (6e-3) and cost the batched kernel 500
+// us of 860 in registers.
+template <int G, class Eq>
+__device__ __forceinline__ void chunk_sequence(int m, int k, double* mine, bool again, Eq&& eq) {
+  double Ap[3][3] = {}, pv[3] = {}, a[3][3], bl[3][3], c[3][3], rhs[3];
+#pragma unroll 1
+  for (int t = 0; t < G; ++t) {
+    if (k == t && again) {
+#pragma unroll 1
+      for (int j = 0; j < m; ++j) {
+        double inv[3][3];
+        eq(j, a, bl, c, rhs);
+        sub_mul3(bl, Ap, a);
+        sub_mul3(bl, pv, rhs);
+        chunk_inverse(a, inv);
+        mul3(inv, c, Ap);
+        mul3(inv, rhs, pv);
+        if (j == m - 1) break;  // (its p and A' stay in registers)
+        double* out = mine + (size_t)j * kChunkElems * 32;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          out[r * 32] = pv[r];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) out[(3 + r * 3 + q) * 32] = Ap[r][q];
+        }
+      }
+    }
+    double up[3][3], pu[3];
+    shfl3<G>(Ap, t, up);
+    shfl3<G>(pv, t, pu);
+    if (k == t + 1) {
+#pragma unroll
+      for (int r = 0; r < 3; ++r) {
+        pv[r] = pu[r];
+#pragma unroll
+        for (int q = 0; q < 3; ++q) Ap[r][q] = up[r][q];
+      }
+    }
+  }
+  double x[3] = {};  // (the column's last A' is zero)
+#pragma unroll 1
+  for (int t = G - 1; t >= 0; --t) {
+    if (k == t && again) {
+      sub_mul3(Ap, x, pv);
+#pragma unroll
+      for (int r = 0; r < 3; ++r) mine[((size_t)(m - 1) * kChunkElems + r) * 32] = x[r] = pv[r];
+#pragma unroll 1
+      for (int j = m - 2; j >= 0; --j) {
+        double* at = mine + (size_t)j * kChunkElems * 32;
+        double y3[3];
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+          y3[r] = at[r * 32];
+#pragma unroll
+          for (int q = 0; q < 3; ++q) y3[r] = fma(-at[(3 + r * 3 + q) * 32], x[q], y3[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; ++r) at[r * 32] = x[r] = y3[r];
+      }
+    }
+    double above[3];
+    shfl3<G>(x, t, above);
+    if (k == t - 1)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) x[r] = above[r];
+  }
+}
+// the sum that chunk_solve gives, from the solution
+__device__ __forceinline__ double chunk_sum(int m, const double* mine, int left) {
+  double sum_x = 0.;
+  for (int j = m - 1; j >= 0; --j)
+    if (j < left) sum_x += mine[(size_t)j * kChunkElems * 32];
+  return sum_x;
+}
+
+// The equations of one lane's chunk: layers l0 .. l0 + m - 1 of the column at cb.
+template <class B>
+struct ChunkColumn {
+  using T = std::remove_pointer_t<decltype(B::u)>;  // stored precision
+  using BT = ChunkBlockT<B>;
+  const Geo& g;
+  const Phys& p;
+  const B& b;
+  const int cb, l0, m, sv, nl;
+  ChunkBlocks<BT> blocks;
+  BT gog;
+  double idt, rc;  // rc: density of the layer
+  double sum_r2, sum_du;
+  T rawn[5], rawd[3];
+
+  // state of layer l (clamped to the ghost above the column), as stored
+  __device__ __forceinline__ void load_w(int l, T (&raw)[5]) const {
+    const int o = cb + min(l, nl);
+#pragma unroll
+    for (int v = 0; v < 5; ++v) raw[v] = b.w[v * sv + o];
+  }
+  __device__ __forceinline__ void load_d(int l, T (&raw)[3]) const {
+    const int o = cb + min(l, nl - 1);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) raw[r] = b.D[sel<3>(r) * sv + o];
+  }
+  // full density of the layer (returned in FP64) and its cell quantities
+  __device__ __forceinline__ double make(int l, const T (&raw)[5], ChunkCell<BT>& c) const {
+    const int xi = g.il + min(l, nl);
+    const double rho = vic_full(b, (double)raw[IDN], IDN, xi);
+    c.set((BT)rho, (BT)raw[IVX], (BT)raw[IVY], (BT)raw[IVZ], vic_full_blk(b, raw[IPR], IPR, xi),
+          gog);
+    return rho;
+  }
+  __device__ __forceinline__ ChunkColumn(const Geo& g_, const Phys& p_, const B& b_, int cb_,
+                                         int l0_, int m_)
+      : g(g_), p(p_), b(b_), cb(cb_), l0(l0_), m(m_), sv((int)g_.sv), nl(g_.nx1), sum_r2(0.),
+        sum_du(0.) {
+    idt = 1. / *b.dt;
+    gog = (BT)(p.gammad / (p.gammad - 1.));
+    blocks.gm1 = (BT)(p.gammad - 1.);
+    blocks.s = (BT)g.A1 * (BT)(0.5 / g.vol);
+    blocks.idt = (BT)idt;
+    blocks.grav = (BT)p.grav1;
+    T raw0[5];
+    ChunkCell<BT> below, cell;
+    load_w(l0 - 1, rawn);
+    load_w(l0, raw0);
+    load_d(l0, rawd);
+    make(l0 - 1, rawn, below);
+    load_w(l0 + 1, rawn);
+    rc = make(l0, raw0, cell);
+    blocks.start(below, cell);
+  }
+  __device__ __forceinline__ void operator()(int j, double (&a)[3][3], double (&bl)[3][3],
+                                             double (&c)[3][3], double (&rhs)[3]) {
+    const int l = l0 + j;
+    ChunkCell<BT> cn;
+    const double rn = make(l + 1, rawn, cn);
+    double du[3];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) du[r] = l < nl ? (double)rawd[r] : 0.;
+    if (j < m - 1) {  // the next layer's inputs, ahead of this one's arithmetic
+      load_w(l + 2, rawn);
+      load_d(l + 1, rawd);
+    }
+    blocks.template next<false>(cn, l, nl, false, a, bl, c);
+#pragma unroll
+    for (int r = 0; r < 3; ++r) rhs[r] = mul(du[r], idt);
+    if (l < nl) {
+      sum_r2 = fma(rc, rc, sum_r2);
+      sum_du += du[0];
+    }
+    rc = rn;
+  }
+};
+
+// chunk_sequence of a warp's columns.  Not inlined: it is seldom called, and in
+// the body of the kernel it cost the chunked solve its registers (128^3: 50 us a
+// stage).
+template <int G, class B>
+__device__ __noinline__ void chunk_again(const Geo& g, const Phys& p, const B& b, int cb, int m,
+                                         double* mine, bool again) {
+  const int k = threadIdx.x & (G - 1);
+  ChunkColumn<B> column(g, p, b, cb, k * m, m);
+  chunk_sequence<G>(m, k, mine, again, column);
 }
 
 // The columns col0 .. col0 + 32/G - 1 of a block by one warp; sm: the warp's
@@ -452,70 +657,7 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
   double* backs = sm + ((size_t)(m - 1) * kChunkElems + 3) * 32;  // [4], then the columns' cb
   int* cbs = reinterpret_cast<int*>(backs + 4);
 
-  const double dt = *b.dt, idtd = 1. / dt;
-  const BT gog = (BT)(p.gammad / (p.gammad - 1.));
-  ChunkBlocks<BT> blocks;
-  blocks.gm1 = (BT)(p.gammad - 1.);
-  blocks.s = (BT)g.A1 * (BT)(0.5 / g.vol);
-  blocks.idt = (BT)idtd;
-  blocks.grav = (BT)p.grav1;
-
-  // state of layer l (clamped to the ghost above the column), as stored
-  auto load_w = [&](int l, T (&raw)[5]) {
-    const int o = cb + min(l, nl);
-#pragma unroll
-    for (int v = 0; v < 5; ++v) raw[v] = b.w[v * sv + o];
-  };
-  auto load_d = [&](int l, T (&raw)[3]) {
-    const int o = cb + min(l, nl - 1);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) raw[r] = b.D[sel<3>(r) * sv + o];
-  };
-  // full density of the layer (returned in FP64) and its cell quantities
-  auto make = [&](int l, const T (&raw)[5], ChunkCell<BT>& c) {
-    const int xi = g.il + min(l, nl);
-    const double rho = vic_full(b, (double)raw[IDN], IDN, xi);
-    c.set((BT)rho, (BT)raw[IVX], (BT)raw[IVY], (BT)raw[IVZ], vic_full_blk(b, raw[IPR], IPR, xi),
-          gog);
-    return rho;
-  };
-
-  double sum_r2 = 0., sum_du = 0.;
-  T rawn[5], rawd[3];
-  double rc;  // density of the layer
-  {
-    T raw0[5];
-    ChunkCell<BT> below, cell;
-    load_w(l0 - 1, rawn);
-    load_w(l0, raw0);
-    load_d(l0, rawd);
-    make(l0 - 1, rawn, below);
-    load_w(l0 + 1, rawn);
-    rc = make(l0, raw0, cell);
-    blocks.start(below, cell);
-  }
-  auto equation = [&](int j, double (&a)[3][3], double (&bl)[3][3], double (&c)[3][3],
-                      double (&rhs)[3]) {
-    const int l = l0 + j;
-    ChunkCell<BT> cn;
-    const double rn = make(l + 1, rawn, cn);
-    double du[3];
-#pragma unroll
-    for (int r = 0; r < 3; ++r) du[r] = l < nl ? (double)rawd[r] : 0.;
-    if (j < m - 1) {  // the next layer's inputs, ahead of this one's arithmetic
-      load_w(l + 2, rawn);
-      load_d(l + 1, rawd);
-    }
-    blocks.template next<false>(cn, l, nl, false, a, bl, c);
-#pragma unroll
-    for (int r = 0; r < 3; ++r) rhs[r] = mul(du[r], idtd);
-    if (l < nl) {
-      sum_r2 = fma(rc, rc, sum_r2);
-      sum_du += du[0];
-    }
-    rc = rn;
-  };
-
+  ChunkColumn<B> column(g, p, b, cb, l0, m);
   // The finish's inputs of the lane's first IT cells, fetched before the
   // reduction so that it hides their latency; further ones batch by batch.
   constexpr int IT = sizeof(T) == 4 ? (NS == 0 ? 4 : 2) : (NS == 0 ? 2 : 1), NSA = NS > 0 ? NS : 1;
@@ -595,14 +737,15 @@ __device__ __forceinline__ void vic_chunk(const Geo& g, const Phys& p, const B& 
       }
     }
   };
-  double sum_x = 0.;
-  chunk_solve<G>(m, k, mine, equation, [&] { fetch(lane); },
-                 [&](int j, const double (&x)[3]) {
-                   if (l0 + j < nl) sum_x += x[0];
-                 });
-
-  // ---- mass redistribution factor of the column: sum(du - x) / sum(rho^2) ----
-  double lost = sum_du - sum_x;
+  double sum_x;
+  const bool again =
+      chunk_solve<G>(m, k, mine, kGrowthLimit<BT>, column, [&] { fetch(lane); }, nl - l0, sum_x);
+  if (__any_sync(0xffffffffu, again)) {
+    chunk_again<G, B>(g, p, b, cb, m, mine, again);
+    sum_x = chunk_sum(m, mine, nl - l0);
+  }
+  double sum_r2 = column.sum_r2;
+  double lost = column.sum_du - sum_x;
 #pragma unroll
   for (int h = 1; h < G; h *= 2) {
     lost += __shfl_xor_sync(0xffffffffu, lost, h, G);
