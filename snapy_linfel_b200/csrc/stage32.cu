@@ -99,8 +99,15 @@ struct Shared32 {
   Phys p;
   Finish32 fin;
 };
+// (one variable for the kernels and the functions they call, so that these know its
+// address: through a pointer every field was a generic load)
+__device__ __forceinline__ Shared32& shared32() {
+  __shared__ Shared32 s;
+  return s;
+}
 
-template <int NS>
+// UPDATE: the RK combination, else du for the implicit solve
+template <int NS, bool UPDATE>
 __device__ __forceinline__ void finalize32(const Finish32& c, int off, int xi, const float* d,
                                            const float* wc) {
   const int sv = c.sv;
@@ -125,31 +132,46 @@ __device__ __forceinline__ void finalize32(const Finish32& c, int off, int xi, c
   float ds[NS > 0 ? NS : 1];
 #pragma unroll
   for (int n = 0; n < NS; ++n) ds[n] = -dt * (d[5 + n] * c.ivol);
-  if (c.write_du) {
+  if constexpr (!UPDATE) {
 #pragma unroll
     for (int v = 0; v < 5; ++v) c.D[v * sv + off] = du[v];
 #pragma unroll
     for (int n = 0; n < NS; ++n) c.D[(5 + n) * sv + off] = ds[n];
     return;
   }
+  // All loads before the first store: the compiler cannot see that the stores miss
+  // them and would wait for one load per variable.  x3 of an explicit 96^3 block,
+  // Roe 64 -> 37 us, with two tracers 119 -> 57; of 6 members, HLLC 342 -> 149 us.
+  float *u = c.u, *u0 = c.u0, *sc = c.s, *sc0 = c.s0, *mix = c.r;
+  const float w0 = c.w0, w1 = c.w1, w2 = c.w2, rref = c.rbf[xi];
+  const bool stage0 = c.stage0;
+  float uo[5], u0v[5], so[NS > 0 ? NS : 1], s0v[NS > 0 ? NS : 1];
+#pragma unroll
+  for (int v = 0; v < 5; ++v) {
+    uo[v] = u[v * sv + off];
+    u0v[v] = stage0 ? uo[v] : u0[v * sv + off];
+  }
+#pragma unroll
+  for (int n = 0; n < NS; ++n) {
+    so[n] = sc[n * sv + off];
+    s0v[n] = stage0 ? so[n] : sc0[n * sv + off];
+  }
   float unew_rho = 0.f;
 #pragma unroll
   for (int v = 0; v < 5; ++v) {
     const int o = v * sv + off;
-    const float uo = c.u[o], u0v = c.stage0 ? uo : c.u0[o];
-    if (c.stage0) c.u0[o] = uo;
-    const float un = fmaf(c.w2, du[v], fmaf(c.w1, uo, c.w0 * u0v));
-    c.u[o] = un;
-    if (v == IDN) unew_rho = c.rbf[xi] + un;
+    if (stage0) u0[o] = uo[v];
+    const float un = fmaf(w2, du[v], fmaf(w1, uo[v], w0 * u0v[v]));
+    u[o] = un;
+    if (v == IDN) unew_rho = rref + un;
   }
 #pragma unroll
   for (int n = 0; n < NS; ++n) {
     const int o = n * sv + off;
-    const float so = c.s[o], s0v = c.stage0 ? so : c.s0[o];
-    if (c.stage0) c.s0[o] = so;
-    const float sn = fmaf(c.w2, ds[n], fmaf(c.w1, so, c.w0 * s0v));
-    c.s[o] = sn;
-    if (c.r) c.r[o] = sn / unew_rho;
+    if (stage0) sc0[o] = so[n];
+    const float sn = fmaf(w2, ds[n], fmaf(w1, so[n], w0 * s0v[n]));
+    sc[o] = sn;
+    if (mix) mix[o] = sn / unew_rho;
   }
 }
 
@@ -196,12 +218,15 @@ constexpr double kX1Resident32 = 148. * 24.;
 // 384 x 384 x 192, Roe, two tracers 1.29 -> 1.25 ms, 512 x 256 21.0 -> 10.7 us,
 // 48 members of 64 and 128 layers 1.57 -> 1.47 ms.
 template <int NS, int FP>
-__device__ __noinline__ void x1_32_item(const Shared32* sh, int64_t item, float* row, int last) {
+__device__ __noinline__ void x1_32_item(int64_t item, int last) {
   constexpr int NV = 5 + NS;
-  const Geo& g = sh->m.g;
-  const StageBufs32& b = sh->m.b;
-  const Phys& p = sh->p;
-  const X1Split sp = sh->m.x1;
+  extern __shared__ float x1_rows32[];
+  float* row = x1_rows32;
+  const Shared32& sh = shared32();
+  const Geo& g = sh.m.g;
+  const StageBufs32& b = sh.m.b;
+  const Phys& p = sh.p;
+  const X1Split sp = sh.m.x1;
   const int lane = threadIdx.x & 31;
   const int nc1 = g.nc1, il = g.il, iu = g.iu, ng = g.ng, pitch = sp.pitch;
   const int sv = (int)g.sv;  // (element indices stay below 2^31: check_config)
@@ -343,7 +368,10 @@ __device__ __noinline__ void x1_32_item(const Shared32* sh, int64_t item, float*
           wc[IDN] = w[IDN * sv + off];
 #pragma unroll
           for (int v = 1; v < 5; ++v) wc[v] = cell[v * pitch - 1];
-          finalize32<NS>(sh->fin, off, c - 1, d, wc);
+          if (sh.fin.write_du)
+            finalize32<NS, false>(sh.fin, off, c - 1, d, wc);
+          else
+            finalize32<NS, true>(sh.fin, off, c - 1, d, wc);
         } else {
 #pragma unroll
           for (int v = 0; v < NV; ++v) D[v * sv + off] = d[v];
@@ -363,8 +391,7 @@ __device__ __noinline__ void x1_32_item(const Shared32* sh, int64_t item, float*
 template <int NS, int FP>
 __global__ void __launch_bounds__(32, 20) k_x1_32(Geo g, Phys p, StageBufs32 b, X1Split sp,
                                                   int last) {
-  extern __shared__ float x1_rows32[];
-  __shared__ Shared32 sh;
+  Shared32& sh = shared32();
   if (threadIdx.x == 0) {
     sh.m.g = g;
     sh.m.b = b;
@@ -373,16 +400,25 @@ __global__ void __launch_bounds__(32, 20) k_x1_32(Geo g, Phys p, StageBufs32 b, 
     sh.fin.set(g, p, b);
   }
   __syncwarp();
-  x1_32_item<NS, FP>(&sh, blockIdx.x, x1_rows32, last);
+  x1_32_item<NS, FP>(blockIdx.x, last);
 }
 
 // ---------------------------------------------------------------------------
 // x2 / x3 marching sweeps (reference constant along the sweep)
 // ---------------------------------------------------------------------------
-// resident CTAs per SM: the register budget that holds the window of 5 + NS
-// variables without spilling it
-template <int NS, int FP>
-constexpr int kMarchCtas32 = NS >= 2 ? 4 : (NS == 0 && FP == 1 ? 6 : 5);
+// What a march does with a cell's sums: keeps them for the next sweep, forms du for
+// the implicit solve, or updates the cell.
+enum { kKeep = 0, kTendency = 1, kUpdate = 2 };
+inline int march_end(const Phys& p, bool last) {
+  return !last ? kKeep : (p.implicit_scheme ? kTendency : kUpdate);
+}
+// Resident CTAs per SM: the register budget that holds the window of 5 + NS
+// variables, and for kUpdate also the cell's old state, without spilling them.
+// (With the end read at run time every march held what the update needs: x2 of 6
+// members, LMARS, 68 -> 84 us.)
+template <int NS, int FP, int END>
+constexpr int kMarchCtas32 = END == kUpdate ? (NS >= 2 ? 3 : (FP == 1 && NS == 0 ? 5 : 4))
+                                            : (NS >= 2 ? 4 : (FP == 1 ? (NS == 0 ? 6 : 5) : 4));
 
 // One thread's work: line tid (x1 cell x other horizontal index) and face
 // segment seg of the sweep axis.  Cell centred (cells.cuh); per stage x2 and x3
@@ -392,13 +428,13 @@ constexpr int kMarchCtas32 = NS >= 2 ? 4 : (NS == 0 && FP == 1 ? 6 : 5);
 // the batched kernel round alike, and the descriptor's fields are read from
 // shared memory when they are needed instead of being held in registers
 // (copied into registers the batched kernel spilled).
-template <int NS, int AX, int FP>
-__device__ __noinline__ void march32_line(const Shared32* sh, int first, int last, int tid,
-                                          int seg) {
-  const Geo& g = sh->m.g;
-  const StageBufs32& b = sh->m.b;
-  const Phys& p = sh->p;
-  const int seglen = AX == 2 ? sh->m.seglen2 : sh->m.seglen3;
+template <int NS, int AX, int FP, int END>
+__device__ __noinline__ void march32_line(int first, int tid, int seg) {
+  const Shared32& sh = shared32();
+  const Geo& g = sh.m.g;
+  const StageBufs32& b = sh.m.b;
+  const Phys& p = sh.p;
+  const int seglen = AX == 2 ? sh.m.seglen2 : sh.m.seglen3;
   constexpr int NV = 5 + NS;
   const int ni = g.iu - g.il + 1;
   int lo, hi, olo, ohi;
@@ -484,14 +520,14 @@ __device__ __noinline__ void march32_line(const Shared32* sh, int first, int las
           d[v] = A * F[v] - A * Fp[v];
           if (!first) d[v] = dprev[v] + d[v];
         }
-        if (last) {
+        if constexpr (END == kKeep) {
+#pragma unroll
+          for (int v = 0; v < NV; ++v) D[v * svi + off] = d[v];
+        } else {
           float wc[5];
 #pragma unroll
           for (int v = 0; v < 5; ++v) wc[v] = q[v][1];
-          finalize32<NS>(sh->fin, off, i, d, wc);
-        } else {
-#pragma unroll
-          for (int v = 0; v < NV; ++v) D[v * svi + off] = d[v];
+          finalize32<NS, END == kUpdate>(sh.fin, off, i, d, wc);
         }
       }
 #pragma unroll
@@ -506,10 +542,10 @@ __device__ __noinline__ void march32_line(const Shared32* sh, int first, int las
   }
 }
 
-template <int NS, int AX, int FP>
-__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>) k_march32(Geo g, Phys p, StageBufs32 b, int seglen,
-                                                    int first, int last) {
-  __shared__ Shared32 sh;
+template <int NS, int AX, int FP, int END>
+__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP, END>)
+    k_march32(Geo g, Phys p, StageBufs32 b, int seglen, int first) {
+  Shared32& sh = shared32();
   // (each of the copies by its own warp: they are one after the other's latency
   // otherwise)
   if (threadIdx.x == 0) {
@@ -523,7 +559,7 @@ __global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>) k_march32(Geo g, Ph
     sh.fin.set(g, p, b);
   }
   __syncthreads();
-  march32_line<NS, AX, FP>(&sh, first, last, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
+  march32_line<NS, AX, FP, END>(first, blockIdx.x * blockDim.x + threadIdx.x, blockIdx.y);
 }
 
 // ---------------------------------------------------------------------------
@@ -650,8 +686,7 @@ __global__ void __launch_bounds__(256) k_cfl32(Geo g, double gammad, CflUse use,
 template <int NS, int FP>
 __global__ void __launch_bounds__(32, 20)
     k_x1_32_batch(const Member32* __restrict__ mem, Phys p, WorkQueue q, int stage, int last) {
-  extern __shared__ float x1_rows32[];
-  __shared__ Shared32 sh;
+  Shared32& sh = shared32();
   const int lane = threadIdx.x;
   unsigned long long item = 0, ahead = 0;
   if (lane == 0) {
@@ -675,17 +710,15 @@ __global__ void __launch_bounds__(32, 20)
       __syncwarp();
       m = nm;
     }
-    x1_32_item<NS, FP>(&sh, tile, x1_rows32, last);
+    x1_32_item<NS, FP>(tile, last);
     item = __shfl_sync(0xffffffffu, ahead, 0);
   }
 }
 
-template <int NS, int AX, int FP>
-__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>)
-    k_march32_batch(const Member32* __restrict__ mem, Phys p,
-                                                       WorkQueue q, int stage, int first,
-                                                       int last) {
-  __shared__ Shared32 sh;
+template <int NS, int AX, int FP, int END>
+__global__ void __launch_bounds__(128, kMarchCtas32<NS, FP, END>)
+    k_march32_batch(const Member32* __restrict__ mem, Phys p, WorkQueue q, int stage, int first) {
+  Shared32& sh = shared32();
   if (threadIdx.x == 0) sh.p = p;
   int m, have = -1;
   int64_t tile;
@@ -701,7 +734,7 @@ __global__ void __launch_bounds__(128, kMarchCtas32<NS, FP>)
     }
     const int nseg = AX == 2 ? sh.m.nseg2 : sh.m.nseg3;
     const int blk = udiv(tile, nseg);
-    march32_line<NS, AX, FP>(&sh, first, last, blk * blockDim.x + threadIdx.x,
+    march32_line<NS, AX, FP, END>(first, blk * blockDim.x + threadIdx.x,
                              (int)tile - blk * nseg);
   }
 }
@@ -774,18 +807,31 @@ cudaError_t launch_x1_32_batch(const Member32* mem, const Phys& p, const WorkQue
   });
 }
 
+// f(AX, END): the x3 march is the last sweep wherever there is one
+template <class F>
+static cudaError_t with_axis_end(int axis, int end, F&& f) {
+  using std::integral_constant;
+  if (axis == 3)
+    return end == kUpdate ? f(integral_constant<int, 3>{}, integral_constant<int, kUpdate>{})
+                          : f(integral_constant<int, 3>{}, integral_constant<int, kTendency>{});
+  switch (end) {
+    case kKeep: return f(integral_constant<int, 2>{}, integral_constant<int, kKeep>{});
+    case kTendency: return f(integral_constant<int, 2>{}, integral_constant<int, kTendency>{});
+    default: return f(integral_constant<int, 2>{}, integral_constant<int, kUpdate>{});
+  }
+}
+
 cudaError_t launch_march32_batch(int axis, const Member32* mem, const Phys& p,
                                  const WorkQueue& q, int stage, bool first, bool last,
                                  const PersistGrid& pg, cudaStream_t st) {
   return with_ns_profile(p.nscalar, face_profile32(p, axis), [&](auto ns, auto fp) {
-    constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
-    if (axis == 2)
-      k_march32_batch<NS, 2, FP><<<persistent_grid(k_march32_batch<NS, 2, FP>, 128, 0, pg), 128,
-                                   0, st>>>(mem, p, q, stage, first, last);
-    else
-      k_march32_batch<NS, 3, FP><<<persistent_grid(k_march32_batch<NS, 3, FP>, 128, 0, pg), 128,
-                                   0, st>>>(mem, p, q, stage, first, last);
-    return cudaGetLastError();
+    return with_axis_end(axis, march_end(p, last), [&](auto ax, auto end) {
+      constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
+      constexpr int AX = decltype(ax)::value, END = decltype(end)::value;
+      const auto kernel = k_march32_batch<NS, AX, FP, END>;
+      kernel<<<persistent_grid(kernel, 128, 0, pg), 128, 0, st>>>(mem, p, q, stage, first);
+      return cudaGetLastError();
+    });
   });
 }
 
@@ -835,26 +881,22 @@ cudaError_t launch_x1_32(const Geo& g, const Phys& p, const StageBufs32& b, bool
   });
 }
 
-template <int NS, int AX, int FP>
-static cudaError_t launch_march32_t(const Geo& g, const Phys& p, const StageBufs32& b,
-                                    bool first, bool last, cudaStream_t st) {
-  int ni = g.iu - g.il + 1;
-  int no = AX == 2 ? g.ku - g.kl + 1 : g.ju - g.jl + 1;
-  int n = AX == 2 ? g.nx2 : g.nx3;
-  int seglen = 32;
-  int64_t threads = (int64_t)ni * no;
-  while (seglen > 8 && threads * ((n + seglen - 1) / seglen) < 148LL * 1024 * 2) seglen /= 2;
-  dim3 grid((unsigned)((threads + 127) / 128), (unsigned)((n + seglen - 1) / seglen));
-  k_march32<NS, AX, FP><<<grid, 128, 0, st>>>(g, p, b, seglen, first ? 1 : 0, last ? 1 : 0);
-  return cudaGetLastError();
-}
-
 cudaError_t launch_march32(int axis, const Geo& g, const Phys& p, const StageBufs32& b,
                            bool first, bool last, cudaStream_t st) {
+  const int ni = g.iu - g.il + 1;
+  const int no = axis == 2 ? g.ku - g.kl + 1 : g.ju - g.jl + 1;
+  const int n = axis == 2 ? g.nx2 : g.nx3;
+  int seglen = 32;
+  const int64_t threads = (int64_t)ni * no;
+  while (seglen > 8 && threads * ((n + seglen - 1) / seglen) < 148LL * 1024 * 2) seglen /= 2;
+  const dim3 grid((unsigned)((threads + 127) / 128), (unsigned)((n + seglen - 1) / seglen));
   return with_ns_profile(p.nscalar, face_profile32(p, axis), [&](auto ns, auto fp) {
-    constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
-    return axis == 2 ? launch_march32_t<NS, 2, FP>(g, p, b, first, last, st)
-                     : launch_march32_t<NS, 3, FP>(g, p, b, first, last, st);
+    return with_axis_end(axis, march_end(p, last), [&](auto ax, auto end) {
+      constexpr int NS = decltype(ns)::value, FP = decltype(fp)::value;
+      constexpr int AX = decltype(ax)::value, END = decltype(end)::value;
+      k_march32<NS, AX, FP, END><<<grid, 128, 0, st>>>(g, p, b, seglen, first ? 1 : 0);
+      return cudaGetLastError();
+    });
   });
 }
 
