@@ -1,6 +1,5 @@
 // sweep64.cuh — the FP64 sweeps of one RK stage as templates over the scalar
-// count and the face profile; instantiated per scalar count by
-// sweep64_ns{0,1,2,3}.cu so that they compile side by side.
+// count and the face profile, instantiated by the launchers of stage.cu.
 //
 //   k_x1     x1 (the contiguous, vertical axis): each WARP works on its own
 //            group of x1 columns (or one segment of a long column when there
@@ -150,9 +149,11 @@ constexpr size_t march_smem_bytes() {
 // thread's window now lives in its own ring of six cells in shared memory
 // (layout [slot][variable][thread], no barriers; the incoming cell by cp.async
 // a step ahead), which leaves 128 registers and 16 warps.  384 x 384 x 192,
-// Roe, two tracers: x2 3.67 -> 1.42 ms, x3 4.19 -> 1.49 ms a stage.
+// Roe, two tracers: x2 3.67 -> 1.42 ms, x3 4.19 -> 1.49 ms a stage.  The run-time
+// profile needs more than 128 registers: three CTAs, 96^3 with WENO3 x2 69.6 -> 61.9
+// us, x3 120 -> 112.
 template <int NS, int AX, int RP, int SV>
-__global__ void __launch_bounds__(kMarchThreads, 4)
+__global__ void __launch_bounds__(kMarchThreads, RP == 0 ? 3 : 4)
     k_march(Geo g, Phys p, StageBufs b, int seglen, int first, int last) {
   constexpr int NV = 5 + NS;
   constexpr int SL = NV * kMarchThreads;  // doubles per slot
