@@ -2,18 +2,20 @@
 //
 // Many independent mesh blocks (ensemble members of different sizes, same
 // physics) advance together: each sweep of an RK stage is ONE persistent
-// launch over all members, whose CTAs pull (member, tile) work items from a
-// device counter until the queue is drained, so small and large members
-// share the SMs without a launch per member and without tail effects at
-// member boundaries.  Per stage: x1 sweep, x2 sweep, x3 sweep, implicit
-// column, implicit finish, boundary fills — six to seven launches for the
-// whole ensemble.  dt is per member and stays on the device (a per-member CFL
-// reduction), so a whole step can be captured in one CUDA graph.
+// launch over all members, whose CTAs pull (member, item) work from a device
+// counter until the queue is drained, so small and large members share the SMs
+// without a launch per member and without tail effects at member boundaries.
+// Per stage: x1, x2 and x3 sweep, the implicit solve, boundary fills.  The solve
+// is one launch per lane count that some member's columns take (8, 16 or 32, one
+// to three of them; vic_chunk.cu), and the column + finish pair for members that
+// it does not take: five to nine launches for the whole ensemble.  dt is per
+// member and stays on the device (a per-member CFL reduction), so a whole step
+// can be captured in one CUDA graph.
 //
-// The tile shapes (x1 columns per CTA, march segment length, implicit column
-// block, persistent CTAs per SM) are parameters of the plan; the project's
-// autotuner (snapy_linfel_b200/ensemble.py) times candidates on the live
-// ensemble and keeps the fastest.
+// The item shapes (x1 columns per item, march segment length, the column
+// kernel's block, persistent CTAs per SM) are parameters of the plan; the
+// project's autotuner (snapy_linfel_b200/ensemble.py) times candidates on the
+// live ensemble and keeps the fastest.
 //
 // Reference: each member is one snapy MeshBlock (MeshBlockImpl::forward,
 // src/mesh/meshblock.cpp:577-786); the reference has no batched form.

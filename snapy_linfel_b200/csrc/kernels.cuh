@@ -91,8 +91,6 @@ struct WorkQueue {
   unsigned long long* counter;
 };
 
-// Next (member, tile) for the whole CTA; false when the queue is drained.
-// Every thread of the CTA must call it.
 // (member, tile) of a work item (false past the last item): binary search of
 // the per-member prefix table
 __device__ __forceinline__ bool queue_find(const WorkQueue& q, int64_t item, int& m,
@@ -109,6 +107,8 @@ __device__ __forceinline__ bool queue_find(const WorkQueue& q, int64_t item, int
   return true;
 }
 
+// Next (member, tile) for the whole CTA; false when the queue is drained.
+// Every thread of the CTA must call it.
 __device__ __forceinline__ bool queue_next(const WorkQueue& q, int& m, int64_t& tile) {
   __shared__ unsigned long long s_item;
   __syncthreads();
@@ -135,18 +135,18 @@ inline void raise_smem_limit(K kernel, size_t bytes) {
   done.emplace_back(dev, f);
 }
 
-// Copy member m's descriptor into shared memory, whole CTA, then barrier.  Call
-// it right after queue_next (whose leading barrier ends the previous tile).
+// Copy member m's descriptor into shared memory by one warp (no CTA barrier; the
+// warp's lanes see it after __syncwarp, the others after the next CTA barrier).
 // Kernels then read the fields as they need them instead of holding the
 // ~50-word struct in registers for the whole tile.
-// the same copy by one warp (no CTA barrier; the warp's lanes see it after
-// __syncwarp, the others after the next CTA barrier)
 __device__ __forceinline__ void load_member_warp(Member32& dst, const Member32* mem, int m) {
   const int* src = reinterpret_cast<const int*>(mem + m);
   int* d = reinterpret_cast<int*>(&dst);
   for (int k = threadIdx.x & 31; k < (int)(sizeof(Member32) / sizeof(int)); k += 32) d[k] = src[k];
   __syncwarp();
 }
+// The same by the whole CTA, then a barrier; right after queue_next (whose leading
+// barrier ends the previous tile).
 __device__ __forceinline__ void load_member(Member32& dst, const Member32* mem, int m) {
   static_assert(sizeof(Member32) % sizeof(int) == 0, "member descriptor copy");
   const int* src = reinterpret_cast<const int*>(mem + m);

@@ -184,14 +184,6 @@ __device__ __forceinline__ void riemann_flux_split(int solver, const float* L, c
 // 3 are the default reconstruction (WENO5 for density and scalars, the linear
 // 5-point interpolation for velocities and pressure, no scaling) with the
 // LMARS, HLLC and Roe solvers.  The host picks the profile (face_profile32).
-template <int FP>
-__device__ __forceinline__ void sweep_face_states(int typ, bool scale, int v, const float* q,
-                                                  float& wl, float& wr) {
-  if constexpr (FP == 0)
-    face_states<float>(typ, scale, q, wl, wr);
-  else
-    face_states<float>(v == IDN || v >= 5 ? SNAPB_RECON_WENO5 : SNAPB_RECON_CP5, false, q, wl, wr);
-}
 // the face values of a cell (cells.cuh), the mixing ratios clipped at zero
 template <int FP>
 __device__ __forceinline__ void sweep_cell_states(int typ, bool scale, int v, const float* q,
@@ -216,17 +208,6 @@ __device__ __forceinline__ void sweep_riemann(int solver, const float* L, const 
     roe_flux_split(L, R, pl, pr, ivx, gamma, F);
   else
     riemann_flux_split(solver, L, R, pl, pr, pf, ivx, gamma, F);
-}
-
-// linear interpolation weights of the face states (cp5, cp3, dc): the value at
-// the right face of q[2] (wl) and the left face of q[3] (wr) from six cells
-__device__ __forceinline__ bool linear_face_states(int type, const float* q, float& wl,
-                                                   float& wr) {
-  if (type == SNAPB_RECON_CP5 || type == SNAPB_RECON_CP3 || type == SNAPB_RECON_DC) {
-    face_states<float>(type, false, q, wl, wr);
-    return true;
-  }
-  return false;
 }
 
 }  // namespace snapb

@@ -197,7 +197,8 @@ size_t x1_smem32_per_column(const Geo& g, int nvt) {
 // ---------------------------------------------------------------------------
 // x1 sweep
 // ---------------------------------------------------------------------------
-constexpr size_t kX1RowBytes32 = 7 * 1024;  // rows of a warp: 24 and more warps per SM
+constexpr size_t kX1RowBytes32 = 7 * 1024;  // rows of a warp: shared memory for 24 of them per SM
+// warps that the split's rule takes to be resident (the registers hold 20 per SM)
 constexpr double kX1Resident32 = 148. * 24.;
 
 // One item (X1Split, cells.cuh) by one warp, with its rows (full density
@@ -762,7 +763,7 @@ __global__ void __launch_bounds__(256) k_bc32_batch(const Member32* __restrict__
   }
 }
 
-// Face profile of the FP32 sweeps along `axis` (sweep_face_states, pert.cuh):
+// Face profile of the FP32 sweeps along `axis` (sweep_cell_states, pert.cuh):
 // 1, 2, 3 for the default reconstruction with LMARS, HLLC, Roe; 0 otherwise.
 int face_profile32(const Phys& p, int axis) {
   const int typ = axis == 1 ? p.r1_type : p.r23_type;
