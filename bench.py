@@ -113,12 +113,18 @@ def kernel_io_bytes_per_cell(name, cfg, elem=8) -> int:
 
 
 def launches_per_step(cfg) -> int:
-    diff = cfg.nu_iso > 0 or cfg.kappa_iso > 0
-    a2, a3 = cfg.nx2 > 1, cfg.nx3 > 1
-    sep_final = (not a2 and not a3) and diff
-    per_stage = 1 + int(diff) + int(a2) + int(a3) + int(sep_final) + 3 * int(cfg.implicit_scheme != 0)
-    per_stage += 1 + int(cfg.nscalar > 0)  # boundary fills of u (and s)
-    return 3 * per_stage + 4  # + CFL fill / reduce / final + dt scaling
+    """kernels of one FP64 step: CFL reduction + dt scaling, then per stage the
+    sweeps (and diffusion), a 1-D block's finish, the implicit solve (one kernel
+    for 3x3 blocks and columns of up to 1216 layers, two for 5x5, three for longer
+    ones) and the boundary fills, which an explicit 1-D block's finish does itself"""
+    line = cfg.nx2 == 1 and cfg.nx3 == 1
+    vic = (0 if not cfg.implicit_scheme else
+           2 if cfg.implicit_scheme & 8 else 1 if cfg.nx1 <= 1216 else 3)
+    per_stage = (1 + int(cfg.nu_iso > 0 or cfg.kappa_iso > 0) + int(cfg.nx2 > 1) +
+                 int(cfg.nx3 > 1) + int(line) + vic)
+    if not (line and not cfg.implicit_scheme):
+        per_stage += 1 + int(cfg.nscalar > 0)
+    return 3 * per_stage + 2
 
 
 class ClockSampler:
@@ -310,8 +316,8 @@ def rel_errors(a, b, it):
 # member groups of the end-to-end form (copies of one group overlap the others' steps)
 E2E_GROUPS = 4
 
-NCU_TRAFFIC_PER_CELL_F32 = {"x1_sweep": 69.3, "x2_sweep": 66.1, "x3_sweep": 66.1,
-                            "implicit_vic": 347.2}
+NCU_TRAFFIC_PER_CELL_F32 = {"x1_sweep": 67.7, "x2_sweep": 64.3, "x3_sweep": 64.2,
+                            "implicit_vic": 101.8}
 
 
 def dominant_roofline(kern, cfg, cells, elem, peak, peak_src):
@@ -519,17 +525,24 @@ def run_adjoint_timing(args, opts, state, cells, stream, barrier):
             "value": cells * 3 / (rev_ms / 1e3) / 1e6, "unit": "Mcell-updates/s (reverse)"}
 
 
-def ensemble_launches_per_step(cfg, tuning=None) -> int:
-    """kernels of one batched step: CFL fill + reduce + final, then per stage
-    the x1 ghost revision (gravity along x1), the x1, x2, x3 sweeps, the
-    implicit solve (one cyclic-reduction or fused launch, or column + finish)
-    and the boundary fill(s)"""
+def ensemble_launches_per_step(cfgs, tuning=None) -> int:
+    """kernels of one batched step: CFL fill + reduce + final, then per stage the
+    x1, x2, x3 sweeps, the implicit solve (one cyclic-reduction or fused launch; by
+    default one per lane count that some member's columns take, and column +
+    finish for members that these do not take) and the boundary fill(s)"""
+    cfg = cfgs[0]
     kernel = (tuning or {}).get("vic_kernel", 0)
-    cyclic = (kernel == 1 and cfg.implicit_scheme and not (cfg.implicit_scheme >> 3) & 1
-              and cfg.nx1 <= 256)
-    vic = 1 if kernel == 2 or cyclic else 2
-    per_stage = (1 + int(cfg.grav1 != 0) + int(cfg.nx2 > 1) + int(cfg.nx3 > 1) +
-                 (vic if cfg.implicit_scheme else 0) + 1 + int(cfg.nscalar > 0))
+    cyclic = (kernel == 1 and not cfg.implicit_scheme & 8 and
+              all(c.nx1 <= 256 for c in cfgs))
+    if not cfg.implicit_scheme:
+        vic = 0
+    elif kernel == 2 or cyclic:
+        vic = 1
+    else:
+        chunk = [c.nx1 for c in cfgs if not cfg.implicit_scheme & 8 and c.nx1 <= 1216]
+        lanes = {8 if n <= 32 else 16 if n <= 64 else 32 for n in chunk}
+        vic = len(lanes) + (2 if len(chunk) < len(cfgs) else 0)
+    per_stage = 1 + int(cfg.nx2 > 1) + int(cfg.nx3 > 1) + vic + 1 + int(cfg.nscalar > 0)
     return 3 + 3 * per_stage
 
 
@@ -905,7 +918,8 @@ def run_ensemble(args):
                     "form": f"StreamedEnsemble, {E2E_GROUPS} groups on their own streams",
                     "one_stream_value": e2e_serial,
                     "d2h_bytes_per_step": nbytes},
-            "gpu_launches": ensemble_launches_per_step(cfg0, tune["best"]) * args.steps,
+            "gpu_launches": ensemble_launches_per_step([o.hydro for o, _, _ in members],
+                                                       tune["best"]) * args.steps,
             "gpu_launches_counts": "this rank's kernels in the timed region",
             "clocks": clk.summary(),
         }

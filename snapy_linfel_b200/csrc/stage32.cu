@@ -213,11 +213,12 @@ constexpr double kX1Resident32 = 148. * 24.;
 // Not inlined: the one-block and the batched kernel run this very code, so a
 // member of an ensemble rounds as it does alone.
 //
-// Bound: instruction issue (62 % active at 20 warps per SM) and the latency of
+// Bound: instruction issue (72 % active at 20 warps per SM) and the latency of
 // the conversion's loads.  Per stage, against a tile of columns per CTA (bulk
 // copies into shared memory, barriers, the revision in its own kernel):
 // 384 x 384 x 192, Roe, two tracers 1.29 -> 1.25 ms, 512 x 256 21.0 -> 10.7 us,
-// 48 members of 64 and 128 layers 1.57 -> 1.47 ms.
+// 48 members of 64 and 128 layers 1.57 -> 1.22 ms; a 1-D block of 1024 cells, whose
+// column is not cut, 85 -> 107 us.
 template <int NS, int FP>
 __device__ __noinline__ void x1_32_item(int64_t item, int last) {
   constexpr int NV = 5 + NS;
@@ -423,12 +424,13 @@ constexpr int kMarchCtas32 = END == kUpdate ? (NS >= 2 ? 3 : (FP == 1 && NS == 0
 
 // One thread's work: line tid (x1 cell x other horizontal index) and face
 // segment seg of the sweep axis.  Cell centred (cells.cuh); per stage x2 and x3
-// 0.81 + 0.85 -> 0.75 + 0.79 ms on the 48 members, 43 + 45 -> 35 + 40 us on 7
-// members of 29 to 129 layers, 0.80 + 0.84 -> 0.79 + 0.84 ms on 384 x 384 x 192
-// with two tracers.  Bound by instruction issue.  Not inlined, as x1_32_item: the one-block and
-// the batched kernel round alike, and the descriptor's fields are read from
-// shared memory when they are needed instead of being held in registers
-// (copied into registers the batched kernel spilled).
+// 0.81 + 0.85 -> 0.71 + 0.74 ms on the 48 members, 0.80 + 0.84 -> 0.79 + 0.83 on
+// 384 x 384 x 192 with two tracers.  Bound by instruction issue (70 to 74 %
+// active).  Not inlined, as x1_32_item: the one-block and the batched kernel round
+// alike (inlined into the one-block kernel it rounded Roe fluxes with one tracer
+// otherwise), and the descriptor's fields are read from shared memory when they are
+// needed instead of being held in registers (copied into registers the batched
+// kernel spilled).
 template <int NS, int AX, int FP, int END>
 __device__ __noinline__ void march32_line(int first, int tid, int seg) {
   const Shared32& sh = shared32();

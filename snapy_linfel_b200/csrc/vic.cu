@@ -1089,9 +1089,10 @@ static cudaError_t launch_vic_n(const Geo& g, const Phys& p, const B& b, cudaStr
 // of vicf.cu, =cr block cyclic reduction (vic_cr.cu, FP32 form, where it
 // applies).  The one-warp kernel was the faster at every size measured, ms per
 // stage before (pair) and after: FP64, 512 x 256 columns x layers 0.241 ->
-// 0.017, 128^3 0.327 -> 0.190, 384 x 384 x 192 with two tracers 4.38 -> 3.00;
-// FP32, 512 x 256 0.238 -> 0.017, 384 x 384 x 192 3.58 -> 2.49, 48 members of
-// 64 and 128 layers 4.30 -> 4.00.
+// 0.02, 128^3 0.327 -> 0.173, 384 x 384 x 192 with two tracers 4.38 -> 3.14;
+// FP32, 512 x 256 0.238 -> 0.02, 384 x 384 x 192 3.58 -> 2.57, 48 members of
+// 64 and 128 layers 4.30 -> 3.79.  Columns that it solves in sequence
+// (chunk_solve) are the exception: 128^3 with every column so 1.82.
 static const char* vic_kernel_env() {
   const char* v = std::getenv("SNAPB_VIC_KERNEL");
   return v ? v : "";
