@@ -218,7 +218,7 @@ constexpr double kX1Resident32 = 148. * 24.;
 // copies into shared memory, barriers, the revision in its own kernel):
 // 384 x 384 x 192, Roe, two tracers 1.29 -> 1.25 ms, 512 x 256 21.0 -> 10.7 us,
 // 48 members of 64 and 128 layers 1.57 -> 1.22 ms; a 1-D block of 1024 cells, whose
-// column is not cut, 85 -> 107 us.
+// column is not cut, 90 -> 57 us.
 template <int NS, int FP>
 __device__ __noinline__ void x1_32_item(int64_t item, int last) {
   constexpr int NV = 5 + NS;
